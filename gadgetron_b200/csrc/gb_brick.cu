@@ -1,0 +1,679 @@
+// Gridding (NC2C), 2D and 3D: one warp per brick of cells.
+//
+// Reference kernels this replaces:
+//   toolboxes/nfft/gpu/ConvolverNC2C_standard.cuh:229-355 (+ the wrap pass
+//   :358-477 and the cell/sample pair sort of
+//   toolboxes/nfft/gpu/cuGriddingConvolution.cu:361-422)
+//
+// A tile of the oversampled grid is cut into bricks; a warp owns one brick for
+// one coil group and walks the tile's sample list alone: it tests 32 samples
+// at a time against its brick (one ballot over the packed footprint ranges) and
+// queues the hits; batches of queued hits are staged into a small ring of the
+// warp's own shared memory by asynchronous copies (coil values, and the x, y, z
+// weights of the brick from the sample's pair row -- weights laid over the
+// tile, zero outside the footprint) two batches ahead of the one being summed.
+// A lane is a (few coils, x column[, y block]) of the brick and keeps YC x ZC
+// cells of 1 to 4 coils in registers; a hit costs it a few shared loads and
+// packed FP32x2 multiply-adds over pairs of y cells.  Warps never wait for one
+// another inside a list (only the chunks of a split tile meet, through a
+// counter), and a lane's cells go straight from registers to the grid.  No
+// atomics on the grid; per-cell sums follow the list order: results are
+// bit-reproducible.
+//
+// What bounds it, and what was tried: loading a hit's operands straight from
+// L2 one hit ahead left every warp waiting on that latency (118 us for the
+// launch below against 36 us); one staged hit per copy spent 115 instructions
+// a hit on staging, batches of 4 to 8 spend about 15.  Now 16 coils in 2D run
+// at 52 % of the issue slots with the shared-memory pipe at 75 % (value and
+// weight loads, scattered 32-byte stores); 3D is issue- and latency-bound at
+// 16 warps per SM (64 accumulators a lane).  Launch times before (a CTA per
+// tile staging chunks through registers or a producer warp) and after:
+//   32768 radial samples, 1 coil, 256^2 grid           63.6 -> 17 us
+//   98304 spiral samples, 32 coils, compensated, 640^2  411 -> 140 us
+//   5.12 M kooshball samples, 32 coils, 192^3          13.2 -> 7.5 ms
+//   1.29 M samples in 64 frames, 12 coils, 384^2        630 -> 490 us
+//   49152 radial samples, 16 coils, 512^2                37 -> 35 us
+//
+// A zero weight times an infinity would put a NaN into cells the footprint
+// does not touch, so a brick whose sums came out non-finite is summed again
+// with the zero-weight cells skipped (the values of finite data never change).
+#include <algorithm>
+#include <type_traits>
+
+#include "gb_conv.cuh"
+
+namespace gb {
+
+// CPL coils per lane, LPC lanes over the coils of a group, XL x YL lanes over
+// the columns, YC x ZC cells per lane, at most NT threads (warps * 32) per CTA,
+// MB resident CTAs asked of the register allocation.
+template <int CPL_, int LPC_, int XL_, int YL_, int YC_, int ZC_, bool D3_, int NT_, int MB_>
+struct BrickShape {
+    static constexpr int CPL = CPL_, LPC = LPC_, XL = XL_, YL = YL_, YC = YC_, ZC = ZC_, NT = NT_, MB = MB_;
+    static constexpr bool D3 = D3_;
+    static constexpr int CG = CPL * LPC, BX = XL, BY = YL * YC, BZ = ZC, YP = YC / 2, V = 2 * CPL;
+    static constexpr int NACC = ZC * YP * V;   // float2 accumulators of a lane
+    // A staged hit, in 16-byte chunks: coil values, x, y and z weights of the
+    // brick (x and z from the aligned group of 4 that holds them).
+    static constexpr int VC = (CG * 8 + 15) / 16, XC = (BX + 3) / 4, YCH = BY / 4, ZCH = D3 ? 1 : 0;
+    static constexpr int WCH = XC + YCH + ZCH, WL = WCH <= 4 ? 4 : 8;       // weight chunks, lanes staging them
+    static constexpr int SLOT = VC + WCH + 1;                               // one more: the density weight
+    static constexpr int UH = NACC > 16 ? 1 : 2;                            // hits summed together
+    static constexpr int HB = CG >= 12 ? 4 : 8;                             // hits staged together
+    static_assert(LPC * XL * YL == 32 && YC % 2 == 0 && BY % 4 == 0, "a brick fills a warp");
+};
+
+constexpr int kBrickDepth = 3;    // batches of hits in the ring of a warp
+constexpr int kBrickQueue = 64;   // pending hits of a warp
+// Bricks (warps) per CTA: a CTA's slot is held until its slowest brick is done
+// (samples crowd), so a tile of more bricks is spread over several CTAs.
+constexpr int kBrickCtaWarps = 4;
+constexpr int kBrickFillWarps = 148 * 12;   // warps that fill the GPU
+constexpr int kBrickWideWarps = 148 * 24 * 4;   // narrow-form warps from which the wide form is taken
+
+// Asynchronous copy of BYTES to shared memory; zeros instead when !full.
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src, bool full) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(BYTES), "r"(full ? BYTES : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ float2 f2neg(float2 a) { return make_float2(-a.x, -a.y); }
+
+// Compensated sum += v.
+__device__ __forceinline__ void comp_add(float2 &sum, float2 &err, float2 v) {
+    const float2 t = __fadd2_rn(v, f2neg(err));
+    const float2 n = __fadd2_rn(sum, t);
+    err = __fadd2_rn(__fadd2_rn(n, f2neg(sum)), f2neg(t));
+    sum = n;
+}
+
+template <class S, bool COMP, bool IL>
+__global__ void __launch_bounds__(S::NT, COMP ? (S::MB + 1) / 2 : S::MB)
+k_grid_brick(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict__ grid) {
+    constexpr int CPL = S::CPL, LPC = S::LPC, YC = S::YC, ZC = S::ZC, YP = S::YP, V = S::V;
+    constexpr bool D3 = S::D3;
+    constexpr int VC = S::VC, XC = S::XC, YCH = S::YCH, WCH = S::WCH, WL = S::WL, SLOT = S::SLOT, HB = S::HB;
+    constexpr int DEPTH = kBrickDepth;
+    // [warps][DEPTH][HB][SLOT] staged hits, [warps][kBrickQueue] pending hits;
+    // afterwards the sums of list parts
+    extern __shared__ float4 brick_sm[];
+    __shared__ int s_last;
+    const KParams &k = a.k;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int b0 = (int)blockIdx.y * S::CG;
+    // a tile's bricks are spread over `groups` CTAs of 1 << lcta bricks
+    const int groups = 1 << (a.lbricks - a.lcta), group = (int)blockIdx.x & (groups - 1);
+    const WorkItem it = a.items[blockIdx.x >> (a.lbricks - a.lcta)];
+    const int T0 = k.tile[0], T1 = k.tile[1];
+    // `parts` warps share a brick: part p takes blocks p, p + parts, ... of the list
+    const int nbricks = 1 << a.lcta, parts = 1 << a.lparts;   // bricks of this CTA
+    const int slot_id = warp & (nbricks - 1), part_id = warp >> a.lcta;
+    const int brick = (group << a.lcta) + slot_id;
+    const int bx = brick & ((1 << a.lbx) - 1), by = (brick >> a.lbx) & ((1 << a.lby) - 1), bz = brick >> (a.lbx + a.lby);
+    const int x0 = bx * S::BX, y0 = by * S::BY, z0 = bz * S::BZ;   // the brick within the tile
+    const int cp = lane % LPC, lx = (lane / LPC) % S::XL, ly = lane / (LPC * S::XL);
+    const int coil = b0 + CPL * cp;
+    const bool coil_ok = coil < a.nb;
+    float4 *ring = brick_sm + warp * (DEPTH * HB * SLOT);
+    uint2 *queue = reinterpret_cast<uint2 *>(brick_sm + (blockDim.x >> 5) * (DEPTH * HB * SLOT)) + warp * kBrickQueue;
+
+    float2 acc[ZC][YP][V];                                    // [z][y pair][re, im of each coil]
+    float2 cmp[COMP ? ZC : 1][COMP ? YP : 1][COMP ? V : 1];
+
+    // This lane's weight chunk when staging (WL lanes per hit).
+    const int wch = lane % WL;
+    const int woff = wch < XC ? (x0 & ~3) + 4 * wch
+                              : (wch < XC + YCH ? T0 + y0 + 4 * (wch - XC) : T0 + T1 + (z0 & ~3));
+    const float *wsrc = a.prows + woff;
+
+    auto pass = [&](auto safe_c) {
+        constexpr bool SAFE = decltype(safe_c)::value;
+#pragma unroll
+        for (int z = 0; z < ZC; z++)
+#pragma unroll
+            for (int y = 0; y < YP; y++)
+#pragma unroll
+                for (int c = 0; c < V; c++) {
+                    acc[z][y][c] = make_float2(0.f, 0.f);
+                    if (COMP) cmp[z][y][c] = make_float2(0.f, 0.f);
+                }
+        // values of coils beyond nb are never staged: zero them once
+        for (int e = lane; e < DEPTH * HB * SLOT; e += 32) ring[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        // Blocks of 32 list entries: the next block's entries are loaded
+        // while the current block's hits are staged and summed.
+        const int bstep = 32 * parts;
+        uint32_t p_id = 0;
+        uint2 p_rg = make_uint2(0u, 0u);
+        int next = it.begin + 32 * part_id;
+        int q_head = 0, q_tail = 0;   // pending hits (sample, pair) in the queue
+        auto fetch = [&](int b) {
+            if (b + lane >= it.end) return;
+            p_rg = __ldg(a.prng + b + lane);
+            p_id = __ldg(a.list + b + lane);
+            if (!IL && a.layout == LAYOUT_ORIGINAL) p_id = __ldg(a.perm + p_id);
+        };
+        fetch(next);
+        // Stages the next (at most HB) hits into batch `t`; returns how many.
+        auto stage = [&](int t) -> int {
+            while (q_tail - q_head < HB && next < it.end) {
+                const int xlo = p_rg.x & 0xff, xhi = (p_rg.x >> 8) & 0xff;
+                const int ylo = (p_rg.x >> 16) & 0xff, yhi = p_rg.x >> 24;
+                bool hit = next + lane < it.end && xlo < x0 + S::BX && xhi >= x0 && ylo < y0 + S::BY && yhi >= y0;
+                if (D3) hit = hit && (int)(p_rg.y & 0xff) < z0 + S::BZ && (int)((p_rg.y >> 8) & 0xff) >= z0;
+                const uint32_t bits = __ballot_sync(0xffffffffu, hit);
+                if (hit)
+                    queue[(q_tail + __popc(bits & ((1u << lane) - 1u))) % kBrickQueue] =
+                        make_uint2(p_id, (uint32_t)(next + lane));
+                q_tail += __popc(bits);
+                next += bstep;
+                fetch(next);
+            }
+            __syncwarp();   // the queue is visible; the batch summed before may be overwritten
+            const int n = min(HB, q_tail - q_head);
+            float4 *batch = ring + t * (HB * SLOT);
+            if (n > 0) {
+#pragma unroll
+                for (int e0 = 0; e0 < HB * WL; e0 += 32) {   // weights, zero for the missing hits of a short batch
+                    const int h = (e0 + lane) / WL;
+                    if (h < HB && wch < WCH) {
+                        const uint32_t pair = queue[(q_head + (h < n ? h : 0)) % kBrickQueue].y;
+                        cp_async<16>(batch + h * SLOT + VC + wch, wsrc + (int64_t)pair * a.prow_floats, h < n);
+                    }
+                }
+                if (IL) {
+#pragma unroll
+                    for (int e0 = 0; e0 < HB * VC; e0 += 32) {
+                        const int h = (e0 + lane) / VC, c = (e0 + lane) % VC;
+                        if (h < n && b0 + 2 * c < a.nb) {
+                            const uint32_t id = queue[(q_head + h) % kBrickQueue].x;
+                            cp_async<16>(batch + h * SLOT + c, samples + (int64_t)id * a.il_stride + b0 + 2 * c, true);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int e0 = 0; e0 < HB * S::CG; e0 += 32) {
+                        const int h = (e0 + lane) / S::CG, c = (e0 + lane) % S::CG;
+                        if (h < n && b0 + c < a.nb) {
+                            const uint32_t id = queue[(q_head + h) % kBrickQueue].x;
+                            cp_async<8>(reinterpret_cast<float2 *>(batch + h * SLOT) + c,
+                                        samples + (int64_t)(b0 + c) * a.Mtot + id, true);
+                        }
+                    }
+                    if (a.dcw && lane < n) {
+                        const uint32_t id = queue[(q_head + lane) % kBrickQueue].x;
+                        const uint32_t j = a.layout == LAYOUT_ORIGINAL ? id : __ldg(a.perm + id);
+                        cp_async<4>(batch + lane * SLOT + VC + WCH, a.dcw + j, true);
+                    }
+                }
+                q_head += n;
+            }
+            cp_async_commit();
+            return n;
+        };
+        auto add = [&](const float4 *slot) {
+            const float *wf = reinterpret_cast<const float *>(slot + VC);
+            float v[V];
+            if (CPL % 2 == 0) {
+#pragma unroll
+                for (int c = 0; c < CPL / 2; c++) {
+                    const float4 q = slot[cp * (CPL / 2) + c];
+                    v[(4 * c) % V] = q.x;
+                    v[(4 * c + 1) % V] = q.y;
+                    v[(4 * c + 2) % V] = q.z;
+                    v[(4 * c + 3) % V] = q.w;
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < CPL; c++) {
+                    const float2 q = reinterpret_cast<const float2 *>(slot)[cp * CPL + c];
+                    v[2 * c] = q.x;
+                    v[2 * c + 1] = q.y;
+                }
+            }
+            if (!IL && a.dcw) {
+                const float dw = *reinterpret_cast<const float *>(slot + VC + WCH);
+#pragma unroll
+                for (int c = 0; c < V; c++) v[c] = dw * v[c];
+            }
+            const float wx = wf[(x0 & 3) * (S::BX < 4) + lx];
+            float2 wxy[YP];
+            const float2 wx2 = make_float2(wx, wx);
+            if (YC % 4 == 0) {
+#pragma unroll
+                for (int q = 0; q < YC / 4; q++) {
+                    const float4 w = reinterpret_cast<const float4 *>(slot + VC + XC)[ly * (YC / 4) + q];
+                    wxy[2 * q] = __fmul2_rn(make_float2(w.x, w.y), wx2);
+                    wxy[(2 * q + 1) % YP] = __fmul2_rn(make_float2(w.z, w.w), wx2);
+                }
+            } else {
+#pragma unroll
+                for (int y = 0; y < YP; y++)
+                    wxy[y] = __fmul2_rn(reinterpret_cast<const float2 *>(wf + 4 * XC + ly * YC)[y], wx2);
+            }
+            float wzs[4] = {1.f, 1.f, 1.f, 1.f};
+            if (D3) {
+                const float4 w = slot[VC + XC + YCH];
+                wzs[0] = w.x;
+                wzs[1] = w.y;
+                wzs[2] = w.z;
+                wzs[3] = w.w;
+                if (S::BZ < 4 && (z0 & 2)) {
+                    wzs[0] = w.z;
+                    wzs[1] = w.w;
+                }
+            }
+            float2 vd[V];
+#pragma unroll
+            for (int c = 0; c < V; c++) vd[c] = make_float2(v[c], v[c]);
+#pragma unroll
+            for (int z = 0; z < ZC; z++) {
+                const float wz = wzs[z];
+                if (ZC > 2 && wz == 0.f) continue;   // a slice the footprint misses (the same for every lane)
+#pragma unroll
+                for (int y = 0; y < YP; y++) {
+                    const float2 w = D3 ? __fmul2_rn(wxy[y], make_float2(wz, wz)) : wxy[y];
+#pragma unroll
+                    for (int c = 0; c < V; c++) {
+                        float2 &t = acc[z][y][c];
+                        float2 n;
+                        if (COMP) {
+                            float2 &e = cmp[z][y][c];
+                            const float2 u = __ffma2_rn(w, vd[c], f2neg(e));
+                            n = __fadd2_rn(t, u);
+                            const float2 ne = __fadd2_rn(__fadd2_rn(n, f2neg(t)), f2neg(u));
+                            if (!SAFE) e = ne;
+                            else {
+                                if (w.x != 0.f) e.x = ne.x;
+                                if (w.y != 0.f) e.y = ne.y;
+                            }
+                        } else {
+                            n = __ffma2_rn(w, vd[c], t);
+                        }
+                        if (!SAFE) t = n;
+                        else {
+                            if (w.x != 0.f) t.x = n.x;
+                            if (w.y != 0.f) t.y = n.y;
+                        }
+                    }
+                }
+            }
+        };
+        // DEPTH - 1 batches are in flight (an empty group stands for a batch
+        // past the end); where registers allow, hits are summed in pairs, a
+        // missing second one with zero weights.
+        int cnt[DEPTH];
+#pragma unroll
+        for (int t = 0; t < DEPTH - 1; t++) cnt[t] = stage(t);
+        bool live = cnt[0] > 0;
+        while (live) {
+#pragma unroll
+            for (int t = 0; t < DEPTH; t++) {
+                if (!live) break;
+                cp_async_wait<DEPTH - 2>();
+                cnt[(t + DEPTH - 1) % DEPTH] = stage((t + DEPTH - 1) % DEPTH);
+                const float4 *slot = ring + t * (HB * SLOT);
+#pragma unroll 1
+                for (int h = 0; h < cnt[t]; h += S::UH, slot += S::UH * SLOT) {
+#pragma unroll
+                    for (int u = 0; u < S::UH; u++) add(slot + u * SLOT);
+                }
+                live = cnt[(t + 1) % DEPTH] > 0;
+            }
+        }
+        cp_async_wait<0>();
+        __syncwarp();
+    };
+    pass(std::false_type{});
+    float2 odd = make_float2(0.f, 0.f);   // stays 0 while every sum is finite
+#pragma unroll
+    for (int z = 0; z < ZC; z++)
+#pragma unroll
+        for (int y = 0; y < YP; y++)
+#pragma unroll
+            for (int c = 0; c < V; c++) odd = __ffma2_rn(acc[z][y][c], make_float2(0.f, 0.f), odd);
+    if (__any_sync(0xffffffffu, !(odd.x + odd.y == 0.f))) pass(std::true_type{});
+
+    if (parts > 1) {
+        // The first part's warp adds the other parts' sums in order.
+        __syncthreads();   // the rings are free
+        float4 *sums = brick_sm;
+        constexpr int N4 = S::NACC / 2;
+        if (part_id > 0) {
+            float4 *o = sums + ((part_id - 1) * nbricks + slot_id) * (N4 * 32) + lane;
+            int q = 0;
+#pragma unroll
+            for (int z = 0; z < ZC; z++)
+#pragma unroll
+                for (int y = 0; y < YP; y++)
+#pragma unroll
+                    for (int c = 0; c < V; c += 2, q++)
+                        o[q * 32] = make_float4(acc[z][y][c].x, acc[z][y][c].y, acc[z][y][c + 1].x, acc[z][y][c + 1].y);
+        }
+        __syncthreads();
+        if (part_id == 0) {
+            for (int p = 1; p < parts; p++) {
+                const float4 *o = sums + ((p - 1) * nbricks + slot_id) * (N4 * 32) + lane;
+                int q = 0;
+#pragma unroll
+                for (int z = 0; z < ZC; z++)
+#pragma unroll
+                    for (int y = 0; y < YP; y++)
+#pragma unroll
+                        for (int c = 0; c < V; c += 2, q++) {
+                            const float4 w = o[q * 32];
+                            if (COMP) {
+                                comp_add(acc[z][y][c], cmp[z][y][c], make_float2(w.x, w.y));
+                                comp_add(acc[z][y][c + 1], cmp[z][y][c + 1], make_float2(w.z, w.w));
+                            } else {
+                                acc[z][y][c] = __fadd2_rn(acc[z][y][c], make_float2(w.x, w.y));
+                                acc[z][y][c + 1] = __fadd2_rn(acc[z][y][c + 1], make_float2(w.z, w.w));
+                            }
+                        }
+            }
+        }
+    }
+
+    if (it.split >= 0) {
+        // Chunk of a split tile: write the partial bricks; the CTA of this
+        // group that arrives last sums the partials in chunk order.
+        const SplitInfo si = a.splits[it.split];
+        auto part = [&](int slot) -> float4 * {
+            return reinterpret_cast<float4 *>(a.partials + ((int64_t)slot * a.ncg + blockIdx.y) * a.part_elems) +
+                   32 * brick + lane;
+        };
+        const int nthr = 32 * nbricks * groups;   // lanes of the whole tile
+        if (part_id == 0) {
+            float4 *pp = part(si.first_slot + it.chunk);
+#pragma unroll
+            for (int z = 0; z < ZC; z++)
+#pragma unroll
+                for (int y = 0; y < YP; y++)
+#pragma unroll
+                    for (int c = 0; c < V; c += 2) {
+                        *pp = make_float4(acc[z][y][c].x, acc[z][y][c].y, acc[z][y][c + 1].x, acc[z][y][c + 1].y);
+                        pp += nthr;
+                    }
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned int *ctr = a.counters + ((int64_t)it.split * a.ncg + blockIdx.y) * groups + group;
+            const unsigned int old = atomicAdd(ctr, 1u);
+            s_last = (old == (unsigned int)(si.nchunks - 1));
+            if (s_last) *ctr = 0u;   // ready for the next launch
+        }
+        __syncthreads();
+        if (!s_last || part_id > 0) return;
+        __threadfence();
+#pragma unroll
+        for (int z = 0; z < ZC; z++)
+#pragma unroll
+            for (int y = 0; y < YP; y++)
+#pragma unroll
+                for (int c = 0; c < V; c++) {
+                    acc[z][y][c] = make_float2(0.f, 0.f);
+                    if (COMP) cmp[z][y][c] = make_float2(0.f, 0.f);
+                }
+#pragma unroll 2
+        for (int ch = 0; ch < si.nchunks; ch++) {
+            const float4 *pp = part(si.first_slot + ch);
+#pragma unroll
+            for (int z = 0; z < ZC; z++)
+#pragma unroll
+                for (int y = 0; y < YP; y++)
+#pragma unroll
+                    for (int c = 0; c < V; c += 2) {
+                        const float4 q = __ldcg(pp);
+                        pp += nthr;
+                        const float2 two[2] = {make_float2(q.x, q.y), make_float2(q.z, q.w)};
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            if (COMP) comp_add(acc[z][y][c + h], cmp[z][y][c + h], two[h]);
+                            else acc[z][y][c + h] = __fadd2_rn(acc[z][y][c + h], two[h]);
+                        }
+                    }
+        }
+    }
+
+    // Out: a lane's cells go straight to the grid (the x lanes of a coil are
+    // neighbours, so a store instruction writes whole 32-byte sectors).
+    if (!coil_ok || part_id > 0) return;
+    if (a.accumulate && it.begin == it.end && it.split < 0) return;
+    const int gx = it.tx * T0 + x0 + lx, gy0 = it.ty * T1 + y0 + ly * YC, gz0 = it.tz * k.tile[2] + z0;
+    const float s0 = (a.sign_fold && ((gx + gy0 + gz0) & 1)) ? -1.f : 1.f;
+    const float s1 = a.sign_fold ? -s0 : s0;
+    const int64_t plane = (int64_t)a.F * a.kl.s_bf;   // from coil to coil
+    float2 *cell = grid + (int64_t)coil * plane + (int64_t)it.f * a.kl.s_bf + (int64_t)gz0 * a.kl.s_z +
+                   (int64_t)gy0 * a.kl.s_y + gx;
+#pragma unroll
+    for (int z = 0; z < ZC; z++) {
+        const float2 sg = (z & 1) ? make_float2(s1, s0) : make_float2(s0, s1);
+#pragma unroll
+        for (int c = 0; c < CPL; c++) {
+            if (c > 0 && coil + c >= a.nb) break;
+            float2 *o = cell + c * plane + (int64_t)z * a.kl.s_z;
+#pragma unroll
+            for (int y = 0; y < YP; y++) {
+                const float2 re = __fmul2_rn(acc[z][y][2 * c], sg), im = __fmul2_rn(acc[z][y][2 * c + 1], sg);
+                float2 v0 = make_float2(re.x, im.x), v1 = make_float2(re.y, im.y);
+                float2 *o1 = o + a.kl.s_y;
+                if (a.accumulate) {
+                    const float2 p0 = *o, p1 = *o1;
+                    v0 = make_float2(v0.x + p0.x, v0.y + p0.y);
+                    v1 = make_float2(v1.x + p1.x, v1.y + p1.y);
+                }
+                *o = v0;
+                *o1 = v1;
+                o = o1 + a.kl.s_y;
+            }
+        }
+    }
+}
+
+// 32 samples x 32 coils per block through shared memory: the planes are read
+// along the samples, the rows written along the coils.
+__global__ void __launch_bounds__(256) k_samples_il(const float2 *__restrict__ samples, const float *__restrict__ dcw,
+                                                    const uint32_t *__restrict__ perm, int64_t M, int nb, int il,
+                                                    float2 *__restrict__ rows) {
+    __shared__ float2 t[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t i0 = (int64_t)blockIdx.x * 32;
+    const int c0 = (int)blockIdx.y * 32;
+    const int64_t i = i0 + lane;
+    uint32_t j = 0;
+    float w = 1.f;
+    if (i < M) {
+        j = perm[i];
+        if (dcw) w = dcw[j];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int c = c0 + warp + 8 * q;
+        float2 v = make_float2(0.f, 0.f);
+        if (i < M && c < nb) {
+            v = samples[(int64_t)c * M + j];
+            if (dcw) v = make_float2(w * v.x, w * v.y);
+        }
+        t[warp + 8 * q][lane] = v;
+    }
+    __syncthreads();
+    const int cn = min(32, il - c0);
+    for (int e = threadIdx.x; e < 32 * cn; e += 256) {
+        const int r = e / cn, c = e - r * cn;
+        if (i0 + r < M) rows[(i0 + r) * il + c0 + c] = t[c][r];
+    }
+}
+
+void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *dcw, int nb, float2 *rows,
+                       cudaStream_t st) {
+    const int il = il_stride_for(nb);
+    const dim3 g((unsigned)((p.Mtot + 31) / 32), (unsigned)((il + 31) / 32));
+    k_samples_il<<<g, 256, 0, st>>>(samples, dcw, p.perm.get(), p.Mtot, nb, il, rows); note_launch();
+    GB_CUDA(cudaGetLastError());
+}
+
+// ------------------------------------------------------------- dispatch ---
+//
+// The lanes left over by the coils of a group run along x (then y), so that a
+// group of any size fills the warp.  A brick of 8 x 8 cells is met by 2.4
+// times as many (sample, brick) pairs as there are samples at W = 5.5, one of
+// 4 x 8 by 3.3 times: the wide form of 16 coils (4 coils per lane, 4 warps a
+// tile) runs fewer instructions and serves launches with many waves of tiles,
+// the narrow one (2 coils per lane, 8 warps a tile) has shorter chains and
+// serves the small ones.  12 coils have a form of their own (3 per lane, no idle lanes).
+// 3D bricks are two slices thick (W = 4 meets 2.5 of them: 80 % of the slices
+// computed are hit).
+using Brick2D16 = BrickShape<2, 8, 4, 1, 8, 1, false, 256, 3>;
+using Brick2D16C = BrickShape<2, 8, 4, 1, 8, 1, false, 128, 6>;   // compensated
+using Brick2D16W = BrickShape<4, 4, 8, 1, 8, 1, false, 128, 4>;
+using Brick2D12 = BrickShape<3, 4, 8, 1, 8, 1, false, 128, 5>;
+using Brick2D8 = BrickShape<2, 4, 8, 1, 8, 1, false, 256, 3>;
+using Brick2D4 = BrickShape<2, 2, 8, 2, 4, 1, false, 512, 2>;
+using Brick2D2 = BrickShape<2, 1, 8, 4, 2, 1, false, 512, 2>;
+using Brick2D1 = BrickShape<1, 1, 8, 4, 2, 1, false, 512, 2>;
+using Brick3D32 = BrickShape<2, 16, 2, 1, 4, 4, true, 128, 4>;
+using Brick3D16 = BrickShape<2, 8, 4, 1, 4, 4, true, 128, 4>;
+using Brick3D8 = BrickShape<2, 4, 8, 1, 4, 4, true, 128, 4>;
+using Brick3D16C = BrickShape<2, 8, 4, 1, 4, 2, true, 128, 4>;    // compensated
+using Brick3D8C = BrickShape<2, 4, 8, 1, 4, 2, true, 128, 4>;
+using Brick3D4 = BrickShape<2, 2, 8, 2, 4, 2, true, 256, 3>;
+using Brick3D2 = BrickShape<2, 1, 8, 4, 2, 2, true, 256, 3>;
+using Brick3D1 = BrickShape<1, 1, 8, 4, 2, 2, true, 256, 4>;
+
+template <class S>
+static int bricks_of(const KParams &k) {
+    if (k.tile[0] % S::BX || k.tile[1] % S::BY || k.tile[2] % S::BZ) return 0;
+    const int n = (k.tile[0] / S::BX) * (k.tile[1] / S::BY) * (k.tile[2] / S::BZ);
+    // tile extents are powers of two (a tile holds a divisor of 256 cells, 512 or 1024)
+    return (n <= 4 * kBrickCtaWarps && (n & (n - 1)) == 0) ? n : 0;
+}
+
+static int bricks_for(const KParams &k, int cg, bool comp) {
+    if (k.D == 2) {
+        switch (cg) {
+            case 16: return bricks_of<Brick2D16>(k);
+            case 12: return comp ? 0 : bricks_of<Brick2D12>(k);
+            case 8: return bricks_of<Brick2D8>(k);
+            case 4: return bricks_of<Brick2D4>(k);
+            case 2: return bricks_of<Brick2D2>(k);
+            default: return bricks_of<Brick2D1>(k);
+        }
+    }
+    switch (cg) {
+        case 32: return comp ? 0 : bricks_of<Brick3D32>(k);
+        case 16: return comp ? bricks_of<Brick3D16C>(k) : bricks_of<Brick3D16>(k);
+        case 8: return comp ? bricks_of<Brick3D8C>(k) : bricks_of<Brick3D8>(k);
+        case 4: return bricks_of<Brick3D4>(k);
+        case 2: return bricks_of<Brick3D2>(k);
+        default: return bricks_of<Brick3D1>(k);
+    }
+}
+
+bool brick_config(const NufftPlan &p, int nb, GridCfg &c) {
+    const KParams &k = p.kp;
+    if (k.D < 2 || p.pair_row_stride <= 0 || p.pair_row_stride != pair_row_floats(k)) return false;
+    const bool comp = (p.flags & GB_FLAG_COMPENSATED) != 0;
+    int cg = choose_cg(p.tiling.cg, nb);
+    // 3D, more than 16 coils: one group of 32 visits a sample's bricks once
+    // instead of twice
+    if (k.D == 3 && cg == 16 && nb > 16 && bricks_for(k, 32, comp)) cg = 32;
+    if (k.D == 2 && cg == 16 && nb % 12 == 0 && nb % 16 != 0 && bricks_for(k, 12, comp)) cg = 12;
+    int n = bricks_for(k, cg, comp);
+    if (!n) return false;
+    c.brick = true;
+    c.cg = cg;
+    c.wide = false;
+    if (k.D == 2 && cg == 16 && !comp && bricks_of<Brick2D16W>(k) &&
+        (int64_t)p.n_grd_items * ((nb + cg - 1) / cg) * n >= kBrickWideWarps) {
+        c.wide = true;
+        n = bricks_of<Brick2D16W>(k);
+    }
+    c.nbricks = n;
+    // (the short lists of the narrow 2D form leave no such imbalance: 8 bricks)
+    c.groups = std::max(1, n / (k.D == 2 && cg == 16 && !comp ? 2 * kBrickCtaWarps : kBrickCtaWarps));
+    return true;
+}
+
+template <class S, bool COMP>
+static void brick_launch(const GridCfg &c, const ConvArgs &args, const float2 *samples, float2 *grid, cudaStream_t st) {
+    ConvArgs a = args;
+    const int cta = c.nbricks / c.groups;   // bricks per CTA
+    // Warps per brick: one when the bricks alone fill the GPU, more (each with
+    // its share of the list) when the launch is small and bound by its longest
+    // list.  Powers of two, as the tile's extents.
+    int parts = 1;
+    while (2 * parts * cta * 32 <= S::NT && (int64_t)a.n_items * c.ncg * c.nbricks * parts < kBrickFillWarps)
+        parts *= 2;
+    auto log2i = [](int v) {
+        int l = 0;
+        while ((1 << l) < v) l++;
+        return l;
+    };
+    a.lbx = log2i(a.k.tile[0] / S::BX);
+    a.lby = log2i(a.k.tile[1] / S::BY);
+    a.lbricks = log2i(c.nbricks);
+    a.lcta = log2i(cta);
+    a.lparts = log2i(parts);
+    const int warps = cta * parts;
+    const dim3 g((unsigned)(a.n_items * c.groups), (unsigned)c.ncg);
+    const size_t ring = (size_t)warps * (kBrickDepth * S::HB * S::SLOT * 16 + kBrickQueue * sizeof(uint2));
+    const size_t smem = std::max(ring, (size_t)(warps - cta) * S::NACC * 32 * 8);
+    auto go = [&](auto kern) {
+        if (smem > 48 * 1024)
+            GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<g, 32 * warps, smem, st>>>(a, samples, grid); note_launch();
+    };
+    if constexpr (S::CPL >= 2) {
+        if (a.layout == LAYOUT_SORTED_IL) {
+            go(k_grid_brick<S, COMP, true>);
+            return;
+        }
+    }
+    go(k_grid_brick<S, COMP, false>);
+}
+
+void launch_grid_brick(const GridCfg &c, const NufftPlan &p, const ConvArgs &a, const float2 *samples, float2 *grid,
+                       cudaStream_t st) {
+    const bool comp = (p.flags & GB_FLAG_COMPENSATED) != 0;
+    if (a.layout == LAYOUT_SORTED_IL && (c.cg < 2 || a.dcw))
+        fail(GB_ERR_INTERNAL, "interleaved samples need a coil pair per lane and carry their density weights");
+#define GB_BRICK(S) (comp ? brick_launch<S, true>(c, a, samples, grid, st) : brick_launch<S, false>(c, a, samples, grid, st))
+    if (p.kp.D == 2) {
+        switch (c.cg) {
+            case 12: brick_launch<Brick2D12, false>(c, a, samples, grid, st); break;
+            case 16:
+                if (c.wide) brick_launch<Brick2D16W, false>(c, a, samples, grid, st);
+                else if (comp) brick_launch<Brick2D16C, true>(c, a, samples, grid, st);
+                else brick_launch<Brick2D16, false>(c, a, samples, grid, st);
+                break;
+            case 8: GB_BRICK(Brick2D8); break;
+            case 4: GB_BRICK(Brick2D4); break;
+            case 2: GB_BRICK(Brick2D2); break;
+            default: GB_BRICK(Brick2D1); break;
+        }
+    } else {
+        switch (c.cg) {
+            case 32: brick_launch<Brick3D32, false>(c, a, samples, grid, st); break;
+            case 16:
+                if (comp) brick_launch<Brick3D16C, true>(c, a, samples, grid, st);
+                else brick_launch<Brick3D16, false>(c, a, samples, grid, st);
+                break;
+            case 8:
+                if (comp) brick_launch<Brick3D8C, true>(c, a, samples, grid, st);
+                else brick_launch<Brick3D8, false>(c, a, samples, grid, st);
+                break;
+            case 4: GB_BRICK(Brick3D4); break;
+            case 2: GB_BRICK(Brick3D2); break;
+            default: GB_BRICK(Brick3D1); break;
+        }
+    }
+#undef GB_BRICK
+    GB_CUDA(cudaGetLastError());
+}
+
+}  // namespace gb

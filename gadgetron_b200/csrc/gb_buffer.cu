@@ -119,7 +119,7 @@ bool SenseBuffer::add_frame_data(const float2 *samples, const float *traj, int64
         GB_CUDA(cudaGetLastError());
         in = scaled.get();
     }
-    nufft_convolve(p, in, cur, GB_CONV_NC2C, true, coils, st);
+    nufft_convolve(p, in, cur, GB_CONV_NC2C, true, coils, st, true);
     bool completed = false;
     if (cur_sub_idx == sub_cycle_length - 1) {
         completed = true;

@@ -1,0 +1,71 @@
+// Arguments and launch configuration shared by the convolution kernels
+// (gridding: gb_brick.cu and k_grid_nc2c in gb_grid.cu; degridding and the
+// trajectory gradient: gb_grid.cu).
+#pragma once
+
+#include "gb_internal.cuh"
+
+namespace gb {
+
+struct ConvArgs {
+    KParams k;
+    const float *pos;         // [D][Mtot] sorted positions
+    const float *wtab;        // [Mtot][D][kWMax] tap weights of sorted samples
+    const uint32_t *perm;     // sorted -> original
+    const uint32_t *list;     // gridding list (sorted positions) or unused
+    const WorkItem *items;
+    int n_items;
+    int64_t Mtot;
+    int F;
+    int nb;
+    int layout;               // SampleLayout
+    int il_stride;            // SORTED_IL: float2 per sample row (nb rounded up to even)
+    const uint32_t *home_key; // sorted home keys (frame * ntiles_total + tile)
+    const float *dcw;         // original order, may be null
+    int dcw_pow;
+    int sign_fold;
+    int accumulate;
+    // gridding split bookkeeping
+    const SplitInfo *splits;
+    float2 *partials;
+    unsigned int *counters;
+    int ncg;
+    long long part_elems;     // float2 elements of one CTA's partial tile
+    KLayout kl;               // k-space array layout
+    const float *prows;       // gridding pair rows
+    const uint2 *prng;        // footprint ranges of the gridding pairs
+    int prow_floats;
+    int lbx, lby, lbricks;    // brick kernel, log2: bricks per tile along x and y, in all,
+    int lcta, lparts;         //   per CTA, warps per brick
+};
+
+__device__ __forceinline__ float sign_of(int g) { return (g & 1) ? -1.f : 1.f; }
+
+// Which gridding kernel runs for a plan and batch count, with its coil group
+// and the size of one CTA's partial tile (split tiles).
+struct GridCfg {
+    bool brick;       // k_grid_brick (else k_grid_nc2c)
+    int cg;
+    int nbricks;      // brick kernel: bricks per tile
+    bool wide;        // brick kernel: wide form of 16 coils
+    int groups = 1;   // CTAs (split-tile counters) per tile
+    int cpt;          // cell variant: cells per thread
+    int ncg;
+    int64_t part_elems;
+};
+
+// Coil group for nb batches: the requested one, halved while half of it
+// still covers all of them.
+int choose_cg(int requested, int nb);
+
+// gb_brick.cu: fills cg and nbricks for this plan's tile; false when no brick
+// shape divides the tile (1D plans, unusual tiles).
+bool brick_config(const NufftPlan &p, int nb, GridCfg &c);
+void launch_grid_brick(const GridCfg &c, const NufftPlan &p, const ConvArgs &a, const float2 *samples, float2 *grid,
+                       cudaStream_t st);
+// Samples [nb][Mtot] in the caller's order -> sorted coil-interleaved rows
+// [Mtot][il] (padding zero), density weights folded in (dcw may be null).
+void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *dcw, int nb, float2 *rows,
+                       cudaStream_t st);
+
+}  // namespace gb

@@ -15,66 +15,34 @@
 // cell is folded by -pad/2; for C2NC s - pad/2 is used directly
 // (ConvolverC2NC.cuh:239-241).
 //
-// B200 design:
+// The 2D and 3D kernels for the usual tiles are in gb_brick.cu (gridding) and
+// gb_degrid.cu (degridding, trajectory gradient); the kernels here serve 1D
+// plans, tiles that the bricks do not divide and kernels of fewer than 4 taps:
 //   * gridding is output-driven per tile: a CTA owns a tile of the
 //     oversampled grid, each thread owns CPT cells and accumulates a group of
 //     CG coils in registers; a warp covers an 8x4 patch of cells so that a
 //     sample footprint lights up a dense block of lanes.  Samples touching the
-//     tile are staged 32 at a time in shared memory (positions -> separable
+//     tile are staged 64 at a time in shared memory (positions -> separable
 //     weights, values with the density weights folded in).  No atomics: the
 //     result is bit-reproducible.  Tiles with long sample lists are split
 //     over several CTAs whose partial tiles are summed in a fixed order by
 //     the last CTA to finish.
 //   * degridding stages the home tile plus a halo of pad/2 cells, coil
-//     fastest, in shared memory; a warp serves one sample at a time with its
-//     lanes over (coil, re/im), the separable weights are computed by 8 lanes
-//     per dimension and broadcast by shuffles.
-//   * the centring checkerboard of the centred FFT ((-1)^(sum of cell
-//     coordinates), cuNDFFT.cu:6-36) is folded into the separable weights
-//     (sign_fold), and the density weights are folded into the sample loads
-//     (gridding) or stores (degridding).
+//     fastest, in shared memory; a warp serves 32 / (lanes per sample) samples
+//     at once with the separable weights staged per warp.
+// In all of them the centring checkerboard of the centred FFT ((-1)^(sum of
+// cell coordinates), cuNDFFT.cu:6-36) is folded into the weights or the stores
+// (sign_fold), and the density weights into the sample loads (gridding) or
+// stores (degridding).
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
 
+#include "gb_conv.cuh"
 #include "gb_internal.cuh"
 #include "gb_ops.hpp"
 
 namespace gb {
-
-struct ConvArgs {
-    KParams k;
-    const float *pos;         // [D][Mtot] sorted positions
-    const float *wtab;        // [Mtot][D][kWMax] tap weights of sorted samples
-    const uint32_t *perm;     // sorted -> original
-    const uint32_t *list;     // gridding list (sorted positions) or unused
-    const WorkItem *items;
-    int n_items;
-    int64_t Mtot;
-    int F;
-    int nb;
-    int layout;               // SampleLayout
-    int il_stride;            // SORTED_IL: float2 per sample row (nb rounded up to even)
-    const uint32_t *home_key; // sorted home keys (frame * ntiles_total + tile)
-    const float *dcw;         // original order, may be null
-    int dcw_pow;
-    int sign_fold;
-    int accumulate;
-    // gridding split bookkeeping
-    const SplitInfo *splits;
-    float2 *partials;
-    unsigned int *counters;
-    int ncg;
-    long long part_elems;     // float2 elements of one CTA's partial tile
-    KLayout kl;               // k-space array layout
-    const float *prows;       // gridding pair rows (row variant)
-    int prow_floats;
-    unsigned int *err;        // bounded-wait failure flag
-    unsigned int *queue;      // persistent gridding: [0] next work unit, [1] CTAs finished
-    int n_work;               // persistent gridding: work units (items x coil groups)
-};
-
-__device__ __forceinline__ float sign_of(int g) { return (g & 1) ? -1.f : 1.f; }
 
 // --------------------------------------------------------------- NC2C -----
 
@@ -96,11 +64,7 @@ k_grid_nc2c(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict__
     const int grp = blockIdx.y;
     const int b0 = grp * CG;
     const WorkItem it = a.items[item_idx];
-    const int f = it.ft / k.ntiles_total;
-    const int tile = it.ft - f * k.ntiles_total;
-    const int tx = tile % k.ntiles[0];
-    const int ty = (tile / k.ntiles[0]) % k.ntiles[1];
-    const int tz = tile / (k.ntiles[0] * k.ntiles[1]);
+    const int f = it.f, tx = it.tx, ty = it.ty, tz = it.tz;
     const int org[3] = {tx * k.tile[0], ty * k.tile[1], tz * k.tile[2]};
 
     __shared__ GridStage<CG> stage[2];
@@ -373,1031 +337,6 @@ k_grid_nc2c(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict__
     }
 }
 
-// ------------------------------------------------- NC2C, row variant -----
-//
-// Gridding for coil groups of 8 or 16 without compensation.  The tile is cut
-// into regions of ROWS x RW cells (ROWS = 64 / CG rows of RW columns, one
-// z-slice); warp w owns regions w, w + 8, ... (RPW of them).  A lane is a
-// (coil pair, row) of a region and accumulates that row's RW cells for two
-// coils in registers, so every lane of a warp works on every sample that
-// touches the region.  One visit (sample, region) costs a 16-byte value load,
-// the row's y (and z) weight, RW x-weights read as float4 from a per-sample
-// weight row laid over the tile (zero outside the footprint) and 4*RW FMAs.
-// Sample order per cell is the list order, as in k_grid_nc2c: the result is
-// bit-reproducible.
-
-constexpr int kChunkR = 64;   // samples staged per pass (row variant)
-
-// Per stage: the chunk's pair rows (one bulk copy) and its values (sample
-// stride cg + 2 float2: an odd number of 16-byte chunks).
-__host__ __device__ __forceinline__ int row_stage_bytes(const KParams &k, int cg) {
-    return kChunkR * (pair_row_floats(k) * 4 + (cg + 2) * 8);
-}
-
-// mbarrier + bulk-copy (TMA) helpers.  Waits are bounded: after ~1 s a wait
-// records the failure in *err and waits once more (also bounded) for the copy
-// still in flight, then gives up; the results are then wrong but no thread
-// spins forever.
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() {
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity, unsigned int *err) {
-    for (int round = 0; round < 2; round++) {
-        for (uint32_t i = 0; i < (1u << 22); i++) {
-            if (mbar_try_wait(bar, parity)) return;
-            if (i >= 16) __nanosleep(256);
-        }
-        if (round == 0 && err) atomicOr(err, 1u);
-    }
-}
-
-template <int CG, int RW, int RPW, bool D3>
-__global__ void __launch_bounds__(kThreads, (RPW * RW <= 8) ? 3 : 2)
-k_grid_rows(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict__ grid) {
-    constexpr int CP = CG / 2;      // lanes per row: one per coil pair
-    constexpr int ROWS = 32 / CP;   // rows per region
-    constexpr int SVS = CG + 2;     // staged values: float2 per sample (padded)
-    constexpr int kVE = (kChunkR * CG + kThreads - 1) / kThreads;
-    extern __shared__ __align__(128) unsigned char g_rows_smem[];
-    __shared__ int s_last;
-
-    const KParams &k = a.k;
-    const int grp = blockIdx.y;
-    const int b0 = grp * CG;
-    const WorkItem it = a.items[blockIdx.x];
-    const int f = it.ft / k.ntiles_total;
-    const int tile = it.ft - f * k.ntiles_total;
-    const int tx = tile % k.ntiles[0];
-    const int ty = (tile / k.ntiles[0]) % k.ntiles[1];
-    const int tz = tile / (k.ntiles[0] * k.ntiles[1]);
-    const int org0 = tx * k.tile[0], org1 = ty * k.tile[1], org2 = tz * k.tile[2];
-    const int T0 = k.tile[0], T1 = k.tile[1];
-    const int PRF = a.prow_floats;   // floats per pair row
-    const int PRW = PRF - 4;         // weight part; the last 4 words are the footprint ranges
-    const int stage_bytes = row_stage_bytes(k, CG);
-    __shared__ __align__(8) unsigned long long s_bar[2];   // one mbarrier per stage
-
-    auto stage_wt = [&](int s) { return reinterpret_cast<float *>(g_rows_smem + s * stage_bytes); };
-    auto stage_v = [&](int s) {
-        return reinterpret_cast<float2 *>(g_rows_smem + s * stage_bytes + kChunkR * PRF * 4);
-    };
-
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int cp = lane % CP, row = lane / CP;
-    const int nrx = T0 / RW, nry = T1 / ROWS;
-    int qx0[RPW], qy0[RPW], qz[RPW];
-#pragma unroll
-    for (int c = 0; c < RPW; c++) {
-        const int q = warp + 8 * c;
-        qx0[c] = (q % nrx) * RW;
-        qy0[c] = ((q / nrx) % nry) * ROWS;
-        qz[c] = q / (nrx * nry);
-    }
-
-    // acc[c][j][h]: (re, im) of coil 2 cp + h at cell j of region c, updated
-    // with packed FP32x2 multiply-adds (each component rounds as fmaf).
-    float2 acc[RPW][RW][2];
-#pragma unroll
-    for (int c = 0; c < RPW; c++)
-#pragma unroll
-        for (int j = 0; j < RW; j++) acc[c][j][0] = acc[c][j][1] = make_float2(0.f, 0.f);
-
-    // A tile no sample touches: its cells are zero (nothing to add when
-    // accumulating) -- one pass of coalesced stores, no staging.
-    if (it.begin == it.end && it.split < 0) {
-        if (a.accumulate) return;
-        const int cells = T0 * T1 * k.tile[2];
-        const int64_t ostep = (int64_t)a.F * a.kl.s_bf;
-        float2 *gbase = grid + ((int64_t)b0 * a.F + f) * a.kl.s_bf;
-        for (int e = threadIdx.x; e < cells; e += kThreads) {
-            const int x = e % T0, yz = e / T0, y = yz % T1, z = yz / T1;
-            float2 *o = gbase + (int64_t)(org2 + z) * a.kl.s_z + (int64_t)(org1 + y) * a.kl.s_y + org0 + x;
-            for (int c = 0; c < CG && b0 + c < a.nb; c++) {
-                *o = make_float2(0.f, 0.f);
-                o += ostep;
-            }
-        }
-        return;
-    }
-
-    const uint32_t bar[2] = {smem_u32(&s_bar[0]), smem_u32(&s_bar[1])};
-    if (threadIdx.x == 0) {
-        mbar_init(bar[0], 1);
-        mbar_init(bar[1], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    uint32_t phase = 0;   // bit s: parity of stage s's next barrier completion
-
-    // The pair rows of a chunk are contiguous (list order): thread 0 starts
-    // one bulk copy (TMA) of them into stage s.  Stage s was last read before
-    // the preceding __syncthreads; the proxy fence orders those reads before
-    // the asynchronous write.
-    auto issue_rows = [&](int s, int base, int cnt) {
-        if (threadIdx.x == 0) {
-            fence_proxy_async_smem();
-            const uint32_t bytes = (uint32_t)cnt * (uint32_t)PRF * 4u;
-            mbar_expect_tx(bar[s], bytes);
-            bulk_copy_g2s(smem_u32(stage_wt(s)), a.prows + (int64_t)base * PRF, bytes, bar[s]);
-        }
-    };
-
-    float2 pv[kVE];
-    float pd[kVE];
-    // values: lanes run along samples (one coil per load instruction)
-    auto prefetch = [&](int base, int cnt) {
-#pragma unroll
-        for (int q = 0; q < kVE; q++) {
-            const int e = threadIdx.x + q * kThreads;
-            const int i = e % kChunkR, c = e / kChunkR;
-            pv[q] = make_float2(0.f, 0.f);
-            pd[q] = 1.f;
-            if (e < kChunkR * CG && i < cnt && b0 + c < a.nb) {
-                const uint32_t si = a.list[base + i];
-                const bool need_j = a.layout == LAYOUT_ORIGINAL || a.dcw;
-                const uint32_t j = need_j ? a.perm[si] : si;
-                const int64_t idx = (a.layout == LAYOUT_SORTED) ? (int64_t)si : (int64_t)j;
-                pv[q] = samples[(int64_t)(b0 + c) * a.Mtot + idx];
-                if (a.dcw) pd[q] = a.dcw[j];
-            }
-        }
-    };
-    // Values of the prefetched chunk into stage s, density weights folded in.
-    auto stage_values = [&](int s) {
-        float2 *sv = stage_v(s);
-#pragma unroll
-        for (int q = 0; q < kVE; q++) {
-            const int e = threadIdx.x + q * kThreads;
-            if (e >= kChunkR * CG) break;
-            float2 v = pv[q];
-            if (a.dcw) {
-                v.x = pd[q] * v.x;
-                v.y = pd[q] * v.y;
-            }
-            sv[(e % kChunkR) * SVS + e / kChunkR] = v;
-        }
-    };
-
-    int cur = 0;
-    if (it.begin < it.end) {
-        const int cnt0 = min(kChunkR, it.end - it.begin);
-        issue_rows(0, it.begin, cnt0);
-        prefetch(it.begin, cnt0);
-        stage_values(0);
-    }
-    __syncthreads();
-    for (int base = it.begin; base < it.end; base += kChunkR) {
-        const int cnt = min(kChunkR, it.end - base);
-        const int nbase = base + kChunkR;
-        const int ncnt = nbase < it.end ? min(kChunkR, it.end - nbase) : 0;
-        if (ncnt > 0) {
-            issue_rows(cur ^ 1, nbase, ncnt);
-            prefetch(nbase, ncnt);
-        }
-        mbar_wait_bounded(bar[cur], (phase >> cur) & 1u, a.err);
-        phase ^= 1u << cur;
-        const float *wt = stage_wt(cur);
-        const float4 *sv4 = reinterpret_cast<const float4 *>(stage_v(cur));
-#pragma unroll
-        for (int c = 0; c < RPW; c++) {
-            const int ry = qy0[c] + row;
-#pragma unroll
-            for (int half = 0; half < kChunkR / 32; half++) {
-                const int il = half * 32 + lane;
-                bool hit = false;
-                if (il < cnt) {
-                    const uint4 r = *reinterpret_cast<const uint4 *>(wt + il * PRF + PRW);
-                    hit = (int)(r.x & 0xffffu) <= qx0[c] + RW - 1 && (int)(r.x >> 16) >= qx0[c] &&
-                          (int)(r.y & 0xffffu) <= qy0[c] + ROWS - 1 && (int)(r.y >> 16) >= qy0[c];
-                    if (D3) hit = hit && (int)(r.z & 0xffffu) <= qz[c] && (int)(r.z >> 16) >= qz[c];
-                }
-                uint32_t bits = __ballot_sync(0xffffffffu, hit);
-                while (bits) {
-                    const int i = half * 32 + __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    const float4 v = sv4[i * (SVS / 2) + cp];
-                    const float2 v0 = make_float2(v.x, v.y), v1 = make_float2(v.z, v.w);
-                    const float *wr = wt + i * PRF;
-                    float wyz = wr[T0 + ry];
-                    if (D3) wyz *= wr[T0 + T1 + qz[c]];
-                    const float2 wyz2 = make_float2(wyz, wyz);
-#pragma unroll
-                    for (int jj = 0; jj < RW / 4; jj++) {
-                        const float4 w4 = *reinterpret_cast<const float4 *>(wr + qx0[c] + 4 * jj);
-                        const float2 w01 = __fmul2_rn(make_float2(w4.x, w4.y), wyz2);
-                        const float2 w23 = __fmul2_rn(make_float2(w4.z, w4.w), wyz2);
-                        const float wj[4] = {w01.x, w01.y, w23.x, w23.y};
-#pragma unroll
-                        for (int m = 0; m < 4; m++) {
-                            const float2 wm = make_float2(wj[m], wj[m]);
-                            float2 *ac = acc[c][4 * jj + m];
-                            ac[0] = __ffma2_rn(wm, v0, ac[0]);
-                            ac[1] = __ffma2_rn(wm, v1, ac[1]);
-                        }
-                    }
-                }
-            }
-        }
-        if (ncnt > 0) stage_values(cur ^ 1);
-        __syncthreads();
-        cur ^= 1;
-    }
-
-    // The centring checkerboard (-1)^(gx+gy+gz) is a property of the output
-    // cell, so it is applied here rather than to every weight.
-    auto store = [&](int c, int j, float4 v) {
-        const int gx = org0 + qx0[c] + j, gy = org1 + qy0[c] + row, gz = org2 + qz[c];
-        const int64_t g = (int64_t)gz * a.kl.s_z + (int64_t)gy * a.kl.s_y + gx;
-        const float sgn = (a.sign_fold && ((gx + gy + gz) & 1)) ? -1.f : 1.f;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int q = 2 * cp + h;
-            if (b0 + q >= a.nb) break;
-            float2 *o = grid + ((int64_t)(b0 + q) * a.F + f) * a.kl.s_bf + g;
-            float2 w = h ? make_float2(sgn * v.z, sgn * v.w) : make_float2(sgn * v.x, sgn * v.y);
-            if (a.accumulate) { const float2 old = *o; w.x += old.x; w.y += old.y; }
-            *o = w;
-        }
-    };
-    // Writes the accumulators to the grid.  Through shared memory when the
-    // tile fits the stage buffers: lanes put their cells into a [coil][z][y][x]
-    // tile (rows padded by one cell, coil planes to 2 mod 8 cells: conflict-
-    // free), then threads store whole rows of one coil plane (coalesced).
-    // Every thread of the CTA calls it (it has a barrier).
-    auto epilogue = [&]() {
-        const int T2 = k.tile[2];
-        const int RS = T0 + 1, ZS = T1 * RS;
-        int PS = T2 * ZS;
-        PS += (10 - PS % 8) % 8;   // PS = 2 (mod 8)
-        if ((int64_t)CG * PS * 8 > 2 * (int64_t)stage_bytes) {
-#pragma unroll
-            for (int c = 0; c < RPW; c++)
-#pragma unroll
-                for (int j = 0; j < RW; j++)
-                    store(c, j, make_float4(acc[c][j][0].x, acc[c][j][0].y, acc[c][j][1].x, acc[c][j][1].y));
-            return;
-        }
-        float2 *tl = reinterpret_cast<float2 *>(g_rows_smem);
-#pragma unroll
-        for (int c = 0; c < RPW; c++)
-#pragma unroll
-            for (int j = 0; j < RW; j++) {
-                const int o = qz[c] * ZS + (qy0[c] + row) * RS + qx0[c] + j;
-                tl[(2 * cp) * PS + o] = acc[c][j][0];
-                tl[(2 * cp + 1) * PS + o] = acc[c][j][1];
-            }
-        __syncthreads();
-        const int x = threadIdx.x % T0, r0 = threadIdx.x / T0, rpp = kThreads / T0;
-        if (r0 >= rpp) return;
-        const int rows_c = T2 * T1;
-        const int gx = org0 + x;
-        for (int r = r0; r < rows_c; r += rpp) {
-            const int z = r / T1, y = r - z * T1;
-            const int gy = org1 + y, gz = org2 + z;
-            const float sgn = (a.sign_fold && ((gx + gy + gz) & 1)) ? -1.f : 1.f;
-            const int64_t cell = (int64_t)gz * a.kl.s_z + (int64_t)gy * a.kl.s_y + gx;
-            const float2 *src = tl + z * ZS + y * RS + x;
-            float2 *o = grid + ((int64_t)b0 * a.F + f) * a.kl.s_bf + cell;
-            const int64_t ostep = (int64_t)a.F * a.kl.s_bf;
-            for (int c = 0; c < CG && b0 + c < a.nb; c++) {
-                float2 v = src[c * PS];
-                v.x *= sgn;
-                v.y *= sgn;
-                if (a.accumulate) { const float2 old = *o; v.x += old.x; v.y += old.y; }
-                *o = v;
-                o += ostep;
-            }
-        }
-    };
-    if (it.split < 0) {
-        epilogue();
-        return;
-    }
-    // Split tile: write this chunk's partial tile, the last CTA sums the
-    // partials in chunk order.
-    const SplitInfo si = a.splits[it.split];
-    auto part = [&](int slot) -> float4 * {
-        return reinterpret_cast<float4 *>(a.partials + ((int64_t)slot * a.ncg + grp) * a.part_elems);
-    };
-    {
-        float4 *pp = part(si.first_slot + it.chunk);
-#pragma unroll
-        for (int c = 0; c < RPW; c++)
-#pragma unroll
-            for (int j = 0; j < RW; j++)
-                pp[(c * RW + j) * kThreads + threadIdx.x] =
-                    make_float4(acc[c][j][0].x, acc[c][j][0].y, acc[c][j][1].x, acc[c][j][1].y);
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int *ctr = a.counters + (int64_t)it.split * a.ncg + grp;
-        const unsigned int old = atomicAdd(ctr, 1u);
-        s_last = (old == (unsigned int)(si.nchunks - 1));
-        if (s_last) *ctr = 0u;   // ready for the next launch
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-#pragma unroll
-    for (int c = 0; c < RPW; c++)
-#pragma unroll
-        for (int j = 0; j < RW; j++) {
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int ch = 0; ch < si.nchunks; ch++) {
-                const float4 v = __ldcg(&part(si.first_slot + ch)[(c * RW + j) * kThreads + threadIdx.x]);
-                s.x += v.x;
-                s.y += v.y;
-                s.z += v.z;
-                s.w += v.w;
-            }
-            acc[c][j][0] = make_float2(s.x, s.y);
-            acc[c][j][1] = make_float2(s.z, s.w);
-        }
-    epilogue();
-}
-
-// ------------------------------------- NC2C, row variant, warp-specialized --
-//
-// The row variant for SORTED_IL samples (the E^H E workspace, where every
-// sample's coils are one contiguous row).  Nothing is staged through
-// registers: a producer warp (warp 8) streams each chunk's pair rows and
-// sample rows into a ring of kWsStages shared-memory stages with bulk copies
-// (cp.async.bulk), announcing the bytes on the stage's "full" mbarrier; the
-// eight consumer warps run the same region visits as k_grid_rows and release
-// a stage on its "empty" mbarrier (one arrival per warp) when done with it.
-// Warps never wait for each other inside the chunk loop, and the copies of
-// the next kWsStages - 1 chunks are in flight while a chunk is summed.  All
-// waits are bounded (err bit 0).  Same per-cell summation order as
-// k_grid_rows, so the result is bit-identical.
-
-constexpr int kWsStages = 4;
-constexpr int kWsThreads = kThreads + 32;   // 8 consumer warps + 1 producer warp
-constexpr int kWsMinBlocks = 2;             // resident CTAs per SM (96 registers a thread)
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-
-__host__ __device__ __forceinline__ int ws_stage_bytes(const KParams &k, int cg) {
-    return kChunkR * (pair_row_floats(k) * 4 + cg * 8);
-}
-
-template <int CG, int RW, int RPW, bool D3>
-__global__ void __launch_bounds__(kWsThreads, kWsMinBlocks)
-k_grid_rows_ws(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict__ grid) {
-    constexpr int CP = CG / 2;      // lanes per row: one per coil pair
-    constexpr int ROWS = 32 / CP;   // rows per region
-    extern __shared__ __align__(128) unsigned char g_ws_smem[];
-    __shared__ int s_last;
-    __shared__ __align__(8) unsigned long long s_full[kWsStages], s_empty[kWsStages];
-
-    const KParams &k = a.k;
-    const int grp = blockIdx.y;
-    const int b0 = grp * CG;
-    const WorkItem it = a.items[blockIdx.x];
-    const int f = it.ft / k.ntiles_total;
-    const int tile = it.ft - f * k.ntiles_total;
-    const int tx = tile % k.ntiles[0];
-    const int ty = (tile / k.ntiles[0]) % k.ntiles[1];
-    const int tz = tile / (k.ntiles[0] * k.ntiles[1]);
-    const int org0 = tx * k.tile[0], org1 = ty * k.tile[1], org2 = tz * k.tile[2];
-    const int T0 = k.tile[0], T1 = k.tile[1];
-    const int PRF = a.prow_floats;   // floats per pair row
-    const int PRW = PRF - 4;         // weight part; the last 4 words are the footprint ranges
-    const int stage_bytes = ws_stage_bytes(k, CG);
-    auto stage_wt = [&](int s) { return reinterpret_cast<float *>(g_ws_smem + s * stage_bytes); };
-    auto stage_v = [&](int s) {
-        return reinterpret_cast<float2 *>(g_ws_smem + s * stage_bytes + kChunkR * PRF * 4);
-    };
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool consumer = warp < 8;
-
-    // A tile no sample touches: zero stores, no staging.
-    if (it.begin == it.end && it.split < 0) {
-        if (a.accumulate) return;
-        const int cells = T0 * T1 * k.tile[2];
-        const int64_t ostep = (int64_t)a.F * a.kl.s_bf;
-        float2 *gbase = grid + ((int64_t)b0 * a.F + f) * a.kl.s_bf;
-        for (int e = threadIdx.x; e < cells; e += blockDim.x) {
-            const int x = e % T0, yz = e / T0, y = yz % T1, z = yz / T1;
-            float2 *o = gbase + (int64_t)(org2 + z) * a.kl.s_z + (int64_t)(org1 + y) * a.kl.s_y + org0 + x;
-            for (int c = 0; c < CG && b0 + c < a.nb; c++) {
-                *o = make_float2(0.f, 0.f);
-                o += ostep;
-            }
-        }
-        return;
-    }
-
-    if (threadIdx.x == 0) {
-        for (int st = 0; st < kWsStages; st++) {
-            mbar_init(smem_u32(&s_full[st]), 1);
-            mbar_init(smem_u32(&s_empty[st]), 8);
-        }
-        mbar_fence_init();
-    }
-    __syncthreads();
-    const int nchunks = (it.end - it.begin + kChunkR - 1) / kChunkR;
-
-    const int cp = lane % CP, row = lane / CP;
-    const int nrx = T0 / RW, nry = T1 / ROWS;
-    int qx0[RPW], qy0[RPW], qz[RPW];
-#pragma unroll
-    for (int c = 0; c < RPW; c++) {
-        const int q = (consumer ? warp : 0) + 8 * c;
-        qx0[c] = (q % nrx) * RW;
-        qy0[c] = ((q / nrx) % nry) * ROWS;
-        qz[c] = q / (nrx * nry);
-    }
-    float2 acc[RPW][RW][2];
-#pragma unroll
-    for (int c = 0; c < RPW; c++)
-#pragma unroll
-        for (int j = 0; j < RW; j++) acc[c][j][0] = acc[c][j][1] = make_float2(0.f, 0.f);
-
-    if (!consumer) {
-        // Producer: for chunk ch, stage ch % kWsStages once the consumers
-        // released its previous use; lane 0 announces all bytes (arrival +
-        // transaction count) and copies the pair rows, then every lane copies
-        // up to two sample rows (this coil group's columns).
-        const uint32_t vbytes = (uint32_t)min(CG, a.il_stride - b0) * 8u;
-        for (int ch = 0; ch < nchunks; ch++) {
-            const int st = ch % kWsStages;
-            const int use = ch / kWsStages;
-            const int base = it.begin + ch * kChunkR;
-            const int cnt = min(kChunkR, it.end - base);
-            const uint32_t si0 = lane < cnt ? a.list[base + lane] : 0u;
-            const uint32_t si1 = lane + 32 < cnt ? a.list[base + lane + 32] : 0u;
-            if (use > 0) mbar_wait_bounded(smem_u32(&s_empty[st]), (uint32_t)(use - 1) & 1u, a.err);
-            fence_proxy_async_smem();
-            const uint32_t full = smem_u32(&s_full[st]);
-            if (lane == 0) {
-                const uint32_t rbytes = (uint32_t)cnt * (uint32_t)PRF * 4u;
-                mbar_expect_tx(full, rbytes + (uint32_t)cnt * vbytes);
-                bulk_copy_g2s(smem_u32(stage_wt(st)), a.prows + (int64_t)base * PRF, rbytes, full);
-            }
-            __syncwarp();
-            float2 *sv = stage_v(st);
-            if (lane < cnt)
-                bulk_copy_g2s(smem_u32(sv + lane * CG), samples + (int64_t)si0 * a.il_stride + b0, vbytes, full);
-            if (lane + 32 < cnt)
-                bulk_copy_g2s(smem_u32(sv + (lane + 32) * CG), samples + (int64_t)si1 * a.il_stride + b0, vbytes,
-                              full);
-        }
-    } else {
-        for (int ch = 0; ch < nchunks; ch++) {
-            const int st = ch % kWsStages;
-            const int base = it.begin + ch * kChunkR;
-            const int cnt = min(kChunkR, it.end - base);
-            mbar_wait_bounded(smem_u32(&s_full[st]), (uint32_t)(ch / kWsStages) & 1u, a.err);
-            const float *wt = stage_wt(st);
-            const float4 *sv4 = reinterpret_cast<const float4 *>(stage_v(st));
-#pragma unroll
-            for (int c = 0; c < RPW; c++) {
-                const int ry = qy0[c] + row;
-#pragma unroll
-                for (int half = 0; half < kChunkR / 32; half++) {
-                    const int il = half * 32 + lane;
-                    bool hit = false;
-                    if (il < cnt) {
-                        const uint4 r = *reinterpret_cast<const uint4 *>(wt + il * PRF + PRW);
-                        hit = (int)(r.x & 0xffffu) <= qx0[c] + RW - 1 && (int)(r.x >> 16) >= qx0[c] &&
-                              (int)(r.y & 0xffffu) <= qy0[c] + ROWS - 1 && (int)(r.y >> 16) >= qy0[c];
-                        if (D3) hit = hit && (int)(r.z & 0xffffu) <= qz[c] && (int)(r.z >> 16) >= qz[c];
-                    }
-                    uint32_t bits = __ballot_sync(0xffffffffu, hit);
-                    while (bits) {
-                        const int i = half * 32 + __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        const float4 v = sv4[i * (CG / 2) + cp];
-                        const float2 v0 = make_float2(v.x, v.y), v1 = make_float2(v.z, v.w);
-                        const float *wr = wt + i * PRF;
-                        float wyz = wr[T0 + ry];
-                        if (D3) wyz *= wr[T0 + T1 + qz[c]];
-                        const float2 wyz2 = make_float2(wyz, wyz);
-#pragma unroll
-                        for (int jj = 0; jj < RW / 4; jj++) {
-                            const float4 w4 = *reinterpret_cast<const float4 *>(wr + qx0[c] + 4 * jj);
-                            const float2 w01 = __fmul2_rn(make_float2(w4.x, w4.y), wyz2);
-                            const float2 w23 = __fmul2_rn(make_float2(w4.z, w4.w), wyz2);
-                            const float wj[4] = {w01.x, w01.y, w23.x, w23.y};
-#pragma unroll
-                            for (int m = 0; m < 4; m++) {
-                                const float2 wm = make_float2(wj[m], wj[m]);
-                                float2 *ac = acc[c][4 * jj + m];
-                                ac[0] = __ffma2_rn(wm, v0, ac[0]);
-                                ac[1] = __ffma2_rn(wm, v1, ac[1]);
-                            }
-                        }
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&s_empty[st]));
-        }
-    }
-    __syncthreads();   // every stage consumed; every copy landed
-
-    auto store = [&](int c, int j, float4 v) {
-        const int gx = org0 + qx0[c] + j, gy = org1 + qy0[c] + row, gz = org2 + qz[c];
-        const int64_t g = (int64_t)gz * a.kl.s_z + (int64_t)gy * a.kl.s_y + gx;
-        const float sgn = (a.sign_fold && ((gx + gy + gz) & 1)) ? -1.f : 1.f;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int q = 2 * cp + h;
-            if (b0 + q >= a.nb) break;
-            float2 *o = grid + ((int64_t)(b0 + q) * a.F + f) * a.kl.s_bf + g;
-            float2 w = h ? make_float2(sgn * v.z, sgn * v.w) : make_float2(sgn * v.x, sgn * v.y);
-            if (a.accumulate) { const float2 old = *o; w.x += old.x; w.y += old.y; }
-            *o = w;
-        }
-    };
-    // Tile out through shared memory (as k_grid_rows), the stage ring as the
-    // staging area.  Every thread calls it (it has a barrier).
-    auto epilogue = [&]() {
-        const int T2 = k.tile[2];
-        const int RS = T0 + 1, ZS = T1 * RS;
-        int PS = T2 * ZS;
-        PS += (10 - PS % 8) % 8;   // PS = 2 (mod 8)
-        if ((int64_t)CG * PS * 8 > (int64_t)kWsStages * stage_bytes) {
-            if (consumer) {
-#pragma unroll
-                for (int c = 0; c < RPW; c++)
-#pragma unroll
-                    for (int j = 0; j < RW; j++)
-                        store(c, j, make_float4(acc[c][j][0].x, acc[c][j][0].y, acc[c][j][1].x, acc[c][j][1].y));
-            }
-            return;
-        }
-        float2 *tl = reinterpret_cast<float2 *>(g_ws_smem);
-        if (consumer) {
-#pragma unroll
-            for (int c = 0; c < RPW; c++)
-#pragma unroll
-                for (int j = 0; j < RW; j++) {
-                    const int o = qz[c] * ZS + (qy0[c] + row) * RS + qx0[c] + j;
-                    tl[(2 * cp) * PS + o] = acc[c][j][0];
-                    tl[(2 * cp + 1) * PS + o] = acc[c][j][1];
-                }
-        }
-        __syncthreads();
-        const int x = threadIdx.x % T0, r0 = threadIdx.x / T0, rpp = kThreads / T0;
-        if (r0 >= rpp) return;
-        const int rows_c = T2 * T1;
-        const int gx = org0 + x;
-        for (int r = r0; r < rows_c; r += rpp) {
-            const int z = r / T1, y = r - z * T1;
-            const int gy = org1 + y, gz = org2 + z;
-            const float sgn = (a.sign_fold && ((gx + gy + gz) & 1)) ? -1.f : 1.f;
-            const int64_t cell = (int64_t)gz * a.kl.s_z + (int64_t)gy * a.kl.s_y + gx;
-            const float2 *src = tl + z * ZS + y * RS + x;
-            float2 *o = grid + ((int64_t)b0 * a.F + f) * a.kl.s_bf + cell;
-            const int64_t ostep = (int64_t)a.F * a.kl.s_bf;
-            for (int c = 0; c < CG && b0 + c < a.nb; c++) {
-                float2 v = src[c * PS];
-                v.x *= sgn;
-                v.y *= sgn;
-                if (a.accumulate) { const float2 old = *o; v.x += old.x; v.y += old.y; }
-                *o = v;
-                o += ostep;
-            }
-        }
-    };
-    if (it.split < 0) {
-        epilogue();
-        return;
-    }
-    // Split tile: write this chunk's partial tile, the last CTA sums the
-    // partials in chunk order.
-    const SplitInfo si = a.splits[it.split];
-    auto part = [&](int slot) -> float4 * {
-        return reinterpret_cast<float4 *>(a.partials + ((int64_t)slot * a.ncg + grp) * a.part_elems);
-    };
-    if (consumer) {
-        float4 *pp = part(si.first_slot + it.chunk);
-#pragma unroll
-        for (int c = 0; c < RPW; c++)
-#pragma unroll
-            for (int j = 0; j < RW; j++)
-                pp[(c * RW + j) * kThreads + threadIdx.x] =
-                    make_float4(acc[c][j][0].x, acc[c][j][0].y, acc[c][j][1].x, acc[c][j][1].y);
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int *ctr = a.counters + (int64_t)it.split * a.ncg + grp;
-        const unsigned int old = atomicAdd(ctr, 1u);
-        s_last = (old == (unsigned int)(si.nchunks - 1));
-        if (s_last) *ctr = 0u;   // ready for the next launch
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (consumer) {
-#pragma unroll
-        for (int c = 0; c < RPW; c++)
-#pragma unroll
-            for (int j = 0; j < RW; j++) {
-                float4 sm = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int ch = 0; ch < si.nchunks; ch++) {
-                    const float4 v = __ldcg(&part(si.first_slot + ch)[(c * RW + j) * kThreads + threadIdx.x]);
-                    sm.x += v.x;
-                    sm.y += v.y;
-                    sm.z += v.z;
-                    sm.w += v.w;
-                }
-                acc[c][j][0] = make_float2(sm.x, sm.y);
-                acc[c][j][1] = make_float2(sm.z, sm.w);
-            }
-    }
-    epilogue();
-}
-
-// ---------------------- NC2C, row variant, warp-specialized, persistent --
-//
-// k_grid_rows_ws as one persistent launch over every work unit (gridding
-// item x coil group) of all frames: kWsMinBlocks CTAs per SM take units from
-// a global counter (units in list order: split chunks of heavy tiles first),
-// and the producer warp streams chunk after chunk across unit boundaries, so
-// the copy pipeline does not drain between tiles and no CTA pays a launch
-// ramp per tile.  Every stage carries a descriptor of its chunk (unit, sample
-// count, first/last flags); the consumer warps zero their accumulators on a
-// unit's first chunk and write the tile out after its last one, through a
-// tile buffer of their own (the producer keeps filling stages meanwhile),
-// synchronising only among themselves (an mbarrier of the 256 consumer
-// threads).  No CTA waits for another; the last CTA to finish resets the
-// counter for the next launch.  Every wait is bounded: a wait that runs out
-// sets err bit 0 and the CTA's bail flag, after which every wait of the CTA
-// returns at once, both loops end, and the producer waits (bounded) for its
-// copies still in flight before the CTA exits.  Per-cell summation order as
-// k_grid_rows: the result is bit-identical.
-
-struct WspDesc {
-    int ft, split, chunk, grp;
-    int cnt, flags, pad0, pad1;
-};
-constexpr int kWspFirst = 1, kWspLast = 2, kWspDone = 4, kWspEmpty = 8;
-
-// Bounded wait that reports whether the phase completed.  It gives up after
-// ~2 s (err bit 0 and *bail set) or as soon as *bail is set (bail may be null).
-__device__ __forceinline__ bool mbar_wait_ok(uint32_t bar, uint32_t parity, unsigned int *err, int *bail) {
-    for (int round = 0; round < 2; round++) {
-        for (uint32_t i = 0; i < (1u << 22); i++) {
-            if (mbar_try_wait(bar, parity)) return true;
-            if (bail && *reinterpret_cast<volatile int *>(bail)) return false;
-            if (i >= 16) __nanosleep(256);
-        }
-    }
-    if (err) atomicOr(err, 1u);
-    if (bail) *reinterpret_cast<volatile int *>(bail) = 1;
-    return false;
-}
-
-// Epilogue tile of the persistent kernel: [coil][z][y][x], rows padded by
-// one cell, coil planes at 2 (mod 8) cells (conflict-free transposition).
-__host__ __device__ __forceinline__ int wsp_plane_cells(const KParams &k) {
-    const int ps = k.tile[2] * k.tile[1] * (k.tile[0] + 1);
-    return ps + (10 - ps % 8) % 8;
-}
-__host__ __device__ __forceinline__ int wsp_smem_bytes(const KParams &k, int cg) {
-    return kWsStages * ws_stage_bytes(k, cg) + cg * wsp_plane_cells(k) * 8;
-}
-
-template <int CG, int RW, int RPW, bool D3>
-__global__ void __launch_bounds__(kWsThreads, kWsMinBlocks)
-k_grid_rows_wsp(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict__ grid) {
-    constexpr int CP = CG / 2;      // lanes per row: one per coil pair
-    constexpr int ROWS = 32 / CP;   // rows per region
-    extern __shared__ __align__(128) unsigned char g_wsp_smem[];
-    __shared__ int s_last, s_bail;
-    __shared__ __align__(8) unsigned long long s_full[kWsStages], s_empty[kWsStages], s_cons[2];
-    __shared__ WspDesc s_desc[kWsStages];
-
-    const KParams &k = a.k;
-    const int T0 = k.tile[0], T1 = k.tile[1], T2 = k.tile[2];
-    const int PRF = a.prow_floats;   // floats per pair row
-    const int PRW = PRF - 4;         // weight part; the last 4 words are the footprint ranges
-    const int stage_bytes = ws_stage_bytes(k, CG);
-    auto stage_wt = [&](int s) { return reinterpret_cast<float *>(g_wsp_smem + s * stage_bytes); };
-    auto stage_v = [&](int s) {
-        return reinterpret_cast<float2 *>(g_wsp_smem + s * stage_bytes + kChunkR * PRF * 4);
-    };
-    float2 *tl = reinterpret_cast<float2 *>(g_wsp_smem + kWsStages * stage_bytes);
-    const int PS = wsp_plane_cells(k);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool consumer = warp < 8;
-
-    if (threadIdx.x == 0) {
-        for (int st = 0; st < kWsStages; st++) {
-            mbar_init(smem_u32(&s_full[st]), 1);
-            mbar_init(smem_u32(&s_empty[st]), 8);
-        }
-        mbar_init(smem_u32(&s_cons[0]), kThreads);
-        mbar_init(smem_u32(&s_cons[1]), kThreads);
-        mbar_fence_init();
-        s_bail = 0;
-    }
-    __syncthreads();
-
-    if (!consumer) {
-        // Producer: takes units from the counter (the next one is fetched
-        // while the current one's chunks are issued); for chunk g of the
-        // CTA's sequence, stage g % kWsStages once the consumers released its
-        // previous use: lane 0 writes the descriptor, announces the bytes
-        // (arrival + transaction count) and copies the pair rows, then every
-        // lane copies up to two sample rows (this coil group's columns).  A
-        // last descriptor flagged kWspDone ends the consumers' loop.
-        const int ncg = a.ncg;
-        uint32_t g = 0;
-        int w = 0;
-        if (lane == 0) w = (int)atomicAdd(&a.queue[0], 1u);
-        w = __shfl_sync(0xffffffffu, w, 0);
-        bool bail = false;
-        while (!bail) {
-            const bool done = w >= a.n_work;
-            int wn = w;
-            if (!done) {
-                if (lane == 0) wn = (int)atomicAdd(&a.queue[0], 1u);
-                wn = __shfl_sync(0xffffffffu, wn, 0);
-            }
-            WorkItem it{};
-            int grp = 0;
-            if (!done) {
-                it = a.items[w / ncg];
-                grp = w - (w / ncg) * ncg;
-            }
-            const int b0 = grp * CG;
-            const int n = done ? 0 : it.end - it.begin;
-            const uint32_t vbytes = n > 0 ? (uint32_t)min(CG, a.il_stride - b0) * 8u : 0u;
-            const int nch = n > 0 ? (n + kChunkR - 1) / kChunkR : 1;
-            for (int ch = 0; ch < nch; ch++, g++) {
-                const int st = (int)(g % kWsStages);
-                const uint32_t use = g / kWsStages;
-                const int base = it.begin + ch * kChunkR;
-                const int cnt = n > 0 ? min(kChunkR, it.end - base) : 0;
-                const uint32_t si0 = lane < cnt ? a.list[base + lane] : 0u;
-                const uint32_t si1 = lane + 32 < cnt ? a.list[base + lane + 32] : 0u;
-                if (use > 0 && !mbar_wait_ok(smem_u32(&s_empty[st]), (use - 1) & 1u, a.err, &s_bail)) bail = true;
-                if (*reinterpret_cast<volatile int *>(&s_bail)) bail = true;
-                if (bail) break;
-                const uint32_t full = smem_u32(&s_full[st]);
-                if (lane == 0) {
-                    WspDesc d;
-                    d.ft = it.ft;
-                    d.split = it.split;
-                    d.chunk = it.chunk;
-                    d.grp = grp;
-                    d.cnt = cnt;
-                    d.flags = (ch == 0 ? kWspFirst : 0) | (ch == nch - 1 ? kWspLast : 0) | (done ? kWspDone : 0) |
-                              (n == 0 ? kWspEmpty : 0);
-                    d.pad0 = d.pad1 = 0;
-                    s_desc[st] = d;
-                }
-                fence_proxy_async_smem();
-                if (lane == 0) {
-                    const uint32_t rbytes = (uint32_t)cnt * (uint32_t)PRF * 4u;
-                    if (cnt > 0) {
-                        mbar_expect_tx(full, rbytes + (uint32_t)cnt * vbytes);
-                        bulk_copy_g2s(smem_u32(stage_wt(st)), a.prows + (int64_t)base * PRF, rbytes, full);
-                    } else {
-                        mbar_arrive(full);
-                    }
-                }
-                __syncwarp();
-                float2 *sv = stage_v(st);
-                if (lane < cnt)
-                    bulk_copy_g2s(smem_u32(sv + lane * CG), samples + (int64_t)si0 * a.il_stride + b0, vbytes, full);
-                if (lane + 32 < cnt)
-                    bulk_copy_g2s(smem_u32(sv + (lane + 32) * CG), samples + (int64_t)si1 * a.il_stride + b0,
-                                  vbytes, full);
-            }
-            if (done) break;
-            w = wn;
-        }
-        if (bail) {
-            // the consumers stopped early: wait for the copies still in flight
-            for (uint32_t gi = g > kWsStages ? g - kWsStages : 0; gi < g; gi++)
-                mbar_wait_ok(smem_u32(&s_full[gi % kWsStages]), (gi / kWsStages) & 1u, nullptr, nullptr);
-        }
-    } else {
-        const int cp = lane % CP, row = lane / CP;
-        const int nrx = T0 / RW, nry = T1 / ROWS;
-        int qx0[RPW], qy0[RPW], qz[RPW];
-#pragma unroll
-        for (int c = 0; c < RPW; c++) {
-            const int q = warp + 8 * c;
-            qx0[c] = (q % nrx) * RW;
-            qy0[c] = ((q / nrx) % nry) * ROWS;
-            qz[c] = q / (nrx * nry);
-        }
-        float2 acc[RPW][RW][2];
-#pragma unroll
-        for (int c = 0; c < RPW; c++)
-#pragma unroll
-            for (int j = 0; j < RW; j++) acc[c][j][0] = acc[c][j][1] = make_float2(0.f, 0.f);
-
-        // Barrier of the 256 consumer threads (every thread arrives: its
-        // shared-memory writes are released to the others).
-        uint32_t ncs = 0;
-        auto consumer_bar = [&]() {
-            const uint32_t b = smem_u32(&s_cons[ncs & 1u]);
-            mbar_arrive(b);
-            mbar_wait_ok(b, (ncs >> 1) & 1u, a.err, &s_bail);
-            ncs++;
-        };
-        // Tile out through the tile buffer: lanes put their cells into the
-        // [coil][z][y][x] tile, then the 256 consumer threads store whole rows
-        // of one coil plane (coalesced).
-        auto epilogue = [&](int f, int org0, int org1, int org2, int b0) {
-            const int RS = T0 + 1, ZS = T1 * RS;
-            consumer_bar();   // the previous tile has left the buffer
-#pragma unroll
-            for (int c = 0; c < RPW; c++)
-#pragma unroll
-                for (int j = 0; j < RW; j++) {
-                    const int o = qz[c] * ZS + (qy0[c] + row) * RS + qx0[c] + j;
-                    tl[(2 * cp) * PS + o] = acc[c][j][0];
-                    tl[(2 * cp + 1) * PS + o] = acc[c][j][1];
-                }
-            consumer_bar();
-            const int x = threadIdx.x % T0, r0 = threadIdx.x / T0, rpp = kThreads / T0;
-            if (r0 >= rpp) return;
-            const int rows_c = T2 * T1;
-            const int gx = org0 + x;
-            const int64_t ostep = (int64_t)a.F * a.kl.s_bf;
-            for (int r = r0; r < rows_c; r += rpp) {
-                const int z = r / T1, y = r - z * T1;
-                const int gy = org1 + y, gz = org2 + z;
-                const float sgn = (a.sign_fold && ((gx + gy + gz) & 1)) ? -1.f : 1.f;
-                const int64_t cell = (int64_t)gz * a.kl.s_z + (int64_t)gy * a.kl.s_y + gx;
-                const float2 *src = tl + z * ZS + y * RS + x;
-                float2 *o = grid + ((int64_t)b0 * a.F + f) * a.kl.s_bf + cell;
-                for (int c = 0; c < CG && b0 + c < a.nb; c++) {
-                    float2 v = src[c * PS];
-                    v.x *= sgn;
-                    v.y *= sgn;
-                    if (a.accumulate) { const float2 old = *o; v.x += old.x; v.y += old.y; }
-                    *o = v;
-                    o += ostep;
-                }
-            }
-        };
-
-        uint32_t g = 0;
-        for (;;) {
-            const int st = (int)(g % kWsStages);
-            if (!mbar_wait_ok(smem_u32(&s_full[st]), (g / kWsStages) & 1u, a.err, &s_bail)) break;
-            const WspDesc d = s_desc[st];
-            if (d.flags & kWspDone) break;
-            if (d.flags & kWspFirst) {
-#pragma unroll
-                for (int c = 0; c < RPW; c++)
-#pragma unroll
-                    for (int j = 0; j < RW; j++) acc[c][j][0] = acc[c][j][1] = make_float2(0.f, 0.f);
-            }
-            const int cnt = d.cnt;
-            const float *wt = stage_wt(st);
-            const float4 *sv4 = reinterpret_cast<const float4 *>(stage_v(st));
-#pragma unroll
-            for (int c = 0; c < RPW; c++) {
-                const int ry = qy0[c] + row;
-#pragma unroll
-                for (int half = 0; half < kChunkR / 32; half++) {
-                    const int il = half * 32 + lane;
-                    bool hit = false;
-                    if (il < cnt) {
-                        const uint4 r = *reinterpret_cast<const uint4 *>(wt + il * PRF + PRW);
-                        hit = (int)(r.x & 0xffffu) <= qx0[c] + RW - 1 && (int)(r.x >> 16) >= qx0[c] &&
-                              (int)(r.y & 0xffffu) <= qy0[c] + ROWS - 1 && (int)(r.y >> 16) >= qy0[c];
-                        if (D3) hit = hit && (int)(r.z & 0xffffu) <= qz[c] && (int)(r.z >> 16) >= qz[c];
-                    }
-                    uint32_t bits = __ballot_sync(0xffffffffu, hit);
-                    while (bits) {
-                        const int i = half * 32 + __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        const float4 v = sv4[i * (CG / 2) + cp];
-                        const float2 v0 = make_float2(v.x, v.y), v1 = make_float2(v.z, v.w);
-                        const float *wr = wt + i * PRF;
-                        float wyz = wr[T0 + ry];
-                        if (D3) wyz *= wr[T0 + T1 + qz[c]];
-                        const float2 wyz2 = make_float2(wyz, wyz);
-#pragma unroll
-                        for (int jj = 0; jj < RW / 4; jj++) {
-                            const float4 w4 = *reinterpret_cast<const float4 *>(wr + qx0[c] + 4 * jj);
-                            const float2 w01 = __fmul2_rn(make_float2(w4.x, w4.y), wyz2);
-                            const float2 w23 = __fmul2_rn(make_float2(w4.z, w4.w), wyz2);
-                            const float wj[4] = {w01.x, w01.y, w23.x, w23.y};
-#pragma unroll
-                            for (int m = 0; m < 4; m++) {
-                                const float2 wm = make_float2(wj[m], wj[m]);
-                                float2 *ac = acc[c][4 * jj + m];
-                                ac[0] = __ffma2_rn(wm, v0, ac[0]);
-                                ac[1] = __ffma2_rn(wm, v1, ac[1]);
-                            }
-                        }
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&s_empty[st]));
-            g++;
-            if (!(d.flags & kWspLast)) continue;
-
-            // The unit's tile is complete in the accumulators.
-            const int f = d.ft / k.ntiles_total;
-            const int tile = d.ft - f * k.ntiles_total;
-            const int tx = tile % k.ntiles[0];
-            const int ty = (tile / k.ntiles[0]) % k.ntiles[1];
-            const int tz = tile / (k.ntiles[0] * k.ntiles[1]);
-            const int org0 = tx * T0, org1 = ty * T1, org2 = tz * T2;
-            const int b0 = d.grp * CG;
-            if (d.split < 0) {
-                if (!((d.flags & kWspEmpty) && a.accumulate)) epilogue(f, org0, org1, org2, b0);
-                continue;
-            }
-            // Split tile: write this chunk's partial tile, the last CTA to
-            // finish one sums the partials in chunk order.
-            const SplitInfo si = a.splits[d.split];
-            auto part = [&](int slot) -> float4 * {
-                return reinterpret_cast<float4 *>(a.partials + ((int64_t)slot * a.ncg + d.grp) * a.part_elems);
-            };
-            {
-                float4 *pp = part(si.first_slot + d.chunk);
-#pragma unroll
-                for (int c = 0; c < RPW; c++)
-#pragma unroll
-                    for (int j = 0; j < RW; j++)
-                        pp[(c * RW + j) * kThreads + threadIdx.x] =
-                            make_float4(acc[c][j][0].x, acc[c][j][0].y, acc[c][j][1].x, acc[c][j][1].y);
-            }
-            __threadfence();
-            consumer_bar();
-            if (threadIdx.x == 0) {
-                unsigned int *ctr = a.counters + (int64_t)d.split * a.ncg + d.grp;
-                const unsigned int old = atomicAdd(ctr, 1u);
-                s_last = (old == (unsigned int)(si.nchunks - 1));
-                if (s_last) *ctr = 0u;   // ready for the next launch
-            }
-            consumer_bar();
-            if (!*reinterpret_cast<volatile int *>(&s_last)) continue;
-            __threadfence();
-#pragma unroll
-            for (int c = 0; c < RPW; c++)
-#pragma unroll
-                for (int j = 0; j < RW; j++) {
-                    float4 sm = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int ch = 0; ch < si.nchunks; ch++) {
-                        const float4 v = __ldcg(&part(si.first_slot + ch)[(c * RW + j) * kThreads + threadIdx.x]);
-                        sm.x += v.x;
-                        sm.y += v.y;
-                        sm.z += v.z;
-                        sm.w += v.w;
-                    }
-                    acc[c][j][0] = make_float2(sm.x, sm.y);
-                    acc[c][j][1] = make_float2(sm.z, sm.w);
-                }
-            epilogue(f, org0, org1, org2, b0);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned int old = atomicAdd(&a.queue[1], 1u);
-        if (old == gridDim.x - 1) {   // every CTA has taken its last unit
-            a.queue[0] = 0u;
-            a.queue[1] = 0u;
-            __threadfence();
-        }
-    }
-}
-
 // ------------------------------------------ reference fold (3D, opt-in) --
 //
 // GB_FLAG_REFERENCE_FOLD.  The reference grids onto a padded grid and folds
@@ -1547,11 +486,7 @@ k_degrid_c2nc(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__ 
     const WorkItem it = a.items[blockIdx.x];
     const int grp = blockIdx.y;
     const int b0 = grp * CG;
-    const int f = it.ft / k.ntiles_total;
-    const int tile = it.ft - f * k.ntiles_total;
-    const int tx = tile % k.ntiles[0];
-    const int ty = (tile / k.ntiles[0]) % k.ntiles[1];
-    const int tz = tile / (k.ntiles[0] * k.ntiles[1]);
+    const int f = it.f, tx = it.tx, ty = it.ty, tz = it.tz;
     const int org[3] = {tx * k.tile[0], ty * k.tile[1], tz * k.tile[2]};
     const int R0 = region_dim(k, 0), R1 = region_dim(k, 1), R2 = region_dim(k, 2);
     const int cellsR = R0 * R1 * R2;
@@ -1734,7 +669,11 @@ k_degrid_c2nc(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__ 
 #pragma unroll
                 for (int c = 0; c < CPL; c++) {
                     const int coil = b0 + ll * CPL + c;
-                    if (coil >= a.nb) break;
+                    if (coil >= a.nb) {
+                        if (a.layout == LAYOUT_SORTED_IL && coil < a.il_stride)   // the row's padding
+                            out[idx * a.il_stride + coil] = make_float2(0.f, 0.f);
+                        break;
+                    }
                     float2 val = make_float2(acc[c][0], acc[c][1]);
                     if (a.dcw) {
                         if (a.dcw_pow == 2) {
@@ -1920,7 +859,11 @@ __device__ __forceinline__ void degrid_table_passes(const ConvArgs &a, const Wor
 #pragma unroll
             for (int c = 0; c < CPL; c++) {
                 const int coil = b0 + ll * CPL + c;
-                if (coil >= a.nb) break;
+                if (coil >= a.nb) {
+                    if (a.layout == LAYOUT_SORTED_IL && coil < a.il_stride)   // the row's padding
+                        out[idx * a.il_stride + coil] = make_float2(0.f, 0.f);
+                    break;
+                }
                 float2 val = acc[c];
                 if (a.dcw) {
                     if (a.dcw_pow == 2) {
@@ -1956,11 +899,7 @@ k_degrid_table(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__
     const WorkItem it = a.items[blockIdx.x];
     const int grp = blockIdx.y;
     const int b0 = grp * CG;
-    const int f = it.ft / k.ntiles_total;
-    const int tile = it.ft - f * k.ntiles_total;
-    const int tx = tile % k.ntiles[0];
-    const int ty = (tile / k.ntiles[0]) % k.ntiles[1];
-    const int tz = tile / (k.ntiles[0] * k.ntiles[1]);
+    const int f = it.f, tx = it.tx, ty = it.ty, tz = it.tz;
     const int org0 = tx * k.tile[0], org1 = ty * k.tile[1], org2 = tz * k.tile[2];
     const int R0 = region_dim(k, 0), R1 = region_dim(k, 1), R2 = region_dim(k, 2);
     const int h2 = D3 ? k.hw : 0;
@@ -2043,8 +982,8 @@ static ConvArgs make_args(NufftPlan &p, int nb, SampleLayout layout, const float
     a.wtab = p.wtab.get();
     a.kl = klayout_standard(p.kp);
     a.prows = p.pair_rows.get();
+    a.prng = p.pair_rng.get();
     a.prow_floats = p.pair_row_stride;
-    a.err = p.err_flag.get();
     a.perm = p.perm.get();
     a.Mtot = p.Mtot;
     a.F = (int)p.F;
@@ -2059,55 +998,25 @@ static ConvArgs make_args(NufftPlan &p, int nb, SampleLayout layout, const float
     return a;
 }
 
-static int choose_cg(int requested, int nb) {
+int choose_cg(int requested, int nb) {
     int cg = requested;
     if (cg != 1 && cg != 2 && cg != 4 && cg != 8 && cg != 16) cg = 8;
     while (cg > 1 && cg / 2 >= nb) cg /= 2;
     return cg;
 }
 
-// Which gridding kernel runs for a plan and batch count, with its coil group
-// and the size of one CTA's partial tile (split tiles).
-struct GridCfg {
-    bool rows;        // k_grid_rows (else k_grid_nc2c)
-    int cg;
-    int rw, rpw;      // row variant: columns per lane, regions per warp
-    int cpt;          // cell variant: cells per thread
-    int ncg;
-    int64_t part_elems;
-    int smem;         // dynamic shared memory (row variant)
-};
-
 static GridCfg grid_config(const NufftPlan &p, int nb) {
     const KParams &k = p.kp;
     GridCfg c{};
     const int cells = k.tile[0] * k.tile[1] * k.tile[2];
     c.cpt = (cells + kThreads - 1) / kThreads;
-    const bool comp = (p.flags & GB_FLAG_COMPENSATED) != 0;
-    int cg = choose_cg(p.tiling.cg, nb);
-    if (!comp && k.D >= 2 && (cg == 8 || cg == 16) && p.pair_row_stride > 0 &&
-        p.pair_row_stride == pair_row_floats(k)) {
-        const int rows = 64 / cg;
-        const int smem = 2 * row_stage_bytes(k, cg);
-        if (k.tile[1] % rows == 0 && smem <= 96 * 1024) {
-            for (int rw = 4; rw <= 8 && !c.rows; rw *= 2) {
-                if (k.tile[0] % rw) continue;
-                const int regions = cells / (rows * rw);
-                if (regions % 8) continue;
-                const int rpw = regions / 8;
-                if ((rpw == 1 || rpw == 2 || rpw == 4) && rpw * rw <= 16) {
-                    c.rows = true;
-                    c.rw = rw;
-                    c.rpw = rpw;
-                    c.smem = smem;
-                }
-            }
-        }
+    if (!brick_config(p, nb, c)) {
+        const bool comp = (p.flags & GB_FLAG_COMPENSATED) != 0;
+        c.cg = choose_cg(p.tiling.cg, nb);
+        if (c.cpt * c.cg > (comp ? 16 : 32)) c.cg = std::max(1, (comp ? 16 : 32) / c.cpt);
     }
-    if (!c.rows && c.cpt * cg > (comp ? 16 : 32)) cg = std::max(1, (comp ? 16 : 32) / c.cpt);
-    c.cg = cg;
-    c.ncg = (nb + cg - 1) / cg;
-    c.part_elems = (int64_t)cg * (c.rows ? cells : kThreads * c.cpt);
+    c.ncg = (nb + c.cg - 1) / c.cg;
+    c.part_elems = (int64_t)c.cg * (c.brick ? cells : kThreads * c.cpt);
     return c;
 }
 
@@ -2127,134 +1036,12 @@ static void grid_dispatch_cpt(int cpt, const ConvArgs &a, dim3 g, const float2 *
     }
 }
 
-template <int CG, int RW, int RPW, bool D3>
-static void grid_rows_launch(const ConvArgs &a, dim3 g, int smem, const float2 *s, float2 *o, cudaStream_t st) {
-    auto kern = k_grid_rows<CG, RW, RPW, D3>;
-    if (smem > 48 * 1024)
-        GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kern<<<g, kThreads, smem, st>>>(a, s, o); ::gb::note_launch();
-}
-
-template <int CG, int RW, int RPW, bool D3>
-static void grid_rows_ws_launch(const ConvArgs &a, dim3 g, const float2 *s, float2 *o, cudaStream_t st) {
-    auto kern = k_grid_rows_ws<CG, RW, RPW, D3>;
-    const int smem = kWsStages * ws_stage_bytes(a.k, CG);
-    if (smem > 48 * 1024)
-        GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kern<<<g, kWsThreads, smem, st>>>(a, s, o); ::gb::note_launch();
-}
-
-template <int CG, bool D3>
-static void grid_rows_ws_shape(const GridCfg &c, const ConvArgs &a, dim3 g, const float2 *s, float2 *o,
-                               cudaStream_t st) {
-    if (c.rw == 4 && c.rpw == 1) grid_rows_ws_launch<CG, 4, 1, D3>(a, g, s, o, st);
-    else if (c.rw == 4 && c.rpw == 2) grid_rows_ws_launch<CG, 4, 2, D3>(a, g, s, o, st);
-    else if (c.rw == 4 && c.rpw == 4) grid_rows_ws_launch<CG, 4, 4, D3>(a, g, s, o, st);
-    else if (c.rw == 8 && c.rpw == 1) grid_rows_ws_launch<CG, 8, 1, D3>(a, g, s, o, st);
-    else if (c.rw == 8 && c.rpw == 2) grid_rows_ws_launch<CG, 8, 2, D3>(a, g, s, o, st);
-    else fail(GB_ERR_INTERNAL, "unsupported gridding region shape");
-}
-
-template <int CG, int RW, int RPW, bool D3>
-static void grid_rows_wsp_launch(const ConvArgs &a, const float2 *s, float2 *o, cudaStream_t st) {
-    auto kern = k_grid_rows_wsp<CG, RW, RPW, D3>;
-    const int smem = wsp_smem_bytes(a.k, CG);
-    // resident CTAs per SM for this shared-memory size (cached per instantiation)
-    static int cached_smem = -1, cached_ctas = 0;
-    if (smem != cached_smem) {
-        GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        int dev = 0, sms = 0, per_sm = 0;
-        GB_CUDA(cudaGetDevice(&dev));
-        GB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWsThreads, smem));
-        cached_ctas = std::max(1, per_sm) * sms;
-        cached_smem = smem;
-    }
-    const int ctas = std::max(1, std::min(a.n_work, cached_ctas));
-    kern<<<ctas, kWsThreads, smem, st>>>(a, s, o); ::gb::note_launch();
-}
-
-template <int CG, bool D3>
-static void grid_rows_wsp_shape(const GridCfg &c, const ConvArgs &a, const float2 *s, float2 *o, cudaStream_t st) {
-    if (c.rw == 4 && c.rpw == 1) grid_rows_wsp_launch<CG, 4, 1, D3>(a, s, o, st);
-    else if (c.rw == 4 && c.rpw == 2) grid_rows_wsp_launch<CG, 4, 2, D3>(a, s, o, st);
-    else if (c.rw == 4 && c.rpw == 4) grid_rows_wsp_launch<CG, 4, 4, D3>(a, s, o, st);
-    else if (c.rw == 8 && c.rpw == 1) grid_rows_wsp_launch<CG, 8, 1, D3>(a, s, o, st);
-    else if (c.rw == 8 && c.rpw == 2) grid_rows_wsp_launch<CG, 8, 2, D3>(a, s, o, st);
-    else fail(GB_ERR_INTERNAL, "unsupported gridding region shape");
-}
-
-template <int CG, bool D3>
-static void grid_rows_shape(const GridCfg &c, const ConvArgs &a, dim3 g, const float2 *s, float2 *o,
-                            cudaStream_t st) {
-    if (c.rw == 4 && c.rpw == 1) grid_rows_launch<CG, 4, 1, D3>(a, g, c.smem, s, o, st);
-    else if (c.rw == 4 && c.rpw == 2) grid_rows_launch<CG, 4, 2, D3>(a, g, c.smem, s, o, st);
-    else if (c.rw == 4 && c.rpw == 4) grid_rows_launch<CG, 4, 4, D3>(a, g, c.smem, s, o, st);
-    else if (c.rw == 8 && c.rpw == 1) grid_rows_launch<CG, 8, 1, D3>(a, g, c.smem, s, o, st);
-    else if (c.rw == 8 && c.rpw == 2) grid_rows_launch<CG, 8, 2, D3>(a, g, c.smem, s, o, st);
-    else fail(GB_ERR_INTERNAL, "unsupported gridding region shape");
-}
-
-// How E^H E grids its own (tile-ordered) samples.
-//   SCHED_ROWS: k_grid_rows on the SORTED workspace, one CTA per work item;
-//   SCHED_WS:   k_grid_rows_ws on the interleaved workspace, one CTA per item;
-//   SCHED_WSP:  k_grid_rows_wsp on the interleaved workspace, one persistent
-//               launch over a work queue.
-// The per-item warp-specialized kernel wins when the launch is a few waves
-// deep: its 4-stage copy pipeline hides the staging latency that dominates a
-// short launch (CG-SENSE 256^2 x 16 coils: 1082 CTAs, 1.25 -> 1.19 ms per
-// recon).  On launches many waves deep the register-staged kernel's higher
-// occupancy (3 CTAs of 8 warps per SM against 2 of 8 + 1) beats it (64 uneven
-// frames x 12 coils: 42.0 against 45.5 ms per batch); the persistent kernel
-// takes those launches.
-enum GridSched { SCHED_ROWS = 0, SCHED_WS = 1, SCHED_WSP = 2 };
-constexpr int kWsMaxWaves = 8;
-
-static GridSched normal_grid_sched(const NufftPlan &p, const GridCfg &c) {
-    if (!c.rows) return SCHED_ROWS;
-    int sms = 0;
-    GB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device));
-    const int64_t ctas = (int64_t)p.n_grd_items * c.ncg;
-    const bool shallow = ctas <= (int64_t)kWsMaxWaves * kWsMinBlocks * sms;
-    const bool wsp_fits = (int64_t)wsp_smem_bytes(p.kp, c.cg) * kWsMinBlocks <= 220 * 1024;
-    switch (p.tiling.schedule) {
-        case 1: return shallow ? SCHED_WS : SCHED_ROWS;
-        case 2: return wsp_fits ? SCHED_WSP : (shallow ? SCHED_WS : SCHED_ROWS);
-        default: return shallow ? SCHED_WS : (wsp_fits ? SCHED_WSP : SCHED_ROWS);
-    }
-}
-
 // Launches the gridding kernel selected by `c` over all work items.
 static void grid_dispatch_cfg(const GridCfg &c, const NufftPlan &p, const ConvArgs &a, const float2 *samples,
                               float2 *grid, cudaStream_t st) {
-    dim3 g(p.n_grd_items, c.ncg);
-    if (c.rows && a.layout == LAYOUT_SORTED_IL && normal_grid_sched(p, c) == SCHED_WSP) {
-        const bool d3 = p.kp.D == 3;
-        if (c.cg == 16) {
-            if (d3) grid_rows_wsp_shape<16, true>(c, a, samples, grid, st);
-            else grid_rows_wsp_shape<16, false>(c, a, samples, grid, st);
-        } else {
-            if (d3) grid_rows_wsp_shape<8, true>(c, a, samples, grid, st);
-            else grid_rows_wsp_shape<8, false>(c, a, samples, grid, st);
-        }
-    } else if (c.rows && a.layout == LAYOUT_SORTED_IL) {
-        const bool d3 = p.kp.D == 3;
-        if (c.cg == 16) {
-            if (d3) grid_rows_ws_shape<16, true>(c, a, g, samples, grid, st);
-            else grid_rows_ws_shape<16, false>(c, a, g, samples, grid, st);
-        } else {
-            if (d3) grid_rows_ws_shape<8, true>(c, a, g, samples, grid, st);
-            else grid_rows_ws_shape<8, false>(c, a, g, samples, grid, st);
-        }
-    } else if (c.rows) {
-        const bool d3 = p.kp.D == 3;
-        if (c.cg == 16) {
-            if (d3) grid_rows_shape<16, true>(c, a, g, samples, grid, st);
-            else grid_rows_shape<16, false>(c, a, g, samples, grid, st);
-        } else {
-            if (d3) grid_rows_shape<8, true>(c, a, g, samples, grid, st);
-            else grid_rows_shape<8, false>(c, a, g, samples, grid, st);
-        }
+    dim3 g(a.n_items, c.ncg);
+    if (c.brick) {
+        launch_grid_brick(c, p, a, samples, grid, st);
     } else if (p.flags & GB_FLAG_COMPENSATED) {
         switch (c.cg) {
             case 1: grid_dispatch_cpt<1, true>(c.cpt, a, g, samples, grid, st); break;
@@ -2279,25 +1066,51 @@ static void grid_dispatch_cfg(const GridCfg &c, const NufftPlan &p, const ConvAr
 // (must run outside stream capture).
 void launch_grid_prepare(NufftPlan &p, int nb, cudaStream_t st) {
     const GridCfg c = grid_config(p, nb);
-    if (p.grid_queue.ensure(2)) GB_CUDA(cudaMemsetAsync(p.grid_queue.get(), 0, 2 * sizeof(unsigned int), st));
     if (p.n_splits > 0) {
-        const size_t need_ctr = (size_t)p.n_splits * c.ncg;
+        const size_t need_ctr = (size_t)p.n_splits * c.ncg * c.groups;
         if (p.split_counters.n < need_ctr || p.split_counter_groups == 0) {
             p.split_counters.ensure(need_ctr);
             GB_CUDA(cudaMemsetAsync(p.split_counters.get(), 0, p.split_counters.n * sizeof(unsigned int), st));
-            p.split_counter_groups = c.ncg;
+            p.split_counter_groups = c.ncg * c.groups;
         }
         p.partials.ensure((size_t)p.n_slots * c.ncg * c.part_elems);
     }
 }
 
+constexpr int kIlMinCoils = 5;
+
 void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, SampleLayout layout,
-                 const float *dcw, bool sign_fold, bool accumulate, cudaStream_t st, const KLayout *kl) {
+                 const float *dcw, bool sign_fold, bool accumulate, cudaStream_t st, const KLayout *kl, bool use_ws) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "preprocess has not been called");
     const GridCfg c = grid_config(p, nb);
-    if (layout == LAYOUT_SORTED_IL && (!c.rows || dcw))
-        fail(GB_ERR_INTERNAL, "interleaved samples need the row-variant gridding kernel and no density weights");
-    ConvArgs a = make_args(p, nb, layout, dcw, 1, sign_fold, accumulate);
+    if (layout == LAYOUT_SORTED_IL && (!c.brick || dcw))
+        fail(GB_ERR_INTERNAL, "interleaved samples need the brick gridding kernel and no density weights");
+    if (p.n_grd_items == 0) return;
+    const ConvArgs orig = make_args(p, nb, layout, dcw, 1, sign_fold, accumulate);
+    // The caller's samples are one plane per coil: from kIlMinCoils coils on
+    // they are first laid into sorted coil-interleaved rows (density weights
+    // folded in), so that a hit loads its coils as one run instead of one
+    // sector per coil.  Not when that would have to allocate during a capture.
+    const float2 *src = samples;
+    SampleLayout lay = layout;
+    if (use_ws && c.brick && layout != LAYOUT_SORTED_IL && nb >= kIlMinCoils && samples != p.samp_ws.get()) {
+        const size_t need = (size_t)il_stride_for(nb) * p.Mtot;
+        bool room = p.samp_ws.n >= need;
+        if (!room) {
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            GB_CUDA(cudaStreamIsCapturing(st, &cs));
+            if (cs == cudaStreamCaptureStatusNone) {
+                p.samp_ws.ensure(need);
+                room = true;
+            }
+        }
+        if (room) {
+            launch_samples_il(p, samples, dcw, nb, p.samp_ws.get(), st);
+            src = p.samp_ws.get();
+            lay = LAYOUT_SORTED_IL;
+        }
+    }
+    ConvArgs a = make_args(p, nb, lay, lay == layout ? dcw : nullptr, 1, sign_fold, accumulate);
     if (kl) a.kl = *kl;
     a.list = p.grid_list.get();
     a.items = p.grd_items.get();
@@ -2310,45 +1123,56 @@ void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, Samp
         a.partials = p.partials.get();
         a.counters = p.split_counters.get();
     }
-    a.queue = p.grid_queue.get();
-    a.n_work = p.n_grd_items * c.ncg;
-    if (p.n_grd_items == 0) return;
-    grid_dispatch_cfg(c, p, a, samples, grid, st);
-    launch_ref_fold_fix(p, a, samples, grid, st);
+    grid_dispatch_cfg(c, p, a, src, grid, st);
+    ConvArgs fix = orig;
+    fix.kl = a.kl;
+    launch_ref_fold_fix(p, fix, samples, grid, st);
 }
 
-// The sample workspace layout of E^H E follows its gridding schedule.
+// The sample workspace layout of E^H E: interleaved rows when the brick
+// gridding runs on coil pairs.
 SampleLayout normal_op_layout(const NufftPlan &p, int nb) {
     const GridCfg c = grid_config(p, nb);
-    return normal_grid_sched(p, c) == SCHED_ROWS ? LAYOUT_SORTED : LAYOUT_SORTED_IL;
+    return c.brick && c.cg >= 2 ? LAYOUT_SORTED_IL : LAYOUT_SORTED;
 }
 
-// Scratch (split-tile partial tiles and their counters) that launch_grid
-// needs for `nb` batches, in elements.
-void grid_scratch_need(const NufftPlan &p, int nb, size_t *partial_elems, size_t *counter_elems) {
+// Scratch (split-tile partial tiles and their counters) that a gridding launch
+// needs for `nb` batches, in elements, with the fine or the coarse chunks.
+void grid_scratch_need(const NufftPlan &p, int nb, bool coarse, size_t *partial_elems, size_t *counter_elems) {
     const GridCfg c = grid_config(p, nb);
-    *partial_elems = p.n_splits > 0 ? (size_t)p.n_slots * c.ncg * c.part_elems : 0;
-    *counter_elems = p.n_splits > 0 ? (size_t)p.n_splits * c.ncg : 0;
+    const int slots = coarse ? p.n_coarse_slots : p.n_slots;
+    *partial_elems = p.n_splits > 0 ? (size_t)slots * c.ncg * c.part_elems : 0;
+    *counter_elems = p.n_splits > 0 ? (size_t)p.n_splits * c.ncg * c.groups : 0;
 }
 
 // The gridding launch of launch_grid with caller-provided scratch: no device
 // allocation.  `counters` must hold counter_elems zeros on entry (the kernel
 // leaves them zero again when it completes).
 void launch_grid_external_scratch(NufftPlan &p, const float2 *samples, float2 *grid, int nb, bool accumulate,
-                                  float2 *partials, unsigned int *counters, cudaStream_t st) {
+                                  bool coarse, float2 *partials, unsigned int *counters, cudaStream_t st) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "preprocess has not been called");
     const GridCfg c = grid_config(p, nb);
     ConvArgs a = make_args(p, nb, LAYOUT_ORIGINAL, nullptr, 1, false, accumulate);
     a.list = p.grid_list.get();
-    a.items = p.grd_items.get();
-    a.n_items = p.n_grd_items;
-    a.splits = p.splits.get();
     a.ncg = c.ncg;
     a.part_elems = c.part_elems;
     a.partials = partials;
     a.counters = counters;
     if (p.n_grd_items == 0) return;
-    grid_dispatch_cfg(c, p, a, samples, grid, st);
+    const WorkItem *items = p.grd_items.get();
+    auto run = [&](const WorkItem *first, int n, const SplitInfo *splits) {
+        if (n == 0) return;
+        a.items = first;
+        a.n_items = n;
+        a.splits = splits;
+        grid_dispatch_cfg(c, p, a, samples, grid, st);
+    };
+    if (coarse) {
+        run(items + p.n_grd_items, p.n_coarse_items, p.splits.get() + p.n_splits);
+        run(items + (p.n_grd_items - p.n_light_items), p.n_light_items, p.splits.get());
+    } else {
+        run(items, p.n_grd_items, p.splits.get());
+    }
     launch_ref_fold_fix(p, a, samples, grid, st);
 }
 

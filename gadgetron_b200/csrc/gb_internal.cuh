@@ -144,15 +144,15 @@ struct KLayout {
     long long s_bf, s_y, s_z;
 };
 
-// One unit of tile work: frame*ntiles + tile, a range of a sample list and,
-// for gridding tiles split across CTAs, the split bookkeeping.
+// One unit of tile work: a frame's tile (tile coordinates), a range of a sample
+// list and, for gridding tiles split across CTAs, the split bookkeeping.
 struct WorkItem {
-    int ft;        // frame * ntiles_total + tile
-    int begin;     // range in the list
+    int begin;       // range in the list
     int end;
-    int split;     // -1: not split; else index into split table
-    int chunk;     // chunk index within the split
-    int pad0, pad1, pad2;
+    int split;       // -1: not split; else index into split table
+    int chunk;       // chunk index within the split
+    int f;           // frame
+    int tx, ty, tz;  // tile
 };
 
 __host__ __device__ inline KLayout klayout_standard(const KParams &k) {
@@ -183,11 +183,10 @@ __host__ __device__ inline long long kaddr(const KLayout &l, long long bf, int x
     return bf * l.s_bf + z * l.s_z + y * l.s_y + x;
 }
 
-// Floats of the weight part of a pair row and of a whole pair row.
-__host__ __device__ inline int pair_row_weights(const KParams &k) {
+// Floats of a pair row: the sample's weights laid over the tile, per dimension.
+__host__ __device__ inline int pair_row_floats(const KParams &k) {
     return (k.tile[0] + k.tile[1] + (k.D == 3 ? k.tile[2] : 0) + 3) & ~3;
 }
-__host__ __device__ inline int pair_row_floats(const KParams &k) { return pair_row_weights(k) + 4; }
 
 // Device-side scalars of one CG segment (a frame, or all frames).
 struct CgSeg {
@@ -217,8 +216,7 @@ struct SplitInfo {
 struct Tiling {
     int tile[kMaxD] = {16, 16, 1};
     int cg = 8;                 // coils per CTA (coil group)
-    int split_len = 0;          // gridding list length above which a tile is split (0 = auto)
-    int schedule = 0;           // E^H E gridding: 0 auto, 1 one CTA per work item, 2 persistent work queue
+    int schedule = 0;           // gb_nufft_set_grid_schedule (kept; one gridding kernel serves all)
 };
 
 struct NufftPlan {
@@ -268,10 +266,11 @@ struct NufftPlan {
     DevBuf<uint32_t> grid_list;    // gridding pair list (sorted positions)
     // Per gridding pair, the sample's 1D weights laid over the tile: rows of
     // pair_row_stride floats = x weights (tile x), y weights (tile y), z
-    // weights (tile z, 3D), padding to a multiple of 4, then 4 words of the
-    // tile-local footprint ranges (lo | hi << 16 per dimension).  Built at
-    // preprocess for D >= 2 (pair_row_stride = 0 when not built).
+    // weights (tile z, 3D), padding to a multiple of 4; and the tile-local
+    // footprint range, bytes (x lo, x hi, y lo, y hi, z lo, z hi, 0, 0).
+    // Built at preprocess for D >= 2 (pair_row_stride = 0 when not built).
     DevBuf<float> pair_rows;
+    DevBuf<uint2> pair_rng;
     int pair_row_stride = 0;
     DevBuf<unsigned int> err_flag;   // set by kernels whose bounded waits ran out
     DevBuf<uint32_t> grid_off;     // [F*ntiles + 1]
@@ -281,8 +280,10 @@ struct NufftPlan {
     int n_grd_items = 0;
     DevBuf<SplitInfo> splits;
     int n_splits = 0, n_slots = 0;
+    // The split tiles in longer chunks: items after the n_grd_items of
+    // grd_items, their n_splits table entries after the first n_splits.
+    int n_light_items = 0, n_coarse_items = 0, n_coarse_slots = 0;
     DevBuf<unsigned int> split_counters;   // [n_splits * max coil groups]
-    DevBuf<unsigned int> grid_queue;       // persistent gridding: next unit, CTAs finished (zero between launches)
     int split_counter_groups = 0;
     DevBuf<float2> partials;               // [n_slots][cg_groups][cells*cg]
     int64_t total_pairs = 0;
@@ -358,12 +359,11 @@ void plan_autotune(NufftPlan &p, int nb, cudaStream_t st);
 //              (il = nb rounded up to even, so a sample's coil group is a
 //              16-byte multiple): the plan's own workspace between
 //              degridding and gridding inside E^H E, which the gridding
-//              kernel stages by bulk copies (no gather through registers).
+//              kernel stages in runs of 16 bytes per coil pair.
 enum SampleLayout { LAYOUT_ORIGINAL = 0, LAYOUT_SORTED = 1, LAYOUT_SORTED_IL = 2 };
 __host__ __device__ inline int il_stride_for(int nb) { return (nb + 1) & ~1; }
 // The layout that E^H E hands from degridding to gridding for nb batches:
-// SORTED_IL when the gridding runs the row variant (bulk-copied values),
-// else SORTED.
+// SORTED_IL when the brick gridding runs on coil pairs, else SORTED.
 SampleLayout normal_op_layout(const NufftPlan &p, int nb);
 
 // Degridding: grid [nb][F][G] -> samples.  sign_fold multiplies the weight of
@@ -375,10 +375,12 @@ void launch_degrid(NufftPlan &p, const float2 *grid, float2 *samples, int nb,
                    bool accumulate, cudaStream_t st, const KLayout *kl = nullptr);
 
 // Gridding: samples -> grid [nb][F][G] (overwritten unless accumulate).
-// dcw multiplies the input samples (may be null).
+// dcw multiplies the input samples (may be null).  use_ws: the plan's sample
+// workspace may hold the interleaved samples (not for calls that may overlap
+// on one plan).
 void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb,
                  SampleLayout layout, const float *dcw, bool sign_fold, bool accumulate,
-                 cudaStream_t st, const KLayout *kl = nullptr);
+                 cudaStream_t st, const KLayout *kl = nullptr, bool use_ws = true);
 
 // Trajectory gradient from a k-space grid (sign folded like the degridder).
 void launch_traj_grad(NufftPlan &p, const float2 *grid, const float2 *weights, int nb,

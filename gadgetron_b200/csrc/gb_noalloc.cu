@@ -79,7 +79,10 @@ extern "C" GB_API gb_status gb_nufft_convolve_nc2c_noalloc(gb_nufft_plan plan, c
             ~Restore() { if (dev != cur && dev >= 0) cudaSetDevice(dev); }
         } restore{old, p->device};
         size_t need_partials = 0, need_counters = 0;
-        grid_scratch_need(*p, nb, &need_partials, &need_counters);
+        grid_scratch_need(*p, nb, false, &need_partials, &need_counters);
+        // split tiles in longer chunks when the short ones' partial tiles do not fit
+        const bool coarse = need_partials > kPartialElems;
+        if (coarse) grid_scratch_need(*p, nb, true, &need_partials, &need_counters);
         if (need_partials > kPartialElems || need_counters > kCounterElems)
             fail(GB_ERR_INVALID_ARGUMENT,
                  "gb_nufft_convolve_nc2c_noalloc: this plan and batch count need " +
@@ -92,7 +95,7 @@ extern "C" GB_API gb_status gb_nufft_convolve_nc2c_noalloc(gb_nufft_plan plan, c
         if (need_counters) check_cuda(cudaMemsetAsync(counters, 0, need_counters * sizeof(unsigned int), st),
                                       "cudaMemsetAsync");
         launch_grid_external_scratch(*p, static_cast<const float2 *>(samples), static_cast<float2 *>(grid),
-                                     nb, accumulate != 0, partials, counters, st);
+                                     nb, accumulate != 0, coarse, partials, counters, st);
         return GB_OK;
     } catch (...) {
         return current_exception_status();

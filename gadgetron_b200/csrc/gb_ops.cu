@@ -278,7 +278,7 @@ void nufft_mult_MH_M(NufftPlan &p, const void *in, void *out, const float *dcw, 
 }
 
 void nufft_convolve(NufftPlan &p, const void *in, void *out, gb_conv_mode mode, bool accumulate, int nb,
-                    cudaStream_t st) {
+                    cudaStream_t st, bool use_ws) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "NFFT_plan::convolve: preprocess has not been called");
     if (!in || !out) fail(GB_ERR_INVALID_ARGUMENT, "NULL input/output");
     if (mode == GB_CONV_C2NC)
@@ -286,7 +286,7 @@ void nufft_convolve(NufftPlan &p, const void *in, void *out, gb_conv_mode mode, 
                       nullptr, 1, false, accumulate, st);
     else
         launch_grid(p, static_cast<const float2 *>(in), static_cast<float2 *>(out), nb, LAYOUT_ORIGINAL,
-                    nullptr, false, accumulate, st);
+                    nullptr, false, accumulate, st, nullptr, use_ws);
 }
 
 void nufft_fft(NufftPlan &p, void *data, gb_fft_mode mode, bool do_scale, int nbf, cudaStream_t st) {

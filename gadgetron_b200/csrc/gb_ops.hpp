@@ -96,8 +96,9 @@ void nufft_compute(NufftPlan &p, const void *in, void *out, const float *dcw, gb
 void nufft_mult_MH_M(NufftPlan &p, const void *in, void *out, const float *dcw, int nb, cudaStream_t st);
 void nufft_time_normal_convolutions(NufftPlan &p, int nb, const float *dcw, int reps, void *flush,
                                     size_t flush_bytes, float *ms_grid, float *ms_degrid, cudaStream_t st);
+// use_ws: gridding may use the plan's sample workspace (the plan serves one call at a time).
 void nufft_convolve(NufftPlan &p, const void *in, void *out, gb_conv_mode mode, bool accumulate, int nb,
-                    cudaStream_t st);
+                    cudaStream_t st, bool use_ws = false);
 void nufft_fft(NufftPlan &p, void *data, gb_fft_mode mode, bool do_scale, int nbf, cudaStream_t st);
 void nufft_deapodize(NufftPlan &p, void *data, int nbf, cudaStream_t st);
 void nufft_traj_grad(NufftPlan &p, const float2 *img, const float2 *weights, const float *dcw, float *grad,
@@ -124,9 +125,9 @@ struct SenseBuffer {
 };
 
 // Gridding with caller-provided scratch (no device allocation).
-void grid_scratch_need(const NufftPlan &p, int nb, size_t *partial_elems, size_t *counter_elems);
+void grid_scratch_need(const NufftPlan &p, int nb, bool coarse, size_t *partial_elems, size_t *counter_elems);
 void launch_grid_external_scratch(NufftPlan &p, const float2 *samples, float2 *grid, int nb, bool accumulate,
-                                  float2 *partials, unsigned int *counters, cudaStream_t st);
+                                  bool coarse, float2 *partials, unsigned int *counters, cudaStream_t st);
 // The plan behind a C handle (defined with the C ABI).
 NufftPlan *plan_from_handle(gb_nufft_plan h);
 // Status code (and error message) for the exception being handled.

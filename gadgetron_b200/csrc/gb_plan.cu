@@ -380,15 +380,15 @@ __global__ void k_write_pairs(KParams k, int64_t M, const float *__restrict__ po
             }
 }
 
-// Pair rows for the row-variant gridding kernel: one thread per (pair,
+// Pair rows for the brick gridding kernel: one thread per (pair,
 // dimension) lays the sample's tap weights (from the weight table, unsigned)
 // over the tile's extent in that dimension -- tap t at tile-local cell
 // (ceil(s - W/2) + t - pad/2 - tile origin) mod mos when that falls inside the
-// tile, zero elsewhere -- and records the tile-local footprint range.
+// tile, zero elsewhere -- and records the tile-local footprint range (bytes).
 __global__ void k_pair_rows(KParams k, int64_t M, int64_t npairs, const float *__restrict__ pos_sorted,
                             const float *__restrict__ wtab, const uint32_t *__restrict__ pair_key,
                             const uint32_t *__restrict__ pair_sample, float *__restrict__ rows, int row_floats,
-                            int row_weights) {
+                            uint16_t *__restrict__ ranges) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= npairs * k.D) return;
     const int64_t q = e / k.D;
@@ -414,7 +414,7 @@ __global__ void k_pair_rows(KParams k, int64_t M, int64_t npairs, const float *_
         wr[c] = t < n ? taps[t] : 0.f;
     }
     if (d == 0)
-        for (int c = k.tile[0] + k.tile[1] + (k.D == 3 ? k.tile[2] : 0); c < row_weights; c++) row[c] = 0.f;
+        for (int c = k.tile[0] + k.tile[1] + (k.D == 3 ? k.tile[2] : 0); c < row_floats; c++) row[c] = 0.f;
     int rlo, rhi;
     if (k.ntiles[d] == 1) {   // the footprint may wrap inside the tile
         rlo = 0;
@@ -424,8 +424,7 @@ __global__ void k_pair_rows(KParams k, int64_t M, int64_t npairs, const float *_
         rlo = max(st, 0);
         rhi = min(st + n - 1, Td - 1);
     }
-    reinterpret_cast<uint32_t *>(row + row_weights)[d] = (uint32_t)rlo | ((uint32_t)rhi << 16);
-    if (d == 0 && k.D == 2) reinterpret_cast<uint32_t *>(row + row_weights)[2] = 0u;
+    ranges[4 * q + d] = (uint16_t)(rlo | (rhi << 8));
 }
 
 static int bits_for(uint64_t n) {
@@ -546,16 +545,20 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
     pkey_sorted.ensure(npairs);
     p.grid_list.ensure(npairs);
     p.grid_off.ensure(nkeys + 1);
-    const bool rows = D >= 2 && pair_row_weights(k) <= 96 && npairs > 0;
+    const bool rows = D >= 2 && pair_row_floats(k) <= 96 && npairs > 0;
     const int rf = rows ? pair_row_floats(k) : 0;
-    if (rows) p.pair_rows.ensure((size_t)npairs * rf);
+    if (rows) {
+        p.pair_rows.ensure((size_t)npairs * rf);
+        p.pair_rng.ensure(npairs);
+    }
     uint64_t key_b = kp_hash;
     for (uint64_t v : {(uint64_t)npairs, (uint64_t)M, (uint64_t)nkeys, (uint64_t)rf,
                        (uint64_t)(uintptr_t)p.pos_sorted.get(), (uint64_t)(uintptr_t)key_sorted.get(),
                        (uint64_t)(uintptr_t)poff.get(), (uint64_t)(uintptr_t)pkey.get(), (uint64_t)(uintptr_t)pval.get(),
                        (uint64_t)(uintptr_t)pkey_sorted.get(), (uint64_t)(uintptr_t)p.grid_list.get(),
                        (uint64_t)(uintptr_t)p.grid_off.get(), (uint64_t)(uintptr_t)p.wtab.get(),
-                       (uint64_t)(uintptr_t)p.pair_rows.get(), (uint64_t)(uintptr_t)p.pp_sort.get(),
+                       (uint64_t)(uintptr_t)p.pair_rows.get(), (uint64_t)(uintptr_t)p.pair_rng.get(),
+                       (uint64_t)(uintptr_t)p.pp_sort.get(),
                        (uint64_t)p.pp_sort.n})
         key_b = mix_key(key_b, v);
     run_prep_segment(p.prep_graph[1], key_b, st, [&](cudaStream_t s) {
@@ -569,7 +572,7 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
         if (rows) {
             k_pair_rows<<<(unsigned)(((int64_t)npairs * D + TB - 1) / TB), TB, 0, s>>>(
                 k, M, npairs, p.pos_sorted.get(), p.wtab.get(), pkey_sorted.get(), p.grid_list.get(), p.pair_rows.get(),
-                rf, pair_row_weights(k)); ::gb::note_launch();
+                rf, reinterpret_cast<uint16_t *>(p.pair_rng.get())); ::gb::note_launch();
             GB_CUDA(cudaGetLastError());
         }
     });
@@ -630,11 +633,32 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     // copy is a large share of an item's work in 2D)
     int deg_chunk = (int)std::max<int64_t>(256, std::min<int64_t>(1024, M / (148 * 4) + 1));
     std::vector<WorkItem> deg;
-    for (uint32_t key = 0; key < nkeys; key++) {
+    // frame and tile coordinates of key 0, 1, ... in turn
+    struct TileCounter {
+        const KParams &k;
+        int f = 0, tx = 0, ty = 0, tz = 0;
+        void place(WorkItem &w) const {
+            w.f = f;
+            w.tx = tx;
+            w.ty = ty;
+            w.tz = tz;
+        }
+        void step() {
+            if (++tx < k.ntiles[0]) return;
+            tx = 0;
+            if (++ty < k.ntiles[1]) return;
+            ty = 0;
+            if (++tz < k.ntiles[2]) return;
+            tz = 0;
+            f++;
+        }
+    };
+    TileCounter dt{k};
+    for (uint32_t key = 0; key < nkeys; key++, dt.step()) {
         uint32_t b = hoff[key], e = hoff[key + 1];
         for (uint32_t s = b; s < e; s += deg_chunk) {
             WorkItem w{};
-            w.ft = (int)key;
+            dt.place(w);
             w.begin = (int)s;
             w.end = (int)std::min<uint32_t>(e, s + deg_chunk);
             w.split = -1;
@@ -643,63 +667,72 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     }
     sort_items_by_length(deg);
 
-    // Gridding items.
-    int64_t total = goff[nkeys];
-    int split_len = p.tiling.split_len;
-    if (split_len <= 0) {
-        int64_t avg = total / std::max<uint32_t>(1, nkeys);
-        split_len = (int)std::max<int64_t>(256, 2 * avg);
-    }
-    std::vector<WorkItem> heavy, light;
-    std::vector<SplitInfo> splits;
-    int slots = 0;
-    for (uint32_t key = 0; key < nkeys; key++) {
-        uint32_t b = goff[key], e = goff[key + 1];
-        uint32_t len = e - b;
+    // Gridding items: tiles of at most split_len pairs as they are, longer ones
+    // in chunks.  The samples of a dense tile (a radial centre) crowd into one
+    // or two of its bricks, so a chunk's time is the chain of the warp that owns
+    // the crowded brick: chunks are kept at the average tile's length (at least
+    // 96), far below the split threshold.  Chunks of that length need more
+    // partial tiles; the entry point with a fixed scratch takes chunks of up
+    // to split_len pairs when those do not fit (the coarse list).
+    const int64_t total = goff[nkeys];
+    const int64_t avg = total / std::max<uint32_t>(1, nkeys);
+    const int split_len = (int)std::max<int64_t>(256, 2 * avg);
+    const int fine_len = (int)std::max<int64_t>(96, avg);
+    std::vector<WorkItem> light, heavy[2];   // [0] fine, [1] coarse
+    std::vector<SplitInfo> splits[2];
+    int slots[2] = {0, 0};
+    TileCounter gt{k};
+    for (uint32_t key = 0; key < nkeys; key++, gt.step()) {
+        const uint32_t b = goff[key], e = goff[key + 1];
+        const uint32_t len = e - b;
+        WorkItem w{};
+        gt.place(w);
         if ((int)len <= split_len) {
-            WorkItem w{};
-            w.ft = (int)key;
             w.begin = (int)b;
             w.end = (int)e;
             w.split = -1;
             light.push_back(w);
-        } else {
-            int nch = (int)((len + split_len - 1) / split_len);
-            int per = (int)((len + nch - 1) / nch);
-            SplitInfo si{slots, nch};
-            int sid = (int)splits.size();
-            splits.push_back(si);
-            for (int c = 0; c < nch; c++) {
-                WorkItem w{};
-                w.ft = (int)key;
-                w.begin = (int)(b + c * per);
-                w.end = (int)std::min<uint32_t>(e, b + (c + 1) * per);
-                w.split = sid;
-                w.chunk = c;
-                heavy.push_back(w);
+            continue;
+        }
+        for (int c = 0; c < 2; c++) {
+            const uint32_t most = (uint32_t)(c == 0 ? fine_len : split_len);
+            const uint32_t nch = (len + most - 1) / most, per = (len + nch - 1) / nch;
+            w.split = (int)splits[c].size();
+            splits[c].push_back(SplitInfo{slots[c], (int)nch});
+            for (uint32_t q = 0; q < nch; q++) {
+                w.begin = (int)(b + q * per);
+                w.end = (int)std::min<uint32_t>(e, b + (q + 1) * per);
+                w.chunk = (int)q;
+                heavy[c].push_back(w);
             }
-            slots += nch;
+            slots[c] += (int)nch;
         }
     }
     sort_items_by_length(light);
-    std::vector<WorkItem> grd(heavy);
+    std::vector<WorkItem> grd(heavy[0]);
     grd.insert(grd.end(), light.begin(), light.end());
+    p.n_light_items = (int)light.size();
+    p.n_coarse_items = (int)heavy[1].size();
+    p.n_coarse_slots = slots[1];
 
     p.n_deg_items = (int)deg.size();
     p.deg_items.ensure(std::max<size_t>(1, deg.size()));
     p.n_grd_items = (int)grd.size();
+    grd.insert(grd.end(), heavy[1].begin(), heavy[1].end());   // after the n_grd_items of a launch
     p.grd_items.ensure(std::max<size_t>(1, grd.size()));
-    p.n_splits = (int)splits.size();
-    p.n_slots = slots;
-    p.splits.ensure(std::max<size_t>(1, splits.size()));
+    p.n_splits = (int)splits[0].size();
+    p.n_slots = slots[0];
+    std::vector<SplitInfo> both(splits[0]);
+    both.insert(both.end(), splits[1].begin(), splits[1].end());
+    p.splits.ensure(std::max<size_t>(1, both.size()));
     // The three lists go up from pinned staging (asynchronous; the staging
     // is not rewritten before these copies have been read).
     const size_t bd = deg.size() * sizeof(WorkItem), bg = grd.size() * sizeof(WorkItem);
-    const size_t bs = splits.size() * sizeof(SplitInfo);
+    const size_t bs = both.size() * sizeof(SplitInfo);
     unsigned char *up = upload_room(p, bd + bg + bs);
     if (bd) std::memcpy(up, deg.data(), bd);
     if (bg) std::memcpy(up + bd, grd.data(), bg);
-    if (bs) std::memcpy(up + bd + bg, splits.data(), bs);
+    if (bs) std::memcpy(up + bd + bg, both.data(), bs);
     if (bd) GB_CUDA(cudaMemcpyAsync(p.deg_items.get(), up, bd, cudaMemcpyHostToDevice, st));
     if (bg) GB_CUDA(cudaMemcpyAsync(p.grd_items.get(), up + bd, bg, cudaMemcpyHostToDevice, st));
     if (bs) GB_CUDA(cudaMemcpyAsync(p.splits.get(), up + bd + bg, bs, cudaMemcpyHostToDevice, st));
@@ -716,7 +749,7 @@ uint64_t plan_layout_signature(const NufftPlan &p, int nbf) {
         }
     };
     const void *ptrs[] = {p.pos_sorted.get(), p.wtab.get(), p.pair_rows.get(), p.perm.get(), p.grid_list.get(), p.grd_items.get(),
-                          p.deg_items.get(), p.splits.get(), p.partials.get(), p.split_counters.get(), p.grid_queue.get(),
+                          p.deg_items.get(), p.splits.get(), p.partials.get(), p.split_counters.get(), p.pair_rng.get(),
                           p.img_os.get(), p.kgrid.get(), p.samp_ws.get(), p.deap_img.get(), p.deap_os.get()};
     for (const void *q : ptrs) mix((uint64_t)(uintptr_t)q);
     const int64_t vals[] = {p.n_deg_items, p.n_grd_items, p.n_splits, p.n_slots, p.Mtot, (int64_t)p.F,

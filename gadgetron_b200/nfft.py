@@ -162,8 +162,8 @@ class cuNFFT_plan:
         check(lib.gb_nufft_set_tiling(self._h, t, int(coil_group)))
 
     def set_grid_schedule(self, schedule: int):
-        """Gridding schedule of the normal operator: 0 by launch depth, 1 one
-        CTA per work item, 2 one persistent work-queue launch (same results)."""
+        """Gridding schedule of the normal operator (0, 1 or 2; kept by the plan:
+        one gridding kernel serves all of them)."""
         check(lib.gb_nufft_set_grid_schedule(self._h, int(schedule)))
 
     def get_grid_schedule(self) -> int:

@@ -207,8 +207,7 @@ GB_API gb_status gb_nufft_get_info(gb_nufft_plan plan, int *D, uint64_t *matrix_
                                    uint64_t *num_samples_total, uint32_t *num_frames);
 
 /* Device-side error word of the plan: kernels whose bounded waits ran out
- * (a bulk copy that did not complete, a grid barrier not reached by every
- * block) set a bit instead of spinning forever.  Synchronises the stream,
+ * (a grid barrier not reached by every block: bit 1) set a bit instead of spinning forever.  Synchronises the stream,
  * writes the word to *error_bits (0: none) and clears it.  No reference
  * counterpart. */
 GB_API gb_status gb_nufft_device_errors(gb_nufft_plan plan, uint32_t *error_bits, void *stream);
@@ -238,12 +237,11 @@ GB_API gb_status gb_nufft_time_normal_convolutions(gb_nufft_plan plan, uint32_t 
 GB_API gb_status gb_nufft_get_tiling(gb_nufft_plan plan, int *tile, int *coil_group);
 GB_API gb_status gb_nufft_set_tiling(gb_nufft_plan plan, const int *tile, int coil_group);
 
-/* How the normal operator (mult_MH_M, the CG-SENSE iteration) grids its own
- * tile-ordered samples: 0 (default) chooses by launch depth; 1 one CTA per
- * gridding work item; 2 one persistent launch whose CTAs take (frame, tile,
- * coil group) work units from a device-side queue.  Results are the same
- * bit for bit; only the speed differs.  Takes effect at the next launch (a
- * captured CG graph is re-captured).  No reference counterpart (tuning). */
+/* Gridding schedule of the normal operator (mult_MH_M, the CG-SENSE
+ * iteration): 0 (default), 1 or 2, kept by the plan and returned by the getter.
+ * One gridding kernel, chosen by shape, now serves every value: results and
+ * speed are the same.  (A captured CG graph is re-captured when it changes.)
+ * No reference counterpart (tuning). */
 GB_API gb_status gb_nufft_set_grid_schedule(gb_nufft_plan plan, int schedule);
 GB_API gb_status gb_nufft_get_grid_schedule(gb_nufft_plan plan, int *schedule);
 

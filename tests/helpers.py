@@ -39,3 +39,17 @@ def rel_l2(a, b):
     a = np.asarray(a, np.complex128).ravel()
     b = np.asarray(b, np.complex128).ravel()
     return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+def footprint_cells(k, mos, W):
+    """Boolean grid [.., y, x] of the cells within W/2 of the sample."""
+    hit = np.ones(tuple(reversed(mos)), bool)
+    for d, m in enumerate(mos):
+        s = np.float32(k[d]) * np.float32(m) + np.float32(m / 2)
+        near = np.zeros(m, bool)
+        c = np.arange(int(np.ceil(s - W / 2)), int(np.floor(s + W / 2)) + 1)
+        near[c % m] = True
+        shape = [1] * len(mos)
+        shape[len(mos) - 1 - d] = m
+        hit &= near.reshape(shape)
+    return hit

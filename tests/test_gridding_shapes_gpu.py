@@ -1,0 +1,126 @@
+"""The gridding kernel over the forms its dispatch chooses between: coil counts
+around every coil group (1 to 33), 2D and 3D, plain and compensated sums,
+tiles with no samples and tiles split into chunks, samples that are not
+finite, and the fixed-scratch entry point's two chunk lengths.
+Against the oracle (float weights, double sums): relative L2 <= PARITY_TOL."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from gadgetron_b200 import synthetic as S
+from oracle import oracle as O
+from tests.helpers import PARITY_TOL, footprint_cells, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+import gadgetron_b200 as gb  # noqa: E402
+from gadgetron_b200._lib import lib  # noqa: E402
+
+COILS = [1, 2, 3, 4, 5, 8, 9, 12, 16, 17, 24, 33]
+
+
+def _samples(coils, m, seed):
+    rng = np.random.default_rng(seed)
+    return (rng.standard_normal((coils, m)) + 1j * rng.standard_normal((coils, m))).astype(np.complex64)
+
+
+def _adjoint_and_normal(N, mos, W, traj, coils, flags, cuda):
+    D = len(N)
+    plan = gb.NFFT.make_plan(N, mos, W, flags=flags)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    orc = O.OraclePlan(N, mos, W)
+    orc.preprocess(traj.reshape(1, -1, D))
+    y = _samples(coils, traj.shape[0], coils)
+    w = S.ramp_dcw(traj)
+    wt = torch.from_numpy(w).to(cuda)
+    x = torch.empty((coils, 1) + tuple(reversed(N)), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(y).to(cuda), x, wt, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+    ref = orc.backwards_nc2c(y, w[None])
+    assert rel_l2(x.cpu().numpy(), ref) <= PARITY_TOL
+    img = S.gaussian_image((coils, 1) + tuple(reversed(N)), coils + 1)
+    nrm = torch.empty_like(x)
+    plan.mult_MH_M(torch.from_numpy(img).to(cuda), nrm, wt)
+    assert rel_l2(nrm.cpu().numpy(), orc.mult_MH_M(img, w[None])) <= PARITY_TOL
+    assert plan.device_errors() == 0
+
+
+@pytest.mark.parametrize("coils", COILS)
+@pytest.mark.parametrize("W,alpha", [(5.5, 2.0), (4.0, 1.5)])
+def test_2d_coil_groups(cuda, coils, W, alpha):
+    """64 spokes through one centre (split tiles) on a rectangular grid."""
+    N = (64, 32)
+    mos = tuple(-(-int(n * alpha) // 32) * 32 for n in N)
+    _adjoint_and_normal(N, mos, W, S.radial_golden_angle_2d(64, 96), coils, 0, cuda)
+
+
+@pytest.mark.parametrize("coils", [1, 3, 8, 12, 17])
+def test_2d_compensated(cuda, coils):
+    _adjoint_and_normal((64, 64), (96, 96), 4.0, S.radial_golden_angle_2d(70, 96), coils, gb.FLAG_COMPENSATED, cuda)
+
+
+@pytest.mark.parametrize("coils", [1, 2, 4, 7, 16, 20])
+@pytest.mark.parametrize("flags", [0, 1])
+def test_3d_coil_groups(cuda, coils, flags):
+    N, mos = (32, 64, 32), (64, 96, 64)
+    _adjoint_and_normal(N, mos, 4.0, S.kooshball_golden_means_3d(300, 48), coils, flags, cuda)
+
+
+def test_wide_form_of_16_coils(cuda):
+    """Enough frames that the 16-coil gridding takes its wide form; the same
+    frames in a plan of their own take the narrow one."""
+    N, mos, W, C, F = (64, 64), (128, 128), 5.5, 16, 40
+    trajs = [S.radial_golden_angle_2d(8 + f % 5, 64, profile_offset=13 * f) for f in range(F)]
+    offs = np.cumsum([0] + [t.shape[0] for t in trajs]).tolist()
+    y = _samples(C, offs[-1], 3)
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(np.concatenate(trajs)).to(cuda), frame_offsets=offs)
+    x = torch.empty((C, F, 64, 64), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(y).to(cuda), x, None, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+    for f in (0, 17, 39):
+        orc = O.OraclePlan(N, mos, W)
+        orc.preprocess(trajs[f][None])
+        ref = orc.backwards_nc2c(y[:, offs[f]:offs[f + 1]])
+        assert rel_l2(x[:, f].cpu().numpy(), ref[:, 0]) <= PARITY_TOL, f
+
+
+@pytest.mark.parametrize("coils", [1, 2, 4, 8, 12, 16])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_nonfinite_sample_stays_in_its_footprint(cuda, coils, bad):
+    N, mos, W = (64, 64), (128, 128), 5.5
+    traj = S.radial_golden_angle_2d(24, 128)
+    y = _samples(coils, traj.shape[0], 9)
+    j = 1700
+    y[coils - 1, j] = bad
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    grid = torch.empty((coils, 1, 128, 128), dtype=torch.complex64, device=cuda)
+    plan.convolve(torch.from_numpy(y).to(cuda), grid, gb.NFFT_conv_mode.NC2C)
+    g = grid.cpu().numpy()[:, 0]
+    hit = footprint_cells(traj[j], mos, W)
+    assert np.all(np.isfinite(g[:coils - 1]))
+    assert np.all(np.isfinite(g[coils - 1][~hit]))
+    assert not np.any(np.isfinite(g[coils - 1][hit]))
+
+
+def test_noalloc_long_chunks_when_the_short_ones_do_not_fit(cuda):
+    """Dense centre, many coils: the partial tiles of the short chunks exceed
+    the fixed 16 MiB scratch, those of the long chunks do not; the call is
+    accepted and equals the regular entry point."""
+    N, mos, W, C = (128, 128), (256, 256), 5.5, 64
+    traj = S.radial_golden_angle_2d(256, 256)
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    y = torch.from_numpy(_samples(C, traj.shape[0], 2)).to(cuda)
+    ref = torch.empty((C, 1, 256, 256), dtype=torch.complex64, device=cuda)
+    plan.convolve(y, ref, gb.NFFT_conv_mode.NC2C)
+    out = torch.full_like(ref, float("nan"))
+    accepted = 0
+    for nb in (1, 8, 16, 32, 64):
+        st = lib.gb_nufft_convolve_nc2c_noalloc(plan._h, ctypes.c_void_p(y.data_ptr()), ctypes.c_void_p(out.data_ptr()),
+                                                0, nb, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        if st == 0:
+            accepted = nb
+            assert rel_l2(out[:nb].cpu().numpy(), ref[:nb].cpu().numpy()) <= PARITY_TOL
+    assert accepted >= 8
