@@ -68,4 +68,12 @@ void launch_grid_brick(const GridCfg &c, const NufftPlan &p, const ConvArgs &a, 
 void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *dcw, int nb, float2 *rows,
                        cudaStream_t st);
 
+// gb_degrid.cu: degridding and trajectory gradient from the weight table.
+bool degrid_table_ok(const NufftPlan &p, int cg);
+void launch_degrid_table(const NufftPlan &p, const ConvArgs &a, int cg, int ncg, bool comp, const float2 *grid,
+                         float2 *out, cudaStream_t st);
+bool grad_table_ok(const NufftPlan &p, int cg);
+void launch_grad_table(const NufftPlan &p, const ConvArgs &a, int cg, const float2 *grid, const float2 *w, float *out,
+                       cudaStream_t st);
+
 }  // namespace gb

@@ -484,10 +484,12 @@ k_degrid_c2nc(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__ 
     extern __shared__ float4 smem_raw[];
     const KParams &k = a.k;
     const WorkItem it = a.items[blockIdx.x];
-    const int grp = blockIdx.y;
-    const int b0 = grp * CG;
     const int f = it.f, tx = it.tx, ty = it.ty, tz = it.tz;
     const int org[3] = {tx * k.tile[0], ty * k.tile[1], tz * k.tile[2]};
+    // the gradient sums its coil groups in turn, the degridding runs one per CTA
+    for (int grp = GRAD ? 0 : (int)blockIdx.y; grp < (GRAD ? a.ncg : (int)blockIdx.y + 1); grp++) {
+    const int b0 = grp * CG;
+    if (GRAD && grp > 0) __syncthreads();   // the region is no longer read
     const int R0 = region_dim(k, 0), R1 = region_dim(k, 1), R2 = region_dim(k, 2);
     const int cellsR = R0 * R1 * R2;
     const int h0 = k.D > 0 ? k.hw : 0, h1 = k.D > 1 ? k.hw : 0, h2 = k.D > 2 ? k.hw : 0;
@@ -708,268 +710,16 @@ k_degrid_c2nc(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__ 
             if (valid && ll == 0) {
                 float scale = 1.f;
                 if (a.dcw) scale = (a.dcw_pow == 2) ? a.dcw[j] * a.dcw[j] : a.dcw[j];
-                float *gp = gout + ((int64_t)grp * a.Mtot + j) * k.D;
-                for (int d = 0; d < k.D; d++) gp[d] = r[d] * k.mos_f[d] * scale;
+                float *gp = gout + (int64_t)j * k.D;
+                for (int d = 0; d < k.D; d++) {
+                    const float v = r[d] * k.mos_f[d] * scale;
+                    gp[d] = grp > 0 ? gp[d] + v : v;
+                }
             }
         }
         __syncwarp();
     }
-}
-
-// Degridding, table variant (plain accumulation, no gradient): the same
-// region staging and lane layout as k_degrid_c2nc, but each lane reads its
-// sample's tap weights straight from the per-trajectory weight table into
-// registers (no per-warp staging, no kernel evaluation) and runs a fully
-// unrolled NT x NT (x NT) tap nest (unpredicated in x and y over the zero
-// weights beyond the footprint; 3D slices predicated on the sample's z
-// count), so the inner loop is loads and FMAs only.  NT = the largest tap count a
-// footprint can have (2*ceil(W/2), plus one when W is an even integer).
-// Per-sample inputs of one pass of the table degridding (loaded a pass ahead).
-struct DegRaw {
-    float sp[3];
-    float4 t0[3], t1[3];
-    uint32_t j;
-    float dw;
-};
-
-template <int CG, int NT, bool D3>
-__device__ __forceinline__ void degrid_table_load_raw(const ConvArgs &a, const WorkItem &it, int bs, DegRaw &r) {
-    using Sh = DegridShape<CG>;
-    constexpr int LPS = Sh::LPS, SPW = Sh::SPW;
-    constexpr int D = D3 ? 3 : 2;
-    const int lane = threadIdx.x & 31;
-    const int sl = lane / LPS;
-    const bool lane_ok = sl < SPW;   // false only for the 2 spare lanes of coil group 12
-    const int i = bs + sl;
-    const bool valid = lane_ok && i < it.end;
-    const int ic = valid ? i : it.begin;   // a valid row for the loads of idle lanes
-#pragma unroll
-    for (int d = 0; d < D; d++) {
-        r.sp[d] = a.pos[(int64_t)d * a.Mtot + ic];
-        const float4 *trow = reinterpret_cast<const float4 *>(a.wtab + ((int64_t)ic * D + d) * kWMax);
-        r.t0[d] = __ldg(trow);
-        r.t1[d] = NT > 4 ? __ldg(trow + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const bool need_j = a.layout == LAYOUT_ORIGINAL || a.dcw;
-    r.j = need_j ? a.perm[ic] : (uint32_t)ic;
-    r.dw = a.dcw ? a.dcw[r.j] : 1.f;
-}
-
-// The sample passes of one degridding work item over its staged region
-// (tile_s: the tile plus halo, cell stride CS, zero pad after it); `cur` holds
-// the first pass's inputs of this warp.
-template <int CG, int NT, bool D3>
-__device__ __forceinline__ void degrid_table_passes(const ConvArgs &a, const WorkItem &it, int b0, int org0,
-                                                    int org1, int org2, const float2 *tile_s,
-                                                    float2 *__restrict__ out, DegRaw cur) {
-    using Sh = DegridShape<CG>;
-    constexpr int CPL = Sh::CPL, LPS = Sh::LPS, SPW = Sh::SPW;
-    constexpr int D = D3 ? 3 : 2;
-    constexpr int CS = (D3 || CG == 12) ? CG : CG + 2;
-    const KParams &k = a.k;
-    const int R0 = region_dim(k, 0), R1 = region_dim(k, 1), R2 = region_dim(k, 2);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int sl = lane / LPS, ll = lane % LPS;
-    const bool lane_ok = sl < SPW;
-    DegRaw nxt;
-    int base = it.begin + warp * SPW;
-    for (; base < it.end; base += 8 * SPW) {
-        const int i = base + sl;
-        const bool valid = lane_ok && i < it.end;
-        if (base + 8 * SPW < it.end) degrid_table_load_raw<CG, NT, D3>(a, it, base + 8 * SPW, nxt);
-        int rs[3] = {0, 0, 0}, n[3] = {1, 1, 1};
-        float w[3][NT];
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-#pragma unroll
-            for (int t = 0; t < NT; t++) w[d][t] = (t == 0) ? 1.f : 0.f;
-        }
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-            const float sp = cur.sp[d] - (float)k.hw;
-            const int lo = (int)ceilf(sp - k.radius);
-            n[d] = valid ? min((int)floorf(sp + k.radius) - lo + 1, NT) : 0;
-            const int od = d == 0 ? org0 : (d == 1 ? org1 : org2);
-            int x = lo - od + k.hw;   // region-local start, |x| < 2 mos
-            x = x < 0 ? x + k.mos[d] : (x >= k.mos[d] ? x - k.mos[d] : x);
-            rs[d] = x;
-            const int Rd = d == 0 ? R0 : (d == 1 ? R1 : R2);
-            n[d] = min(n[d], Rd - x);   // the footprint lies inside the region; keep reads there
-            const float tv[8] = {cur.t0[d].x, cur.t0[d].y, cur.t0[d].z, cur.t0[d].w,
-                                 cur.t1[d].x, cur.t1[d].y, cur.t1[d].z, cur.t1[d].w};
-            // centring checkerboard: (-1)^(cell) with cell = lo + t (mos even)
-            const float s0 = (a.sign_fold && (lo & 1)) ? -1.f : 1.f;
-#pragma unroll
-            for (int t = 0; t < NT; t++) w[d][t] = (a.sign_fold && (t & 1)) ? -s0 * tv[t] : s0 * tv[t];
-        }
-        // (re, im) of each of the lane's coils, packed FP32x2 multiply-adds
-        float2 acc[CPL];
-#pragma unroll
-        for (int c = 0; c < CPL; c++) acc[c] = make_float2(0.f, 0.f);
-        const float2 *base_s = tile_s + (((size_t)rs[2] * R1 + rs[1]) * R0 + rs[0]) * CS + ll * CPL;
-        // Tap nest, unrolled to NTT taps per dimension, with no per-tap
-        // predicates in x and y: the table weights beyond a footprint are zero
-        // and a footprint starts at most NT-1 cells before the region's end,
-        // so the extra taps read at most one row and one cell past a slice --
-        // the next slice, or after the last one the zero pad.  3D slices stay
-        // predicated on the sample's z count.  When every sample of the warp
-        // has fewer than NT taps in every dimension (the common case when W is
-        // an even integer) the NT-1 nest runs.
-        auto nest = [&](auto ntc) {
-            constexpr int NTT = decltype(ntc)::value;
-#pragma unroll
-            for (int tzi = 0; tzi < (D3 ? NTT : 1); tzi++) {
-                if (tzi < n[2]) {
-#pragma unroll
-                    for (int tyi = 0; tyi < NTT; tyi++) {
-                        {
-                            const float wyz = D3 ? w[1][tyi] * w[2][tzi] : w[1][tyi];
-                            const float2 *row = base_s + ((size_t)tzi * R1 + tyi) * R0 * CS;
-#pragma unroll
-                            for (int t = 0; t < NTT; t++) {
-                                {
-                                    const float wv = w[0][t] * wyz;
-                                    const float2 wv2 = make_float2(wv, wv);
-                                    if (CPL == 2) {
-                                        const float4 q = *reinterpret_cast<const float4 *>(row + t * CS);
-                                        acc[0] = __ffma2_rn(wv2, make_float2(q.x, q.y), acc[0]);
-                                        acc[CPL - 1] = __ffma2_rn(wv2, make_float2(q.z, q.w), acc[CPL - 1]);
-                                    } else {
-                                        acc[0] = __ffma2_rn(wv2, row[t * CS], acc[0]);
-                                    }
-                                }
-                            }
-                        }
-                    }
-                }
-            }
-        };
-        // only when W is an even integer can a footprint have NT = W + 1 taps
-        // (an exact-integer position); otherwise NT taps are common
-        const bool shorter = (NT > 4 && 2 * k.hw < NT) &&
-                             __all_sync(0xffffffffu, n[0] < NT && n[1] < NT && n[2] < NT);
-        if (shorter)
-            nest(std::integral_constant<int, (NT > 4 ? NT - 1 : NT)>{});
-        else
-            nest(std::integral_constant<int, NT>{});
-        if (valid) {
-            const uint32_t j = cur.j;
-            const int64_t idx = (a.layout != LAYOUT_ORIGINAL) ? (int64_t)i : (int64_t)j;
-            const float dw = cur.dw;
-#pragma unroll
-            for (int c = 0; c < CPL; c++) {
-                const int coil = b0 + ll * CPL + c;
-                if (coil >= a.nb) {
-                    if (a.layout == LAYOUT_SORTED_IL && coil < a.il_stride)   // the row's padding
-                        out[idx * a.il_stride + coil] = make_float2(0.f, 0.f);
-                    break;
-                }
-                float2 val = acc[c];
-                if (a.dcw) {
-                    if (a.dcw_pow == 2) {
-                        val.x = (val.x * dw) * dw;
-                        val.y = (val.y * dw) * dw;
-                    } else {
-                        val.x *= dw;
-                        val.y *= dw;
-                    }
-                }
-                float2 *o = (a.layout == LAYOUT_SORTED_IL) ? out + idx * a.il_stride + coil
-                                                            : out + (int64_t)coil * a.Mtot + idx;
-                if (a.accumulate) { const float2 ov = *o; val.x += ov.x; val.y += ov.y; }
-                *o = val;
-            }
-        }
-        cur = nxt;
-    }
-}
-
-template <int CG, int NT, bool D3>
-__global__ void __launch_bounds__(kThreads, D3 ? 2 : (CG == 12 ? 4 : 3))
-k_degrid_table(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__ out) {
-    constexpr int SPW = DegridShape<CG>::SPW;
-    // Staged cell stride in float2.  2D: padded to an odd number of 16-byte
-    // chunks (conflict-free staging stores; the region copy is a large share
-    // of a 2D item's work).  3D: unpadded (the copy is a few percent of an
-    // item's work there and the region is large).
-    constexpr int CS = (D3 || CG == 12) ? CG : CG + 2;
-    static_assert(CG >= 4, "table degridding stages coil pairs");
-    extern __shared__ float4 smem_raw[];
-    const KParams &k = a.k;
-    const WorkItem it = a.items[blockIdx.x];
-    const int grp = blockIdx.y;
-    const int b0 = grp * CG;
-    const int f = it.f, tx = it.tx, ty = it.ty, tz = it.tz;
-    const int org0 = tx * k.tile[0], org1 = ty * k.tile[1], org2 = tz * k.tile[2];
-    const int R0 = region_dim(k, 0), R1 = region_dim(k, 1), R2 = region_dim(k, 2);
-    const int h2 = D3 ? k.hw : 0;
-    float2 *tile_s = reinterpret_cast<float2 *>(smem_raw);
-
-    const int warp = threadIdx.x >> 5;
-
-    DegRaw cur;
-    int base = it.begin + warp * SPW;
-    if (base < it.end) degrid_table_load_raw<CG, NT, D3>(a, it, base, cur);
-    {
-        // Region staging through registers.  Thread e of the CTA takes cells
-        // e, e + kThreads, ... of the region in x-fastest order (every load
-        // instruction is a coalesced run of one coil plane, no idle lanes at
-        // row ends), loads all CG coils of UC cells before storing any (the
-        // loads in flight cover the memory latency), then stores each cell's
-        // coils as 16-byte chunks (with padded cells, the chunks that a warp
-        // stores at once fall into different banks).
-        constexpr int UC = CG <= 4 ? 2 : 1;   // cells in flight per thread
-        const int ncell = R0 * R1 * R2;
-        const int gx0 = org0 - k.hw, gy0 = org1 - k.hw, gz0 = org2 - h2;
-        const int64_t pstride = (int64_t)a.F * a.kl.s_bf;
-        const float2 *fbase = grid + (int64_t)b0 * pstride + (int64_t)f * a.kl.s_bf;
-        for (int e0 = threadIdx.x; e0 < ncell; e0 += UC * kThreads) {
-            float2 v[UC][CG];
-#pragma unroll
-            for (int u = 0; u < UC; u++) {
-                const int e = e0 + u * kThreads;
-                const int row = e / R0, xo = e - row * R0;
-                const int rz = row / R1, ry = row - rz * R1;
-                int gx = gx0 + xo, gy = gy0 + ry, gz = gz0 + rz;
-                gx = gx < 0 ? gx + k.mos[0] : (gx >= k.mos[0] ? gx - k.mos[0] : gx);
-                gy = gy < 0 ? gy + k.mos[1] : (gy >= k.mos[1] ? gy - k.mos[1] : gy);
-                gz = gz < 0 ? gz + k.mos[2] : (gz >= k.mos[2] ? gz - k.mos[2] : gz);
-                const float2 *src = fbase + (int64_t)gz * a.kl.s_z + (int64_t)gy * a.kl.s_y + gx;
-                const bool in = e < ncell;
-#pragma unroll
-                for (int c = 0; c < CG; c++)
-                    v[u][c] = (in && b0 + c < a.nb) ? __ldg(src + c * pstride) : make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int u = 0; u < UC; u++) {
-                const int e = e0 + u * kThreads;
-                if (e < ncell) {
-                    float4 *cell = reinterpret_cast<float4 *>(tile_s + (size_t)e * CS);
-#pragma unroll
-                    for (int q = 0; q < CG / 2; q++)
-                        cell[q] = make_float4(v[u][2 * q].x, v[u][2 * q].y, v[u][2 * q + 1].x, v[u][2 * q + 1].y);
-                }
-            }
-        }
-        {
-            // zero pad after the region: a tap with zero weight beyond the
-            // footprint may read up to one row and one cell past it
-            const int npad = (R0 + 1) * CS;
-            for (int e = threadIdx.x; e < npad; e += kThreads)
-                tile_s[(size_t)R0 * R1 * R2 * CS + e] = make_float2(0.f, 0.f);
-        }
-    }
-    __syncthreads();
-    degrid_table_passes<CG, NT, D3>(a, it, b0, org0, org1, org2, tile_s, out, cur);
-}
-
-__global__ void k_sum_groups(const float *__restrict__ part, int ngroups, int64_t n,
-                             float *__restrict__ out) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    float s = 0.f;
-    for (int g = 0; g < ngroups; g++) s += part[(int64_t)g * n + e];
-    out[e] = s;
 }
 
 // ------------------------------------------------------------ launchers ---
@@ -1214,52 +964,6 @@ static void degrid_dispatch(int cg, const ConvArgs &a, dim3 g, size_t smem, cons
     }
 }
 
-static size_t degrid_table_smem(const KParams &k, int cg) {
-    const int cs = (k.D == 3 || cg == 12) ? cg : cg + 2;   // cell stride of k_degrid_table
-    const size_t pad = (size_t)(region_dim(k, 0) + 1) * cs;
-    return ((size_t)region_dim(k, 0) * region_dim(k, 1) * region_dim(k, 2) * cs + pad) * sizeof(float2);
-}
-
-template <int CG, int NT, bool D3>
-static void degrid_table_launch(const ConvArgs &a, dim3 g, size_t smem, const float2 *grid, float2 *out,
-                                cudaStream_t st) {
-    auto kern = k_degrid_table<CG, NT, D3>;
-    if (smem > 48 * 1024)
-        GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<g, kThreads, smem, st>>>(a, grid, out); ::gb::note_launch();
-}
-
-template <int CG, bool D3>
-static void degrid_table_nt(int nt, const ConvArgs &a, dim3 g, size_t smem, const float2 *grid, float2 *out,
-                            cudaStream_t st) {
-    switch (nt) {
-        case 4: degrid_table_launch<CG, 4, D3>(a, g, smem, grid, out, st); break;
-        case 5: degrid_table_launch<CG, 5, D3>(a, g, smem, grid, out, st); break;
-        case 6: degrid_table_launch<CG, 6, D3>(a, g, smem, grid, out, st); break;
-        case 7: degrid_table_launch<CG, 7, D3>(a, g, smem, grid, out, st); break;
-        default: degrid_table_launch<CG, 8, D3>(a, g, smem, grid, out, st); break;
-    }
-}
-
-static void degrid_table_dispatch(int cg, int nt, bool d3, const ConvArgs &a, dim3 g, size_t smem,
-                                  const float2 *grid, float2 *out, cudaStream_t st) {
-    if (d3) {
-        switch (cg) {
-            case 4: degrid_table_nt<4, true>(nt, a, g, smem, grid, out, st); break;
-            case 8: degrid_table_nt<8, true>(nt, a, g, smem, grid, out, st); break;
-            case 12: degrid_table_nt<12, true>(nt, a, g, smem, grid, out, st); break;
-            default: degrid_table_nt<16, true>(nt, a, g, smem, grid, out, st); break;
-        }
-    } else {
-        switch (cg) {
-            case 4: degrid_table_nt<4, false>(nt, a, g, smem, grid, out, st); break;
-            case 8: degrid_table_nt<8, false>(nt, a, g, smem, grid, out, st); break;
-            case 12: degrid_table_nt<12, false>(nt, a, g, smem, grid, out, st); break;
-            default: degrid_table_nt<16, false>(nt, a, g, smem, grid, out, st); break;
-        }
-    }
-}
-
 static int degrid_cg(NufftPlan &p, int nb, bool grad = false) {
     int cg = choose_cg(p.tiling.cg, nb);
     while (cg > 1 && degrid_smem(p.kp, cg, grad) > 200 * 1024) cg /= 2;
@@ -1272,33 +976,31 @@ void launch_degrid(NufftPlan &p, const float2 *grid, float2 *samples, int nb, Sa
                    const KLayout *kl) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "preprocess has not been called");
     int cg = degrid_cg(p, nb);
+    const bool comp = (p.flags & GB_FLAG_COMPENSATED) != 0;
     // 12 coils (or a multiple of 12): one group of 12 for the table kernel
     // instead of a group of 16 with 4 empty coil slots
-    const int nt12 = (int)std::floor(p.W) + 1;
-    if (nb % 12 == 0 && nb % 16 != 0 && cg >= 8 && !(p.flags & GB_FLAG_COMPENSATED) && p.D >= 2 &&
-        nt12 >= 4 && nt12 <= kWMax && degrid_table_smem(p.kp, 12) <= 220 * 1024)
-        cg = 12;
+    if (nb % 12 == 0 && nb % 16 != 0 && cg >= 8 && degrid_table_ok(p, 12)) cg = 12;
     const int ncg = (nb + cg - 1) / cg;
     ConvArgs a = make_args(p, nb, layout, dcw, dcw_pow, sign_fold, accumulate);
     if (kl) a.kl = *kl;
     a.items = p.deg_items.get();
     a.n_items = p.n_deg_items;
     if (p.n_deg_items == 0) return;
-    dim3 g(p.n_deg_items, ncg);
-    const int nt = (int)std::floor(p.W) + 1;   // most taps a footprint can have per dimension
-    if (!(p.flags & GB_FLAG_COMPENSATED) && p.D >= 2 && cg >= 4 && nt >= 4 && nt <= kWMax &&
-        degrid_table_smem(p.kp, cg) <= 220 * 1024) {
-        degrid_table_dispatch(cg, nt, p.D == 3, a, g, degrid_table_smem(p.kp, cg), grid, samples, st);
-    } else {
-        const size_t smem = degrid_smem(p.kp, cg);
-        if (p.flags & GB_FLAG_COMPENSATED)
-            degrid_dispatch<true, false>(cg, a, g, smem, grid, samples, nullptr, nullptr, st);
-        else
-            degrid_dispatch<false, false>(cg, a, g, smem, grid, samples, nullptr, nullptr, st);
+    if (degrid_table_ok(p, cg)) {
+        launch_degrid_table(p, a, cg, ncg, comp, grid, samples, st);
+        return;
     }
+    dim3 g(p.n_deg_items, ncg);
+    const size_t smem = degrid_smem(p.kp, cg);
+    if (comp)
+        degrid_dispatch<true, false>(cg, a, g, smem, grid, samples, nullptr, nullptr, st);
+    else
+        degrid_dispatch<false, false>(cg, a, g, smem, grid, samples, nullptr, nullptr, st);
     GB_CUDA(cudaGetLastError());
 }
 
+// Every sample has one home item, so every gradient is written; the coil
+// groups of an item are summed by its CTA in turn.
 void launch_traj_grad(NufftPlan &p, const float2 *grid, const float2 *weights, int nb,
                       const float *dcw, float *grad, bool sign_fold, cudaStream_t st, const KLayout *kl) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "preprocess has not been called");
@@ -1308,24 +1010,15 @@ void launch_traj_grad(NufftPlan &p, const float2 *grid, const float2 *weights, i
     if (kl) a.kl = *kl;
     a.items = p.deg_items.get();
     a.n_items = p.n_deg_items;
-    const int64_t n = p.Mtot * p.D;
-    DevBuf<float> part;
-    float *target = grad;
-    if (ncg > 1) {
-        part.ensure((size_t)ncg * n);
-        target = part.get();
+    a.ncg = ncg;
+    if (p.n_deg_items == 0) return;
+    if (grad_table_ok(p, cg)) {
+        launch_grad_table(p, a, cg, grid, weights, grad, st);
+        return;
     }
-    GB_CUDA(cudaMemsetAsync(target, 0, (size_t)ncg * n * sizeof(float), st));
-    if (p.n_deg_items > 0) {
-        dim3 g(p.n_deg_items, ncg);
-        degrid_dispatch<false, true>(cg, a, g, degrid_smem(p.kp, cg, true), grid, nullptr, weights, target, st);
-        GB_CUDA(cudaGetLastError());
-    }
-    if (ncg > 1) {
-        k_sum_groups<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part.get(), ncg, n, grad); ::gb::note_launch();
-        GB_CUDA(cudaGetLastError());
-        GB_CUDA(cudaStreamSynchronize(st));   // `part` is freed on return
-    }
+    degrid_dispatch<false, true>(cg, a, dim3(p.n_deg_items), degrid_smem(p.kp, cg, true), grid, nullptr, weights, grad,
+                                 st);
+    GB_CUDA(cudaGetLastError());
 }
 
 }  // namespace gb
