@@ -287,7 +287,6 @@ struct NufftPlan {
     int split_counter_groups = 0;
     DevBuf<float2> partials;               // [n_slots][cg_groups][cells*cg]
     int64_t total_pairs = 0;
-    std::vector<uint32_t> h_home_counts;   // per (frame, tile), for tuning
 
     // deapodization: per-dim reciprocal of the 1D kernel transform
     DevBuf<float> deap_img;   // [D][maxN]    1/psi_d(n + (mos-N)/2)

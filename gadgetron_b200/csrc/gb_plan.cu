@@ -282,14 +282,6 @@ __global__ void k_scale_bin(KParams k, const float *__restrict__ traj, int64_t M
     idx[j] = (uint32_t)j;
 }
 
-__global__ void k_gather_pos(int D, int64_t M, const float *__restrict__ pos,
-                             const uint32_t *__restrict__ perm, float *__restrict__ pos_sorted) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M) return;
-    uint32_t j = perm[i];
-    for (int d = 0; d < D; d++) pos_sorted[(int64_t)d * M + i] = pos[(int64_t)d * M + j];
-}
-
 // Run offsets of a sorted key array: off[k] = first index whose key is >= k,
 // off[nkeys] = n (no atomics: every thread fills the offsets between the key
 // before it and its own).
@@ -327,33 +319,34 @@ __device__ __forceinline__ int touched_tiles(const KParams &k, const float *s, i
     return total;
 }
 
-// Per sorted sample and dimension, the 1D kernel weights of its taps
-// t = 0..kWMax-1 at padded-grid cells ceil(s - W/2) + t (zero beyond the
-// footprint): the values the convolution kernels would compute from the
-// position, evaluated once per trajectory.
-__global__ void k_weight_table(KParams k, int64_t M, const float *__restrict__ pos_sorted,
-                               float4 *__restrict__ wtab) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M * k.D) return;
-    const int64_t j = e / k.D;
-    const int d = (int)(e - j * k.D);
-    const float s = pos_sorted[(int64_t)d * M + j];
-    const int lo = (int)ceilf(s - k.radius);
-    const int n = (int)floorf(s + k.radius) - lo + 1;
-    float w[kWMax];
-#pragma unroll
-    for (int t = 0; t < kWMax; t++)
-        w[t] = t < n ? kb_weight_1d(fabsf(s - (float)(lo + t)), k.mos_f[d], k.one_over_W, k.beta[d], k.radius) : 0.f;
-    wtab[2 * e] = make_float4(w[0], w[1], w[2], w[3]);
-    wtab[2 * e + 1] = make_float4(w[4], w[5], w[6], w[7]);
-}
-
-__global__ void k_count_pairs(KParams k, int64_t M, const float *__restrict__ pos_sorted,
-                              uint32_t *__restrict__ cnt) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Per sorted sample: its position, per dimension the 1D kernel weights of its
+// taps t = 0..kWMax-1 at padded-grid cells ceil(s - W/2) + t (zero beyond the
+// footprint; the values the convolution kernels would compute from the
+// position, evaluated once per trajectory), and the number of tiles it touches.
+// One launch for the three (a real-time frame's samples are a microsecond's
+// work each).
+__global__ void k_sample_tables(KParams k, int64_t M, const float *__restrict__ pos, const uint32_t *__restrict__ perm,
+                                float *__restrict__ pos_sorted, float4 *__restrict__ wtab, uint32_t *__restrict__ cnt) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
+    const uint32_t j = perm[i];
     float s[kMaxD] = {0.f, 0.f, 0.f};
-    for (int d = 0; d < k.D; d++) s[d] = pos_sorted[(int64_t)d * M + i];
+#pragma unroll
+    for (int d = 0; d < kMaxD; d++) {
+        if (d >= k.D) break;
+        s[d] = pos[(int64_t)d * M + j];
+        pos_sorted[(int64_t)d * M + i] = s[d];
+        const int lo = (int)ceilf(s[d] - k.radius);
+        const int n = (int)floorf(s[d] + k.radius) - lo + 1;
+        float w[kWMax];
+#pragma unroll
+        for (int t = 0; t < kWMax; t++)
+            w[t] = t < n ? kb_weight_1d(fabsf(s[d] - (float)(lo + t)), k.mos_f[d], k.one_over_W, k.beta[d], k.radius)
+                         : 0.f;
+        float4 *row = wtab + 2 * (i * k.D + d);
+        row[0] = make_float4(w[0], w[1], w[2], w[3]);
+        row[1] = make_float4(w[4], w[5], w[6], w[7]);
+    }
     int tl[kMaxD][3], nt[kMaxD];
     cnt[i] = (uint32_t)touched_tiles(k, s, tl, nt);
 }
@@ -380,47 +373,60 @@ __global__ void k_write_pairs(KParams k, int64_t M, const float *__restrict__ po
             }
 }
 
-// Pair rows for the brick gridding kernel: one thread per (pair,
-// dimension) lays the sample's tap weights (from the weight table, unsigned)
-// over the tile's extent in that dimension -- tap t at tile-local cell
-// (ceil(s - W/2) + t - pad/2 - tile origin) mod mos when that falls inside the
-// tile, zero elsewhere -- and records the tile-local footprint range (bytes).
-__global__ void k_pair_rows(KParams k, int64_t M, int64_t npairs, const float *__restrict__ pos_sorted,
-                            const float *__restrict__ wtab, const uint32_t *__restrict__ pair_key,
-                            const uint32_t *__restrict__ pair_sample, float *__restrict__ rows, int row_floats,
-                            uint16_t *__restrict__ ranges) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= npairs * k.D) return;
-    const int64_t q = e / k.D;
-    const int d = (int)(e - q * k.D);
+// Pair rows for the brick gridding kernel: one thread per 16-byte chunk of a
+// pair's row (a block serves blockDim / chunks pairs, its stores are one
+// contiguous run) lays the sample's tap weights (from the weight table,
+// unsigned) over the tile's extent in the chunk's dimension -- tap t at
+// tile-local cell (ceil(s - W/2) + t - pad/2 - tile origin) mod mos when that
+// falls inside the tile, zero elsewhere; the first chunk of a dimension also
+// records the tile-local footprint range (bytes).  Preprocess of 5.12 M
+// kooshball samples (13.3 M rows): 3.35 -> 2.35 ms, of 64 frames (1.29 M
+// samples): 2.5 -> 1.2 ms with the work lists below, of one 8192-sample frame:
+// 0.39 -> 0.27 ms with the short sort runs.
+__global__ void __launch_bounds__(256) k_pair_rows(KParams k, int64_t M, int64_t npairs,
+                                                   const float *__restrict__ pos_sorted,
+                                                   const float *__restrict__ wtab,
+                                                   const uint32_t *__restrict__ pair_key,
+                                                   const uint32_t *__restrict__ pair_sample, float *__restrict__ rows,
+                                                   int row_floats, uint16_t *__restrict__ ranges) {
+    const int chunks = row_floats >> 2, ppb = 256 / chunks;
+    const int lp = (int)threadIdx.x / chunks, ch = (int)threadIdx.x - lp * chunks;
+    const int64_t q = (int64_t)blockIdx.x * ppb + lp;
+    if (lp >= ppb || q >= npairs) return;
+    // tile extents are multiples of 4 in x and y, so a chunk lies in one
+    // dimension (z may end short of the row's last chunk: zeros)
+    const int c0 = 4 * ch;
+    const int d = c0 < k.tile[0] ? 0 : (c0 < k.tile[0] + k.tile[1] ? 1 : 2);
+    const int first = d == 0 ? 0 : (d == 1 ? k.tile[0] : k.tile[0] + k.tile[1]);
     const uint32_t si = pair_sample[q];
     const uint32_t tile = pair_key[q] % (uint32_t)k.ntiles_total;
-    const int tc = d == 0 ? (int)(tile % k.ntiles[0])
-                          : (d == 1 ? (int)((tile / k.ntiles[0]) % k.ntiles[1])
-                                    : (int)(tile / (k.ntiles[0] * k.ntiles[1])));
-    const int Td = k.tile[d];
-    const int org = tc * Td;
+    const uint32_t nx = (uint32_t)k.ntiles[0], ny = (uint32_t)k.ntiles[1];
+    const int tc = (int)(d == 0 ? tile % nx : (d == 1 ? (tile / nx) % ny : tile / (nx * ny)));
+    const int Td = d == 0 ? k.tile[0] : (d == 1 ? k.tile[1] : k.tile[2]);
+    const int mos = d == 0 ? k.mos[0] : (d == 1 ? k.mos[1] : k.mos[2]);
+    const int ntl = d == 0 ? k.ntiles[0] : (d == 1 ? k.ntiles[1] : k.ntiles[2]);
     const float sp = pos_sorted[(int64_t)d * M + si];
     const int lo = (int)ceilf(sp - k.radius);
     const int n = min((int)floorf(sp + k.radius) - lo + 1, kWMax);
-    int a0 = lo - k.hw - org;   // tile-local footprint start, mod mos
-    a0 = a0 < 0 ? a0 + k.mos[d] : (a0 >= k.mos[d] ? a0 - k.mos[d] : a0);
-    float *row = rows + q * row_floats;
-    float *wr = row + (d == 0 ? 0 : (d == 1 ? k.tile[0] : k.tile[0] + k.tile[1]));
+    int a0 = lo - k.hw - tc * Td;   // tile-local footprint start, mod mos
+    a0 = a0 < 0 ? a0 + mos : (a0 >= mos ? a0 - mos : a0);
     const float *taps = wtab + ((int64_t)si * k.D + d) * kWMax;
-    for (int c = 0; c < Td; c++) {
+    float w[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int c = c0 - first + i;
         int t = c - a0;
-        if (t < 0) t += k.mos[d];
-        wr[c] = t < n ? taps[t] : 0.f;
+        if (t < 0) t += mos;
+        w[i] = (c < Td && t < n) ? taps[t] : 0.f;
     }
-    if (d == 0)
-        for (int c = k.tile[0] + k.tile[1] + (k.D == 3 ? k.tile[2] : 0); c < row_floats; c++) row[c] = 0.f;
+    reinterpret_cast<float4 *>(rows + q * row_floats)[ch] = make_float4(w[0], w[1], w[2], w[3]);
+    if (c0 != first) return;
     int rlo, rhi;
-    if (k.ntiles[d] == 1) {   // the footprint may wrap inside the tile
+    if (ntl == 1) {   // the footprint may wrap inside the tile
         rlo = 0;
         rhi = Td - 1;
     } else {
-        const int st = (a0 < Td) ? a0 : a0 - k.mos[d];
+        const int st = (a0 < Td) ? a0 : a0 - mos;
         rlo = max(st, 0);
         rhi = min(st + n - 1, Td - 1);
     }
@@ -514,18 +520,14 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
                                                                   key.get(), idx.get(), err.get()); ::gb::note_launch();
         GB_CUDA(cudaGetLastError());
         sort_pairs(key.get(), key_sorted.get(), idx.get(), p.perm.get(), M, bits_for(nkeys), p.pp_sort, s);
-        k_gather_pos<<<(unsigned)((M + TB - 1) / TB), TB, 0, s>>>(D, M, pos.get(), p.perm.get(),
-                                                                   p.pos_sorted.get()); ::gb::note_launch();
-        GB_CUDA(cudaGetLastError());
-        k_weight_table<<<(unsigned)((M * D + TB - 1) / TB), TB, 0, s>>>(k, M, p.pos_sorted.get(),
-                                                                        reinterpret_cast<float4 *>(p.wtab.get())); ::gb::note_launch();
+        k_sample_tables<<<(unsigned)((M + 127) / 128), 128, 0, s>>>(k, M, pos.get(), p.perm.get(), p.pos_sorted.get(),
+                                                                     reinterpret_cast<float4 *>(p.wtab.get()),
+                                                                     pcnt.get()); ::gb::note_launch();
         GB_CUDA(cudaGetLastError());
         k_sorted_offsets<<<(unsigned)((M + TB) / TB), TB, 0, s>>>(key_sorted.get(), M, (uint32_t)nkeys,
                                                                  p.home_off.get()); ::gb::note_launch();
         GB_CUDA(cudaGetLastError());
         GB_CUDA(cudaMemsetAsync(pcnt.get() + M, 0, sizeof(uint32_t), s));
-        k_count_pairs<<<(unsigned)((M + TB - 1) / TB), TB, 0, s>>>(k, M, p.pos_sorted.get(), pcnt.get()); ::gb::note_launch();
-        GB_CUDA(cudaGetLastError());
         exclusive_scan(pcnt.get(), poff.get(), M + 1, p.pp_sort, s);
     });
     uint32_t *hs = stage_words(p, 2);
@@ -570,9 +572,10 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
                                                                                (uint32_t)nkeys, p.grid_off.get()); ::gb::note_launch();
         GB_CUDA(cudaGetLastError());
         if (rows) {
-            k_pair_rows<<<(unsigned)(((int64_t)npairs * D + TB - 1) / TB), TB, 0, s>>>(
-                k, M, npairs, p.pos_sorted.get(), p.wtab.get(), pkey_sorted.get(), p.grid_list.get(), p.pair_rows.get(),
-                rf, reinterpret_cast<uint16_t *>(p.pair_rng.get())); ::gb::note_launch();
+            const int64_t ppb = 256 / (rf / 4);
+            k_pair_rows<<<(unsigned)((npairs + ppb - 1) / ppb), 256, 0, s>>>(
+                k, M, (int64_t)npairs, p.pos_sorted.get(), p.wtab.get(), pkey_sorted.get(), p.grid_list.get(),
+                p.pair_rows.get(), rf, reinterpret_cast<uint16_t *>(p.pair_rng.get())); ::gb::note_launch();
             GB_CUDA(cudaGetLastError());
         }
     });
@@ -593,27 +596,6 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
     p.prepped = true;
 }
 
-// Stable sort of work items by length, longest first (the same order as a
-// std::stable_sort on that key): a counting sort when the lengths are small,
-// as they are for tile lists -- this runs in every preprocess.
-static void sort_items_by_length(std::vector<WorkItem> &v) {
-    if (v.size() < 2) return;
-    int maxlen = 0;
-    for (const WorkItem &w : v) maxlen = std::max(maxlen, w.end - w.begin);
-    if (maxlen > (1 << 16)) {
-        std::stable_sort(v.begin(), v.end(), [](const WorkItem &a, const WorkItem &b) {
-            return (a.end - a.begin) > (b.end - b.begin);
-        });
-        return;
-    }
-    std::vector<uint32_t> start((size_t)maxlen + 2, 0u);
-    for (const WorkItem &w : v) start[(size_t)(maxlen - (w.end - w.begin)) + 1]++;
-    for (size_t i = 1; i < start.size(); i++) start[i] += start[i - 1];
-    std::vector<WorkItem> out(v.size());
-    for (const WorkItem &w : v) out[start[(size_t)(maxlen - (w.end - w.begin))]++] = w;
-    v.swap(out);
-}
-
 // Host-side work lists: degridding chunks of home samples, gridding tiles
 // (heavy tiles split into chunks reduced by the last CTA).
 void plan_build_work(NufftPlan &p, cudaStream_t st) {
@@ -624,48 +606,30 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     GB_CUDA(cudaMemcpyAsync(hoff, p.home_off.get(), (nkeys + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GB_CUDA(cudaMemcpyAsync(goff, p.grid_off.get(), (nkeys + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GB_CUDA(cudaStreamSynchronize(st));
-    p.h_home_counts.resize(nkeys);
-    for (uint32_t i = 0; i < nkeys; i++) p.h_home_counts[i] = hoff[i + 1] - hoff[i];
-
     // Degridding items: chunks of at most `deg_chunk` home samples.
     const int64_t M = p.Mtot;
     // (large enough that a tile is staged once or a few times; the region
     // copy is a large share of an item's work in 2D)
     int deg_chunk = (int)std::max<int64_t>(256, std::min<int64_t>(1024, M / (148 * 4) + 1));
-    std::vector<WorkItem> deg;
-    // frame and tile coordinates of key 0, 1, ... in turn
-    struct TileCounter {
-        const KParams &k;
-        int f = 0, tx = 0, ty = 0, tz = 0;
-        void place(WorkItem &w) const {
-            w.f = f;
-            w.tx = tx;
-            w.ty = ty;
-            w.tz = tz;
+    // Both lists run longest item first, equal lengths in key order: a
+    // counting sort on the length, written straight into the upload staging
+    // (this runs in every preprocess).  First the counts.
+    auto starts = [](std::vector<uint32_t> &count) {   // count[len] -> start of the run of that length
+        uint32_t run = 0;
+        for (size_t l = count.size(); l-- > 0;) {
+            const uint32_t c = count[l];
+            count[l] = run;
+            run += c;
         }
-        void step() {
-            if (++tx < k.ntiles[0]) return;
-            tx = 0;
-            if (++ty < k.ntiles[1]) return;
-            ty = 0;
-            if (++tz < k.ntiles[2]) return;
-            tz = 0;
-            f++;
-        }
+        return run;
     };
-    TileCounter dt{k};
-    for (uint32_t key = 0; key < nkeys; key++, dt.step()) {
-        uint32_t b = hoff[key], e = hoff[key + 1];
-        for (uint32_t s = b; s < e; s += deg_chunk) {
-            WorkItem w{};
-            dt.place(w);
-            w.begin = (int)s;
-            w.end = (int)std::min<uint32_t>(e, s + deg_chunk);
-            w.split = -1;
-            deg.push_back(w);
-        }
+    std::vector<uint32_t> deg_at((size_t)deg_chunk + 1, 0u);
+    for (uint32_t key = 0; key < nkeys; key++) {
+        const uint32_t len = hoff[key + 1] - hoff[key], full = len / deg_chunk;
+        deg_at[deg_chunk] += full;
+        if (len > full * (uint32_t)deg_chunk) deg_at[len - full * deg_chunk]++;
     }
-    sort_items_by_length(deg);
+    const size_t n_deg = starts(deg_at);
 
     // Gridding items: tiles of at most split_len pairs as they are, longer ones
     // in chunks.  The samples of a dense tile (a radial centre) crowd into one
@@ -677,65 +641,84 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     const int64_t total = goff[nkeys];
     const int64_t avg = total / std::max<uint32_t>(1, nkeys);
     const int split_len = (int)std::max<int64_t>(256, 2 * avg);
-    const int fine_len = (int)std::max<int64_t>(96, avg);
-    std::vector<WorkItem> light, heavy[2];   // [0] fine, [1] coarse
-    std::vector<SplitInfo> splits[2];
+    const int most[2] = {(int)std::max<int64_t>(96, avg), split_len};   // chunk lengths: fine, coarse
+    // equal lengths share a run up to 64K pairs; the few lists above keep key order in the last one
+    const uint32_t cap = (uint32_t)std::min(split_len, 1 << 16);
+    std::vector<uint32_t> light_at((size_t)cap + 1, 0u);
+    size_t n_heavy[2] = {0, 0}, n_splits = 0;
+    for (uint32_t key = 0; key < nkeys; key++) {
+        const uint32_t len = goff[key + 1] - goff[key];
+        if ((int)len <= split_len) {
+            light_at[std::min(len, cap)]++;
+            continue;
+        }
+        n_splits++;
+        for (int c = 0; c < 2; c++) n_heavy[c] += (len + most[c] - 1) / most[c];
+    }
+    const size_t n_light = starts(light_at);
+
+    // Then the items: [degridding][fine chunks, light tiles, coarse chunks][splits fine, coarse]
+    const size_t n_grd = n_heavy[0] + n_light + n_heavy[1];
+    const size_t bd = n_deg * sizeof(WorkItem), bg = n_grd * sizeof(WorkItem), bs = 2 * n_splits * sizeof(SplitInfo);
+    unsigned char *up = upload_room(p, bd + bg + bs);
+    WorkItem *deg = reinterpret_cast<WorkItem *>(up), *grd = deg + n_deg;
+    SplitInfo *splits = reinterpret_cast<SplitInfo *>(grd + n_grd);
+    WorkItem *light = grd + n_heavy[0], *heavy[2] = {grd, light + n_light};
     int slots[2] = {0, 0};
-    TileCounter gt{k};
-    for (uint32_t key = 0; key < nkeys; key++, gt.step()) {
-        const uint32_t b = goff[key], e = goff[key + 1];
-        const uint32_t len = e - b;
-        WorkItem w{};
-        gt.place(w);
+    size_t split = 0;
+    WorkItem w{};   // frame and tile of the key at hand
+    for (uint32_t key = 0; key < nkeys; key++) {
+        const uint32_t hb = hoff[key], he = hoff[key + 1], b = goff[key], e = goff[key + 1], len = e - b;
+        w.split = -1;
+        w.chunk = 0;
+        for (uint32_t s = hb; s < he; s += deg_chunk) {
+            w.begin = (int)s;
+            w.end = (int)std::min<uint32_t>(he, s + deg_chunk);
+            deg[deg_at[w.end - w.begin]++] = w;
+        }
         if ((int)len <= split_len) {
             w.begin = (int)b;
             w.end = (int)e;
-            w.split = -1;
-            light.push_back(w);
-            continue;
-        }
-        for (int c = 0; c < 2; c++) {
-            const uint32_t most = (uint32_t)(c == 0 ? fine_len : split_len);
-            const uint32_t nch = (len + most - 1) / most, per = (len + nch - 1) / nch;
-            w.split = (int)splits[c].size();
-            splits[c].push_back(SplitInfo{slots[c], (int)nch});
-            for (uint32_t q = 0; q < nch; q++) {
-                w.begin = (int)(b + q * per);
-                w.end = (int)std::min<uint32_t>(e, b + (q + 1) * per);
-                w.chunk = (int)q;
-                heavy[c].push_back(w);
+            light[light_at[std::min(len, cap)]++] = w;
+        } else {
+            for (int c = 0; c < 2; c++) {
+                const uint32_t nch = (len + most[c] - 1) / most[c], per = (len + nch - 1) / nch;
+                w.split = (int)split;
+                splits[c * n_splits + split] = SplitInfo{slots[c], (int)nch};
+                for (uint32_t q = 0; q < nch; q++) {
+                    w.begin = (int)std::min<uint32_t>(e, b + q * per);
+                    w.end = (int)std::min<uint32_t>(e, b + (q + 1) * per);
+                    w.chunk = (int)q;
+                    *heavy[c]++ = w;
+                }
+                slots[c] += (int)nch;
             }
-            slots[c] += (int)nch;
+            split++;
+        }
+        if (++w.tx == k.ntiles[0]) {
+            w.tx = 0;
+            if (++w.ty == k.ntiles[1]) {
+                w.ty = 0;
+                if (++w.tz == k.ntiles[2]) {
+                    w.tz = 0;
+                    w.f++;
+                }
+            }
         }
     }
-    sort_items_by_length(light);
-    std::vector<WorkItem> grd(heavy[0]);
-    grd.insert(grd.end(), light.begin(), light.end());
-    p.n_light_items = (int)light.size();
-    p.n_coarse_items = (int)heavy[1].size();
+    p.n_deg_items = (int)n_deg;
+    p.deg_items.ensure(std::max<size_t>(1, n_deg));
+    p.n_grd_items = (int)(n_heavy[0] + n_light);   // of a launch; the coarse chunks follow
+    p.n_light_items = (int)n_light;
+    p.n_coarse_items = (int)n_heavy[1];
     p.n_coarse_slots = slots[1];
-
-    p.n_deg_items = (int)deg.size();
-    p.deg_items.ensure(std::max<size_t>(1, deg.size()));
-    p.n_grd_items = (int)grd.size();
-    grd.insert(grd.end(), heavy[1].begin(), heavy[1].end());   // after the n_grd_items of a launch
-    p.grd_items.ensure(std::max<size_t>(1, grd.size()));
-    p.n_splits = (int)splits[0].size();
+    p.grd_items.ensure(std::max<size_t>(1, n_grd));
+    p.n_splits = (int)n_splits;
     p.n_slots = slots[0];
-    std::vector<SplitInfo> both(splits[0]);
-    both.insert(both.end(), splits[1].begin(), splits[1].end());
-    p.splits.ensure(std::max<size_t>(1, both.size()));
-    // The three lists go up from pinned staging (asynchronous; the staging
-    // is not rewritten before these copies have been read).
-    const size_t bd = deg.size() * sizeof(WorkItem), bg = grd.size() * sizeof(WorkItem);
-    const size_t bs = both.size() * sizeof(SplitInfo);
-    unsigned char *up = upload_room(p, bd + bg + bs);
-    if (bd) std::memcpy(up, deg.data(), bd);
-    if (bg) std::memcpy(up + bd, grd.data(), bg);
-    if (bs) std::memcpy(up + bd + bg, both.data(), bs);
-    if (bd) GB_CUDA(cudaMemcpyAsync(p.deg_items.get(), up, bd, cudaMemcpyHostToDevice, st));
-    if (bg) GB_CUDA(cudaMemcpyAsync(p.grd_items.get(), up + bd, bg, cudaMemcpyHostToDevice, st));
-    if (bs) GB_CUDA(cudaMemcpyAsync(p.splits.get(), up + bd + bg, bs, cudaMemcpyHostToDevice, st));
+    p.splits.ensure(std::max<size_t>(1, 2 * n_splits));
+    if (bd) GB_CUDA(cudaMemcpyAsync(p.deg_items.get(), deg, bd, cudaMemcpyHostToDevice, st));
+    if (bg) GB_CUDA(cudaMemcpyAsync(p.grd_items.get(), grd, bg, cudaMemcpyHostToDevice, st));
+    if (bs) GB_CUDA(cudaMemcpyAsync(p.splits.get(), splits, bs, cudaMemcpyHostToDevice, st));
     upload_issued(p, st);
     p.split_counter_groups = 0;   // (re)allocated by the gridding launcher
 }

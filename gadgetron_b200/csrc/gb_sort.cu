@@ -11,8 +11,8 @@
 //
 // Radix sort: ceil(end_bit / 11) passes of equal digits of at most 11 bits
 // (a 10-bit key sorts in one pass), each pass three launches over tiles of
-// kSortTile elements (256 threads, 8 warps; a warp owns a contiguous run of
-// kSortTile / 8 elements):
+// 1024 to 4096 elements (256 threads, 8 warps; a warp owns a contiguous run of
+// an eighth of the tile):
 //   upsweep    per-tile digit histogram (shared-memory atomics), written
 //              digit-major: hist[digit * ntiles + tile];
 //   scan       exclusive scan of hist (the global position of every
@@ -37,15 +37,19 @@ namespace {
 
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortPerWarp = 512;                        // 16 rounds of 32
-constexpr int kSortTile = kSortWarps * kSortPerWarp;     // 4096 elements
 constexpr int kMaxRadixBits = 11;
+
+// Elements a warp walks in turn (PW) and elements per tile.  A tile's time is
+// its warps' chains of rounds of 32, so small arrays take short runs: at 8192
+// keys two tiles of 4096 leave 146 SMs idle and cost 15.5 us in the downsweep
+// alone.  Long ones take 512, which keeps the (digit, tile) counts small.
+__host__ __device__ constexpr int sort_tile(int pw) { return kSortWarps * pw; }
 
 constexpr int kScanThreads = 256;
 constexpr int kScanPerThread = 16;
 constexpr int kScanTile = kScanThreads * kScanPerThread;  // 4096 counts
 
-template <int RB>
+template <int RB, int PW>
 __global__ void __launch_bounds__(kSortThreads) k_radix_upsweep(const uint32_t *__restrict__ keys, int64_t n,
                                                                 int shift, int64_t ntiles,
                                                                 uint32_t *__restrict__ hist) {
@@ -53,8 +57,9 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_upsweep(const uint32_t *
     __shared__ uint32_t h[R];
     for (int d = threadIdx.x; d < R; d += kSortThreads) h[d] = 0u;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    for (int i = threadIdx.x; i < kSortTile; i += kSortThreads) {
+    const int64_t base = (int64_t)blockIdx.x * sort_tile(PW);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < sort_tile(PW); i += kSortThreads) {
         const int64_t e = base + i;
         if (e < n) atomicAdd(&h[(keys[e] >> shift) & (R - 1)], 1u);
     }
@@ -63,7 +68,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_upsweep(const uint32_t *
 }
 
 // Shared memory: kSortWarps x 2^RB counters (dynamic, up to 64 KB).
-template <int RB>
+template <int RB, int PW>
 __global__ void __launch_bounds__(kSortThreads)
 k_radix_downsweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
                   uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int64_t n, int shift,
@@ -74,10 +79,10 @@ k_radix_downsweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restri
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < kSortWarps * R; i += kSortThreads) g_sort_cnt[i] = 0u;
     __syncthreads();
-    const int64_t wbase = (int64_t)blockIdx.x * kSortTile + (int64_t)warp * kSortPerWarp;
+    const int64_t wbase = (int64_t)blockIdx.x * sort_tile(PW) + (int64_t)warp * PW;
     const uint32_t lt = (1u << lane) - 1u;
     // per-warp digit counts
-    for (int r = 0; r < kSortPerWarp; r += 32) {
+    for (int r = 0; r < PW; r += 32) {
         const int64_t e = wbase + r + lane;
         const bool ok = e < n;
         const uint32_t d = ok ? (keys_in[e] >> shift) & (R - 1) : (uint32_t)R;
@@ -95,7 +100,7 @@ k_radix_downsweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restri
         }
     }
     __syncthreads();
-    for (int r = 0; r < kSortPerWarp; r += 32) {
+    for (int r = 0; r < PW; r += 32) {
         const int64_t e = wbase + r + lane;
         const bool ok = e < n;
         uint32_t key = 0u, val = 0u;
@@ -116,20 +121,32 @@ k_radix_downsweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restri
     }
 }
 
-template <int RB>
-void radix_pass(const uint32_t *ki, const uint32_t *vi, uint32_t *ko, uint32_t *vo, int64_t n, int shift,
-                int64_t ntiles, uint32_t *hist, uint32_t *scan_tmp, cudaStream_t st) {
+template <int RB, int PW>
+void radix_pass_pw(const uint32_t *ki, const uint32_t *vi, uint32_t *ko, uint32_t *vo, int64_t n, int shift,
+                   int64_t ntiles, uint32_t *hist, uint32_t *scan_tmp, cudaStream_t st) {
     constexpr int R = 1 << RB;
     const size_t smem = (size_t)kSortWarps * R * sizeof(uint32_t);
     if (smem > 48 * 1024)   // set on every call: the attribute belongs to the current device's context
-        GB_CUDA(cudaFuncSetAttribute(k_radix_downsweep<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        GB_CUDA(cudaFuncSetAttribute(k_radix_downsweep<RB, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
-    k_radix_upsweep<RB><<<(unsigned)ntiles, kSortThreads, 0, st>>>(ki, n, shift, ntiles, hist); note_launch();
+    k_radix_upsweep<RB, PW><<<(unsigned)ntiles, kSortThreads, 0, st>>>(ki, n, shift, ntiles, hist); note_launch();
     GB_CUDA(cudaGetLastError());
     exclusive_scan_u32(hist, hist, (int64_t)R * ntiles, scan_tmp, st);
-    k_radix_downsweep<RB><<<(unsigned)ntiles, kSortThreads, smem, st>>>(ki, vi, ko, vo, n, shift, ntiles, hist);
+    k_radix_downsweep<RB, PW><<<(unsigned)ntiles, kSortThreads, smem, st>>>(ki, vi, ko, vo, n, shift, ntiles, hist);
     note_launch();
     GB_CUDA(cudaGetLastError());
+}
+
+int sort_run(int64_t n) { return n <= 32768 ? 128 : (n <= 131072 ? 256 : 512); }
+
+template <int RB>
+void radix_pass(const uint32_t *ki, const uint32_t *vi, uint32_t *ko, uint32_t *vo, int64_t n, int shift,
+                int64_t ntiles, uint32_t *hist, uint32_t *scan_tmp, cudaStream_t st) {
+    switch (sort_run(n)) {
+        case 128: radix_pass_pw<RB, 128>(ki, vi, ko, vo, n, shift, ntiles, hist, scan_tmp, st); break;
+        case 256: radix_pass_pw<RB, 256>(ki, vi, ko, vo, n, shift, ntiles, hist, scan_tmp, st); break;
+        default: radix_pass_pw<RB, 512>(ki, vi, ko, vo, n, shift, ntiles, hist, scan_tmp, st); break;
+    }
 }
 
 // Exclusive scan of the kScanTile counts of each tile in shared memory,
@@ -186,32 +203,72 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const uint32_t *__r
     }
 }
 
-// One block: exclusive scan of a short array, tile after tile with a running
-// carry (a few tiles: one launch instead of three).  In place allowed.
-__global__ void __launch_bounds__(kScanThreads) k_scan_small(const uint32_t *__restrict__ in, int64_t n,
-                                                             uint32_t *__restrict__ out) {
-    __shared__ uint32_t sh[33];
+// One block of 1024 threads: exclusive scan of a short array, 16384 counts at a
+// time with a running carry (one launch instead of three).  In place allowed.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallTile = kSmallThreads * kScanPerThread;
+
+__global__ void __launch_bounds__(kSmallThreads) k_scan_small(const uint32_t *__restrict__ in, int64_t n,
+                                                              uint32_t *__restrict__ out) {
+    __shared__ uint32_t sh[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t carry = 0u;
-    for (int64_t tb = 0; tb < n; tb += kScanTile) {
+    for (int64_t tb = 0; tb < n; tb += kSmallTile) {
         const int64_t base = tb + (int64_t)threadIdx.x * kScanPerThread;
         uint32_t v[kScanPerThread];
         uint32_t s = 0u;
+        if (base + kScanPerThread <= n) {   // arrays start 16-byte aligned
 #pragma unroll
-        for (int i = 0; i < kScanPerThread; i++) {
-            v[i] = base + i < n ? in[base + i] : 0u;
-            s += v[i];
+            for (int i = 0; i < kScanPerThread / 4; i++) {
+                const uint4 q = reinterpret_cast<const uint4 *>(in + base)[i];
+                v[4 * i] = q.x;
+                v[4 * i + 1] = q.y;
+                v[4 * i + 2] = q.z;
+                v[4 * i + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kScanPerThread; i++) v[i] = base + i < n ? in[base + i] : 0u;
         }
-        uint32_t pre = block_exclusive_scan(s, sh);
-        __syncthreads();
-        const uint32_t total = sh[32];
-        pre += carry;
 #pragma unroll
-        for (int i = 0; i < kScanPerThread; i++) {
-            if (base + i < n) out[base + i] = pre;
-            pre += v[i];
+        for (int i = 0; i < kScanPerThread; i++) s += v[i];
+        uint32_t x = s;   // inclusive over the warp, then over the warps
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) sh[warp] = x;
+        __syncthreads();
+        uint32_t w = sh[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, w, 31);
+        const uint32_t before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+        uint32_t pre = carry + (warp > 0 ? before : 0u) + x - s;
+        if (base + kScanPerThread <= n) {
+#pragma unroll
+            for (int i = 0; i < kScanPerThread / 4; i++) {
+                uint4 q;
+                q.x = pre;
+                q.y = q.x + v[4 * i];
+                q.z = q.y + v[4 * i + 1];
+                q.w = q.z + v[4 * i + 2];
+                pre = q.w + v[4 * i + 3];
+                reinterpret_cast<uint4 *>(out + base)[i] = q;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kScanPerThread; i++) {
+                if (base + i < n) out[base + i] = pre;
+                pre += v[i];
+            }
         }
         carry += total;
-        __syncthreads();
+        __syncthreads();   // sh is rewritten by the next round
     }
 }
 
@@ -241,8 +298,8 @@ void scan_scratch_need(int64_t n, size_t *bytes) {
 void exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *tile_scratch, cudaStream_t st) {
     if (n <= 0) return;
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles <= 4) {   // short: one block, one launch
-        k_scan_small<<<1, kScanThreads, 0, st>>>(in, n, out); note_launch();
+    if (n <= 4 * kSmallTile) {   // short: one block, one launch
+        k_scan_small<<<1, kSmallThreads, 0, st>>>(in, n, out); note_launch();
         GB_CUDA(cudaGetLastError());
         return;
     }
@@ -268,7 +325,7 @@ void sort_pairs(const uint32_t *keys_in, uint32_t *keys_out, const uint32_t *val
     end_bit = std::max(1, std::min(end_bit, 32));
     const int passes = (end_bit + kMaxRadixBits - 1) / kMaxRadixBits;
     const int rb = std::max(4, (end_bit + passes - 1) / passes);   // digit bits, 4..11
-    const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
+    const int64_t ntiles = (n + sort_tile(sort_run(n)) - 1) / sort_tile(sort_run(n));
     const int64_t nhist = ntiles << rb;
     size_t scan_bytes = 0;
     scan_scratch_need(nhist, &scan_bytes);
