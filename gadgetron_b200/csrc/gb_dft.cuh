@@ -127,8 +127,34 @@ __device__ __forceinline__ void dft(float2 (&x)[N]) {
         x[4] = csub(m1, cmi(n1));
         x[2] = cadd(m2, cmi(n2));
         x[3] = csub(m2, cmi(n2));
+    } else if constexpr (N == 7) {
+        // X_k = a + sum_m c_(mk) s_m -/+ i sum_m s_(mk) d_m over the pairs
+        // s_m = x_m + x_(7-m), d_m = x_m - x_(7-m), m = 1..3
+        constexpr float c[4] = {1.f, (float)cx_cos2pi(1, 7), (float)cx_cos2pi(2, 7), (float)cx_cos2pi(3, 7)};
+        constexpr float sn[4] = {0.f, (float)cx_sin2pi(1, 7), (float)cx_sin2pi(2, 7), (float)cx_sin2pi(3, 7)};
+        const float2 a = x[0];
+        float2 s[4], d[4];
+#pragma unroll
+        for (int m = 1; m < 4; m++) {
+            s[m] = cadd(x[m], x[7 - m]);
+            d[m] = csub(x[m], x[7 - m]);
+        }
+        x[0] = make_float2(a.x + s[1].x + s[2].x + s[3].x, a.y + s[1].y + s[2].y + s[3].y);
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+            float2 e = a, o = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int m = 1; m < 4; m++) {
+                const int r = (m * k) % 7, q = r > 3 ? 7 - r : r;
+                const float sg = r > 3 ? -sn[q] : sn[q];
+                e = make_float2(e.x + c[q] * s[m].x, e.y + c[q] * s[m].y);
+                o = make_float2(o.x + sg * d[m].x, o.y + sg * d[m].y);
+            }
+            x[k] = cadd(e, cmi(o));
+            x[7 - k] = csub(e, cmi(o));
+        }
     } else {
-        constexpr int R = (N % 4 == 0) ? 4 : (N % 2 == 0 ? 2 : (N % 3 == 0 ? 3 : 5));
+        constexpr int R = (N % 4 == 0) ? 4 : (N % 2 == 0 ? 2 : (N % 3 == 0 ? 3 : (N % 5 == 0 ? 5 : 7)));
         constexpr int M = N / R;
         static_assert(R * M == N, "unsupported register DFT size");
         float2 s[R][M];

@@ -326,8 +326,8 @@ cufftHandle plan_fft_om(NufftPlan &p, int nbf, FftPass pass, cudaStream_t st);
 int64_t fft_band_offset(const NufftPlan &p, int nbf);
 
 // Project-written FFT passes (gb_fft.cu), used instead of cuFFT for D >= 2
-// when every oversampled size is 16 * n2 with n2 in {2, 4, 6, 8, 10, 12, 16,
-// 20, 24, 32, 40}.  fft_cols: `ncols` columns (col / cpp = plane at
+// when every oversampled size is 16 * n2 with n2 in {2, 4, 6, 8, 10, 12, 14,
+// 16, 18, 20, 24, 28, 30, 32, 36, 40}.  fft_cols: `ncols` columns (col / cpp = plane at
 // plane * pstride, col % cpp = offset), points at o * ostride.  fft_rows:
 // `nrows` rows of n contiguous points (row r at (r / rpp) * pstride +
 // (row_off + r % rpp) * n).  Input points outside [in_lo, in_hi) are taken as

@@ -1185,10 +1185,15 @@ static void launch_rows_crop_t(const RowsArgs &a, dim3 g, int threads, size_t sm
         case 8: CALL(8); break;                     \
         case 10: CALL(10); break;                   \
         case 12: CALL(12); break;                   \
+        case 14: CALL(14); break;                   \
         case 16: CALL(16); break;                   \
+        case 18: CALL(18); break;                   \
         case 20: CALL(20); break;                   \
         case 24: CALL(24); break;                   \
+        case 28: CALL(28); break;                   \
+        case 30: CALL(30); break;                   \
         case 32: CALL(32); break;                   \
+        case 36: CALL(36); break;                   \
         case 40: CALL(40); break;                   \
         default: fail(GB_ERR_INTERNAL, "unsupported FFT length"); \
     }
