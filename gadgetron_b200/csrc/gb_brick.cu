@@ -529,7 +529,9 @@ void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *d
 // 3D bricks are two slices thick (W = 4 meets 2.5 of them: 80 % of the slices
 // computed are hit).
 using Brick2D16 = BrickShape<2, 8, 4, 1, 8, 1, false, 256, 3>;
-using Brick2D16C = BrickShape<2, 8, 4, 1, 8, 1, false, 128, 6>;   // compensated
+// Compensated; 8 CTAs per SM instead of 6: 11.52 -> 11.40 ms per refined solve at
+// 512^2 -> 640^2, 32 coils.
+using Brick2D16C = BrickShape<2, 8, 4, 1, 8, 1, false, 128, 8>;
 using Brick2D16W = BrickShape<4, 4, 8, 1, 8, 1, false, 128, 4>;
 using Brick2D12 = BrickShape<3, 4, 8, 1, 8, 1, false, 128, 5>;
 using Brick2D8 = BrickShape<2, 4, 8, 1, 8, 1, false, 256, 3>;
