@@ -840,7 +840,8 @@ void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, Samp
     // The caller's samples are one plane per coil: from kIlMinCoils coils on
     // they are first laid into sorted coil-interleaved rows (density weights
     // folded in), so that a hit loads its coils as one run instead of one
-    // sector per coil.  Not when that would have to allocate during a capture.
+    // sector per coil.  Not when that would have to allocate during a capture, or
+    // has no room.
     const float2 *src = samples;
     SampleLayout lay = layout;
     if (use_ws && c.brick && layout != LAYOUT_SORTED_IL && nb >= kIlMinCoils && samples != p.samp_ws.get()) {
@@ -849,10 +850,7 @@ void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, Samp
         if (!room) {
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             GB_CUDA(cudaStreamIsCapturing(st, &cs));
-            if (cs == cudaStreamCaptureStatusNone) {
-                p.samp_ws.ensure(need);
-                room = true;
-            }
+            room = cs == cudaStreamCaptureStatusNone && p.samp_ws.try_ensure(need);
         }
         if (room) {
             launch_samples_il(p, samples, dcw, nb, p.samp_ws.get(), st);

@@ -76,15 +76,21 @@ struct DevBuf {
     }
     // Grows to at least `count` elements; returns true if reallocated.
     bool ensure(size_t count) {
-        if (count <= n && ptr) return false;
+        const size_t had = n;
+        if (!try_ensure(count))
+            fail(GB_ERR_OUT_OF_MEMORY, "device allocation of " +
+                 std::to_string((count ? count : 1) * sizeof(T)) + " bytes failed");
+        return n != had;
+    }
+    // Grows to at least `count` elements; false (and empty) without room.
+    bool try_ensure(size_t count) {
+        if (count <= n && ptr) return true;
         release();
         if (count == 0) count = 1;
-        cudaError_t e = cudaMalloc((void **)&ptr, count * sizeof(T));
-        if (e != cudaSuccess) {
+        if (cudaMalloc((void **)&ptr, count * sizeof(T)) != cudaSuccess) {
             ptr = nullptr;
             cudaGetLastError();
-            fail(GB_ERR_OUT_OF_MEMORY, "device allocation of " +
-                 std::to_string(count * sizeof(T)) + " bytes failed");
+            return false;
         }
         n = count;
         return true;

@@ -29,6 +29,7 @@
 // 125 -> 53 us an iteration (footprint arrays indexed by a runtime dimension
 // lived in local memory before); bound by instruction issue (85 %).  The grids and the
 // trajectory-range flag are kept per device between calls.
+#include <algorithm>
 #include <cmath>
 #include <utility>
 
@@ -149,15 +150,12 @@ __global__ void __launch_bounds__(256) k_sdc_degrid_update(SdcArgs a, const floa
     if (lane == 0) w[j] = t == 0.f ? 0.f : w[j] / t;
 }
 
-bool sdc_two_grids(int64_t G) { return G <= ((int64_t)1 << 28); }
-
+// `two`: two grids in turn; one, cleared by itself, otherwise
 template <int D>
-void sdc_iterations(const SdcArgs &a, const float *traj, float *w, float *grid, int64_t G, int iterations,
+void sdc_iterations(const SdcArgs &a, const float *traj, float *w, float *grid, int64_t G, bool two, int iterations,
                     cudaStream_t st) {
     const unsigned int tb = 256;
     const unsigned int wb = (unsigned int)((a.M + (tb / 32) - 1) / (tb / 32));   // one warp per sample
-    // two grids in turn up to 1 GiB each; one, cleared by itself, above
-    const bool two = sdc_two_grids(G);
     float *cur = grid, *next = two ? grid + G : grid;
     for (int it = 0; it < iterations; it++) {
         if (it == 0 || !two) GB_CUDA(cudaMemsetAsync(cur, 0, (size_t)G * sizeof(float), st));
@@ -167,11 +165,141 @@ void sdc_iterations(const SdcArgs &a, const float *traj, float *w, float *grid, 
     }
 }
 
+// ---- 2D, footprints of at most 128 taps: weights evaluated once per call.
+//
+// The weights do not change between iterations, so they are laid into a table
+// of 128 floats per sample (tap t = lane + 32 r of a cap x cap square from the
+// sample's first cell, zero outside the disc) that every iteration reads back
+// from L2: four coalesced loads per lane take the place of the square roots and
+// polynomials that bound the direct passes.  A tap that rounding may put beyond
+// the square lies at |u| = R, where the weight is zero.  49152 samples, width
+// 5.5, 512^2, 10 iterations: 534 -> 352 us a call; bound now by the L2 atomics
+// and gathers of the footprints.  The table is taken up to kSdcTableSamples
+// samples (128 MiB of scratch, what L2 holds); above, for one iteration (nothing
+// to reuse), for other dimensions and for wider kernels, every pass evaluates the
+// weights.
+constexpr int kSdcRounds = 4;
+constexpr int64_t kSdcTableSamples = (int64_t)1 << 18;
+
+struct SdcTaps {
+    int tx[kSdcRounds], ty[kSdcRounds];
+};
+
+__device__ __forceinline__ SdcTaps sdc_lane_taps(int cap, int lane) {
+    SdcTaps q;
+#pragma unroll
+    for (int r = 0; r < kSdcRounds; r++) {
+        const int t = lane + 32 * r;
+        q.ty[r] = t / cap;
+        q.tx[r] = t - q.ty[r] * cap;
+    }
+    return q;
+}
+
+// Position and first cell of sample j along dimension d.
+__device__ __forceinline__ float sdc_pos(const SdcArgs &a, const float *traj, int64_t j, int d, int &lo) {
+    const float s = fmaf(traj[j * 2 + d], (float)a.mos[d], a.half_mos_pad[d]) - a.hp;
+    lo = (int)ceilf(s - a.radius);
+    return s;
+}
+
+__global__ void __launch_bounds__(256) k_sdc_table(SdcArgs a, int cap, const float *__restrict__ traj,
+                                                   float *__restrict__ tab) {
+    const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (j >= a.M) return;
+    const int lane = threadIdx.x & 31;
+    const SdcTaps q = sdc_lane_taps(cap, lane);
+    int lo[2];
+    const float s0 = sdc_pos(a, traj, j, 0, lo[0]), s1 = sdc_pos(a, traj, j, 1, lo[1]);
+    const int n0 = (int)floorf(s0 + a.radius) - lo[0] + 1, n1 = (int)floorf(s1 + a.radius) - lo[1] + 1;
+    const float inv_R = 1.f / a.radius;
+#pragma unroll
+    for (int r = 0; r < kSdcRounds; r++) {
+        float w = 0.f;
+        if (q.tx[r] < n0 && q.ty[r] < n1) {
+            const float u = s0 - (float)(lo[0] + q.tx[r]), v = s1 - (float)(lo[1] + q.ty[r]);
+            float d2 = u * u;
+            d2 += v * v;
+            w = jinc_weight(d2, inv_R);
+        }
+        tab[j * (32 * kSdcRounds) + 32 * r + lane] = w;
+    }
+}
+
+// Calls f(cell, weight) for this lane's taps of sample j with nonzero weight.
+template <class F>
+__device__ __forceinline__ void sdc_table_taps(const SdcArgs &a, const SdcTaps &q, const float *traj,
+                                               const float *tab, int64_t j, int lane, F &&f) {
+    float w[kSdcRounds];
+#pragma unroll
+    for (int r = 0; r < kSdcRounds; r++) w[r] = __ldg(tab + j * (32 * kSdcRounds) + 32 * r + lane);
+    int lo[2];
+    sdc_pos(a, traj, j, 0, lo[0]);
+    sdc_pos(a, traj, j, 1, lo[1]);
+#pragma unroll
+    for (int r = 0; r < kSdcRounds; r++) {
+        if (w[r] != 0.f) {
+            const int cx = wrap_cell(lo[0] + q.tx[r], a.mos[0]), cy = wrap_cell(lo[1] + q.ty[r], a.mos[1]);
+            f((int64_t)cy * a.mos[0] + cx, w[r]);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sdc_table_grid(SdcArgs a, int cap, const float *__restrict__ traj,
+                                                        const float *__restrict__ tab, const float *__restrict__ w,
+                                                        float *__restrict__ grid) {
+    const int lane = threadIdx.x & 31;
+    const SdcTaps q = sdc_lane_taps(cap, lane);
+    for (int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < a.M; j += (int64_t)gridDim.x * 8) {
+        const float v = w[j];
+        sdc_table_taps(a, q, traj, tab, j, lane, [&](int64_t idx, float wt) { atomicAdd(&grid[idx], wt * v); });
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sdc_table_update(SdcArgs a, int cap, const float *__restrict__ traj,
+                                                          const float *__restrict__ tab,
+                                                          const float *__restrict__ grid, float *__restrict__ w,
+                                                          float *__restrict__ clear, int64_t G) {
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t i = i0; i < G; i += (int64_t)gridDim.x * blockDim.x) clear[i] = 0.f;
+    const int lane = threadIdx.x & 31;
+    const SdcTaps q = sdc_lane_taps(cap, lane);
+    for (int64_t j = i0 >> 5; j < a.M; j += (int64_t)gridDim.x * 8) {
+        float t = 0.f;
+        sdc_table_taps(a, q, traj, tab, j, lane, [&](int64_t idx, float wt) { t += wt * grid[idx]; });
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) w[j] = t == 0.f ? 0.f : w[j] / t;
+    }
+}
+
+// Taps per dimension of the table's square; 0 when the table does not apply.
+int sdc_table_cap(const SdcArgs &a, bool two, int iterations) {
+    const int cap = (int)std::floor(2.f * a.radius) + 1;
+    return (a.D == 2 && cap * cap <= 32 * kSdcRounds && a.M <= kSdcTableSamples && two && iterations > 1)
+               ? cap
+               : 0;
+}
+
+void sdc_table_iterations(const SdcArgs &a, int cap, const float *traj, float *w, float *grid, float *tab, int64_t G,
+                          int iterations, cudaStream_t st) {
+    const unsigned int all = (unsigned int)((a.M + 7) / 8);   // one warp per sample
+    const unsigned int blocks = std::min(all, 148u * 16u);    // a few samples per warp
+    k_sdc_table<<<all, 256, 0, st>>>(a, cap, traj, tab); note_launch();
+    float *cur = grid, *next = grid + G;
+    GB_CUDA(cudaMemsetAsync(cur, 0, (size_t)G * sizeof(float), st));
+    for (int it = 0; it < iterations; it++) {
+        k_sdc_table_grid<<<blocks, 256, 0, st>>>(a, cap, traj, tab, w, cur); note_launch();
+        k_sdc_table_update<<<blocks, 256, 0, st>>>(a, cap, traj, tab, cur, w, next, it + 1 < iterations ? G : 0);
+        note_launch();
+        std::swap(cur, next);
+    }
+}
+
 // Scratch kept per device between calls; the mutex is held for a whole call.
 struct SdcScratch {
     std::mutex mu;
     DevBuf<unsigned int> bad;
-    DevBuf<float> grid;
+    DevBuf<float> grid, table;
 };
 
 __global__ void k_fill(float *p, int64_t n, float v) {
@@ -234,10 +362,16 @@ void sdc_estimate_dcw(int D, const uint64_t *N, float os_factor, int iterations,
     } else {
         k_fill<<<sb, tb, 0, st>>>(dcw, M, 1.f); note_launch();
     }
-    sc.grid.ensure((sdc_two_grids(G) ? 2 : 1) * (size_t)G);
-    if (D == 1) sdc_iterations<1>(a, traj, dcw, sc.grid.get(), G, iterations, st);
-    else if (D == 2) sdc_iterations<2>(a, traj, dcw, sc.grid.get(), G, iterations, st);
-    else sdc_iterations<3>(a, traj, dcw, sc.grid.get(), G, iterations, st);
+    // two grids in turn up to 1 GiB each; where they or the table do not fit,
+    // one grid and the direct passes
+    const bool two = G <= ((int64_t)1 << 28) && sc.grid.try_ensure(2 * (size_t)G);
+    if (!two) sc.grid.ensure((size_t)G);
+    const int cap = sdc_table_cap(a, two, iterations);
+    if (cap > 0 && sc.table.try_ensure((size_t)M * 32 * kSdcRounds))
+        sdc_table_iterations(a, cap, traj, dcw, sc.grid.get(), sc.table.get(), G, iterations, st);
+    else if (D == 1) sdc_iterations<1>(a, traj, dcw, sc.grid.get(), G, two, iterations, st);
+    else if (D == 2) sdc_iterations<2>(a, traj, dcw, sc.grid.get(), G, two, iterations, st);
+    else sdc_iterations<3>(a, traj, dcw, sc.grid.get(), G, two, iterations, st);
     GB_CUDA(cudaGetLastError());
     GB_CUDA(cudaStreamSynchronize(st));   // the grids are free for the next call on return
 }

@@ -52,3 +52,15 @@ def test_sdc_repeated_calls_and_call_after_rejection(cuda):
         gb.sdc.estimate_dcw(bad, (32, 32), 2.0, 2)
     w = gb.sdc.estimate_dcw(torch.from_numpy(small).to(cuda), (32, 32), 2.0, 5, 5.5)
     assert O.rel_l2(w.cpu().numpy(), O.estimate_dcw(small, (32, 32), 2.0, 5, 5.5)) <= 1e-5
+
+
+@pytest.mark.parametrize("M,kw,iters", [(1, 5.5, 2), (9, 0.95, 3), (777, 5.65, 2), (777, 5.8, 2), (777, 5.5, 1),
+                                        (18945, 5.5, 2), (1 << 18, 2.0, 2), ((1 << 18) + 1, 2.0, 2)])
+def test_sdc_2d_weight_table_limits(cuda, M, kw, iters):
+    """Both sides of the weight table's limits: the smallest and widest square
+    (2 x 2 and 11 x 11 taps), one wider, one iteration, a warp's second sample,
+    and the largest sample count and one more."""
+    traj = np.random.default_rng(M).uniform(-0.5, 0.5, (M, 2)).astype(np.float32)
+    traj[0] = (-0.5, 0.5)
+    w = gb.sdc.estimate_dcw(torch.from_numpy(traj).to(cuda), (48, 32), 2.0, iters, kw)
+    assert O.rel_l2(w.cpu().numpy(), O.estimate_dcw(traj, (48, 32), 2.0, iters, kw)) <= 1e-5
