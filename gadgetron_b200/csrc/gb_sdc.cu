@@ -31,6 +31,7 @@
 // trajectory-range flag are kept per device between calls.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <utility>
 
 #include "gb_internal.cuh"
@@ -50,15 +51,42 @@ struct SdcArgs {
     int mos[3];
     float half_mos_pad[3];   // (mos + pad) / 2
     float hp;                // pad / 2
-    float radius;
+    float radius, inv_R;
+    float d2_limit;          // squared distances of a disc's cells lie below it
     int64_t M;
 };
 
+// Smallest d2 outside the disc, i.e. with !(sqrtf(d2) / R < kJincNormRadius):
+// the root and the quotient are correctly rounded and monotone, so the
+// reference's rule is a threshold on d2, found by bisection over the floats.
+float jinc_limit(float R) {
+    auto outside = [R](uint32_t bits) {
+        float d2;
+        std::memcpy(&d2, &bits, sizeof(d2));
+        return !(std::sqrt(d2) / R < kJincNormRadius);
+    };
+    uint32_t in = 0u, out = 0x7f800000u;   // 0 and infinity; positive floats order as their bits
+    while (out - in > 1u) {
+        const uint32_t mid = in + (out - in) / 2u;
+        (outside(mid) ? out : in) = mid;
+    }
+    float limit;
+    std::memcpy(&limit, &out, sizeof(limit));
+    return limit;
+}
+
 // Weight of a cell at squared distance d2 from the sample (the any-|u_d| > R
-// rule of the reference cuts nothing that the radius below does not).
-__device__ __forceinline__ float jinc_weight(float d2, float inv_R) {
-    const float r = sqrtf(d2) * inv_R;
-    if (!(r < kJincNormRadius)) return 0.f;
+// rule of the reference cuts nothing that the radius below does not).  The
+// polynomial is 6.6e-4 where the disc ends, so which cells are inside is
+// decided exactly as by sqrtf(d2) / R < kJincNormRadius; with the once more
+// rounded sqrtf(d2) * (1 / R) one tap in 7 million (width 4) changes sides and
+// moves a weight by up to 5e-4.  The polynomial's r is the product corrected by
+// its remainder: half an ulp (and 1e-6 of one) from the quotient.  Direct passes
+// of 300000 samples, width 5.5, 10 iterations: 2.74 ms with a division, 2.65 so.
+__device__ __forceinline__ float jinc_weight(float d2, const SdcArgs &a) {
+    if (!(d2 < a.d2_limit)) return 0.f;
+    const float root = sqrtf(d2), q = root * a.inv_R;
+    const float r = fmaf(fmaf(-q, a.radius, root), a.inv_R, q);
     // the reference's sum c0 + c1 r + ... + c5 r^5 in its order, the powers
     // formed by products (within a few ulp of pow(r, k))
     const float r2 = r * r, r3 = r2 * r, r4 = r2 * r2, r5 = r4 * r;
@@ -86,7 +114,6 @@ __device__ __forceinline__ void for_footprint_lane(const SdcArgs &a, const float
         taps *= n[d];
     }
     if (lane >= taps) return;
-    const float inv_R = 1.f / a.radius;
     // tap coordinates of t, stepped by 32 taps per round without divisions
     int tx = lane % n[0], ty = lane / n[0], tz = 0;
     if (D > 2) {
@@ -101,17 +128,17 @@ __device__ __forceinline__ void for_footprint_lane(const SdcArgs &a, const float
         if (D > 1) {
             const int cy = lo[1 % D] + ty;
             u = s[1 % D] - (float)cy;
-            d2 += u * u;
+            d2 = fmaf(u, u, d2);
             int64_t row = wrap_cell(cy, a.mos[1]);
             if (D > 2) {
                 const int cz = lo[2 % D] + tz;
                 u = s[2 % D] - (float)cz;
-                d2 += u * u;
+                d2 = fmaf(u, u, d2);
                 row += (int64_t)wrap_cell(cz, a.mos[2]) * a.mos[1];
             }
             idx += row * a.mos[0];
         }
-        const float w = jinc_weight(d2, inv_R);
+        const float w = jinc_weight(d2, a);
         if (w != 0.f) f(idx, w);
         tx += 32;
         while (tx >= n[0]) {
@@ -212,15 +239,12 @@ __global__ void __launch_bounds__(256) k_sdc_table(SdcArgs a, int cap, const flo
     int lo[2];
     const float s0 = sdc_pos(a, traj, j, 0, lo[0]), s1 = sdc_pos(a, traj, j, 1, lo[1]);
     const int n0 = (int)floorf(s0 + a.radius) - lo[0] + 1, n1 = (int)floorf(s1 + a.radius) - lo[1] + 1;
-    const float inv_R = 1.f / a.radius;
 #pragma unroll
     for (int r = 0; r < kSdcRounds; r++) {
         float w = 0.f;
         if (q.tx[r] < n0 && q.ty[r] < n1) {
             const float u = s0 - (float)(lo[0] + q.tx[r]), v = s1 - (float)(lo[1] + q.ty[r]);
-            float d2 = u * u;
-            d2 += v * v;
-            w = jinc_weight(d2, inv_R);
+            w = jinc_weight(fmaf(v, v, u * u), a);
         }
         tab[j * (32 * kSdcRounds) + 32 * r + lane] = w;
     }
@@ -327,6 +351,8 @@ void sdc_estimate_dcw(int D, const uint64_t *N, float os_factor, int iterations,
     a.M = M;
     a.radius = kJincNormRadius * kernel_width;
     if (2.f * a.radius < 1.8f) fail(GB_ERR_INVALID_ARGUMENT, "Kernel width must be equal to or larger than 1.8.");
+    a.inv_R = 1.f / a.radius;
+    a.d2_limit = jinc_limit(a.radius);
     const int pad = 2 * (int)std::ceil(a.radius);
     a.hp = (float)(pad / 2);
     int64_t G = 1;
