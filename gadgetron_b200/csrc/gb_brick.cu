@@ -46,10 +46,12 @@ namespace gb {
 
 // CPL coils per lane, LPC lanes over the coils of a group, XL x YL lanes over
 // the columns, YC x ZC cells per lane, at most NT threads (warps * 32) per CTA,
-// MB resident CTAs asked of the register allocation.
-template <int CPL_, int LPC_, int XL_, int YL_, int YC_, int ZC_, bool D3_, int NT_, int MB_>
+// MB resident CTAs asked of the register allocation, at most CTA bricks per CTA
+// (a CTA's slot is held until its slowest brick is done -- samples crowd -- so a
+// tile of more bricks is spread over several CTAs).
+template <int CPL_, int LPC_, int XL_, int YL_, int YC_, int ZC_, bool D3_, int NT_, int MB_, int CTA_ = 4>
 struct BrickShape {
-    static constexpr int CPL = CPL_, LPC = LPC_, XL = XL_, YL = YL_, YC = YC_, ZC = ZC_, NT = NT_, MB = MB_;
+    static constexpr int CPL = CPL_, LPC = LPC_, XL = XL_, YL = YL_, YC = YC_, ZC = ZC_, NT = NT_, MB = MB_, CTA = CTA_;
     static constexpr bool D3 = D3_;
     static constexpr int CG = CPL * LPC, BX = XL, BY = YL * YC, BZ = ZC, YP = YC / 2, V = 2 * CPL;
     static constexpr int NACC = ZC * YP * V;   // float2 accumulators of a lane
@@ -60,14 +62,13 @@ struct BrickShape {
     static constexpr int SLOT = VC + WCH + 1;                               // one more: the density weight
     static constexpr int UH = NACC > 16 ? 1 : 2;                            // hits summed together
     static constexpr int HB = CG >= 12 ? 4 : 8;                             // hits staged together
+    static_assert(32 * CTA <= NT, "a CTA's bricks fit its threads");
     static_assert(LPC * XL * YL == 32 && YC % 2 == 0 && BY % 4 == 0, "a brick fills a warp");
 };
 
 constexpr int kBrickDepth = 3;    // batches of hits in the ring of a warp
 constexpr int kBrickQueue = 64;   // pending hits of a warp
-// Bricks (warps) per CTA: a CTA's slot is held until its slowest brick is done
-// (samples crowd), so a tile of more bricks is spread over several CTAs.
-constexpr int kBrickCtaWarps = 4;
+constexpr int kBrickMax = 16;     // bricks per tile
 constexpr int kBrickFillWarps = 148 * 12;   // warps that fill the GPU
 constexpr int kBrickWideWarps = 148 * 24 * 4;   // narrow-form warps from which the wide form is taken
 
@@ -528,7 +529,8 @@ void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *d
 // serves the small ones.  12 coils have a form of their own (3 per lane, no idle lanes).
 // 3D bricks are two slices thick (W = 4 meets 2.5 of them: 80 % of the slices
 // computed are hit).
-using Brick2D16 = BrickShape<2, 8, 4, 1, 8, 1, false, 256, 3>;
+// (8 bricks per CTA: the short lists of the narrow form leave no imbalance to speak of)
+using Brick2D16 = BrickShape<2, 8, 4, 1, 8, 1, false, 256, 3, 8>;
 // Compensated; 8 CTAs per SM instead of 6: 11.52 -> 11.40 ms per refined solve at
 // 512^2 -> 640^2, 32 coils.
 using Brick2D16C = BrickShape<2, 8, 4, 1, 8, 1, false, 128, 8>;
@@ -547,57 +549,82 @@ using Brick3D4 = BrickShape<2, 2, 8, 2, 4, 2, true, 256, 3>;
 using Brick3D2 = BrickShape<2, 1, 8, 4, 2, 2, true, 256, 3>;
 using Brick3D1 = BrickShape<1, 1, 8, 4, 2, 2, true, 256, 4>;
 
-template <class S>
-static int bricks_of(const KParams &k) {
-    if (k.tile[0] % S::BX || k.tile[1] % S::BY || k.tile[2] % S::BZ) return 0;
-    const int n = (k.tile[0] / S::BX) * (k.tile[1] / S::BY) * (k.tile[2] / S::BZ);
-    // tile extents are powers of two (a tile holds a divisor of 256 cells, 512 or 1024)
-    return (n <= 4 * kBrickCtaWarps && (n & (n - 1)) == 0) ? n : 0;
-}
-
-static int bricks_for(const KParams &k, int cg, bool comp) {
-    if (k.D == 2) {
+// Calls f(shape, compensated) for the form of coil group cg; false for a group
+// that has none.
+template <class F>
+static bool with_brick(int D, int cg, bool comp, bool wide, F &&f) {
+    using P = std::false_type;   // plain sums
+    using C = std::true_type;    // compensated sums
+#define GB_EITHER(S) (comp ? f(S{}, C{}) : f(S{}, P{}))
+    if (D == 2) {
         switch (cg) {
-            case 16: return bricks_of<Brick2D16>(k);
-            case 12: return comp ? 0 : bricks_of<Brick2D12>(k);
-            case 8: return bricks_of<Brick2D8>(k);
-            case 4: return bricks_of<Brick2D4>(k);
-            case 2: return bricks_of<Brick2D2>(k);
-            default: return bricks_of<Brick2D1>(k);
+            case 16:
+                if (comp) f(Brick2D16C{}, C{});
+                else if (wide) f(Brick2D16W{}, P{});
+                else f(Brick2D16{}, P{});
+                return true;
+            case 12:
+                if (!comp) f(Brick2D12{}, P{});
+                return !comp;
+            case 8: GB_EITHER(Brick2D8); return true;
+            case 4: GB_EITHER(Brick2D4); return true;
+            case 2: GB_EITHER(Brick2D2); return true;
+            default: GB_EITHER(Brick2D1); return true;
         }
     }
     switch (cg) {
-        case 32: return comp ? 0 : bricks_of<Brick3D32>(k);
-        case 16: return comp ? bricks_of<Brick3D16C>(k) : bricks_of<Brick3D16>(k);
-        case 8: return comp ? bricks_of<Brick3D8C>(k) : bricks_of<Brick3D8>(k);
-        case 4: return bricks_of<Brick3D4>(k);
-        case 2: return bricks_of<Brick3D2>(k);
-        default: return bricks_of<Brick3D1>(k);
+        case 32:
+            if (!comp) f(Brick3D32{}, P{});
+            return !comp;
+        case 16:
+            if (comp) f(Brick3D16C{}, C{});
+            else f(Brick3D16{}, P{});
+            return true;
+        case 8:
+            if (comp) f(Brick3D8C{}, C{});
+            else f(Brick3D8{}, P{});
+            return true;
+        case 4: GB_EITHER(Brick3D4); return true;
+        case 2: GB_EITHER(Brick3D2); return true;
+        default: GB_EITHER(Brick3D1); return true;
     }
+#undef GB_EITHER
+}
+
+// Cuts the plan's tile into the bricks of the form: bricks per tile, and CTAs a
+// tile's bricks are spread over; false when the form does not divide the tile.
+static bool cut_tile(const KParams &k, int cg, bool comp, bool wide, GridCfg &c) {
+    int n = 0;
+    with_brick(k.D, cg, comp, wide, [&](auto shape, auto) {
+        using S = decltype(shape);
+        if (k.tile[0] % S::BX || k.tile[1] % S::BY || k.tile[2] % S::BZ) return;
+        n = (k.tile[0] / S::BX) * (k.tile[1] / S::BY) * (k.tile[2] / S::BZ);
+        // tile extents are powers of two (a tile holds a divisor of 256 cells, 512 or 1024)
+        if (n > kBrickMax || (n & (n - 1)) != 0) n = 0;
+        c.groups = std::max(1, n / S::CTA);
+    });
+    if (!n) return false;
+    c.brick = true;
+    c.cg = cg;
+    c.wide = wide;
+    c.nbricks = n;
+    return true;
 }
 
 bool brick_config(const NufftPlan &p, int nb, GridCfg &c) {
     const KParams &k = p.kp;
     if (k.D < 2 || p.pair_row_stride <= 0 || p.pair_row_stride != pair_row_floats(k)) return false;
     const bool comp = (p.flags & GB_FLAG_COMPENSATED) != 0;
-    int cg = choose_cg(p.tiling.cg, nb);
+    const int cg = choose_cg(p.tiling.cg, nb);
     // 3D, more than 16 coils: one group of 32 visits a sample's bricks once
     // instead of twice
-    if (k.D == 3 && cg == 16 && nb > 16 && bricks_for(k, 32, comp)) cg = 32;
-    if (k.D == 2 && cg == 16 && nb % 12 == 0 && nb % 16 != 0 && bricks_for(k, 12, comp)) cg = 12;
-    int n = bricks_for(k, cg, comp);
-    if (!n) return false;
-    c.brick = true;
-    c.cg = cg;
-    c.wide = false;
-    if (k.D == 2 && cg == 16 && !comp && bricks_of<Brick2D16W>(k) &&
-        (int64_t)p.n_grd_items * ((nb + cg - 1) / cg) * n >= kBrickWideWarps) {
-        c.wide = true;
-        n = bricks_of<Brick2D16W>(k);
-    }
-    c.nbricks = n;
-    // (the short lists of the narrow 2D form leave no such imbalance: 8 bricks)
-    c.groups = std::max(1, n / (k.D == 2 && cg == 16 && !comp ? 2 * kBrickCtaWarps : kBrickCtaWarps));
+    if (k.D == 3 && cg == 16 && nb > 16 && cut_tile(k, 32, comp, false, c)) return true;
+    if (k.D == 2 && cg == 16 && nb % 12 == 0 && nb % 16 != 0 && cut_tile(k, 12, comp, false, c)) return true;
+    if (!cut_tile(k, cg, comp, false, c)) return false;
+    GridCfg w = c;
+    if (k.D == 2 && cg == 16 && !comp &&
+        (int64_t)p.n_grd_items * ((nb + cg - 1) / cg) * c.nbricks >= kBrickWideWarps && cut_tile(k, cg, comp, true, w))
+        c = w;
     return true;
 }
 
@@ -622,6 +649,7 @@ static void brick_launch(const GridCfg &c, const ConvArgs &args, const float2 *s
     a.lcta = log2i(cta);
     a.lparts = log2i(parts);
     const int warps = cta * parts;
+    if (32 * warps > S::NT) fail(GB_ERR_INTERNAL, "more bricks per CTA than the gridding kernel has warps");
     const dim3 g((unsigned)(a.n_items * c.groups), (unsigned)c.ncg);
     const size_t ring = (size_t)warps * (kBrickDepth * S::HB * S::SLOT * 16 + kBrickQueue * sizeof(uint2));
     const size_t smem = std::max(ring, (size_t)(warps - cta) * S::NACC * 32 * 8);
@@ -644,37 +672,9 @@ void launch_grid_brick(const GridCfg &c, const NufftPlan &p, const ConvArgs &a, 
     const bool comp = (p.flags & GB_FLAG_COMPENSATED) != 0;
     if (a.layout == LAYOUT_SORTED_IL && (c.cg < 2 || a.dcw))
         fail(GB_ERR_INTERNAL, "interleaved samples need a coil pair per lane and carry their density weights");
-#define GB_BRICK(S) (comp ? brick_launch<S, true>(c, a, samples, grid, st) : brick_launch<S, false>(c, a, samples, grid, st))
-    if (p.kp.D == 2) {
-        switch (c.cg) {
-            case 12: brick_launch<Brick2D12, false>(c, a, samples, grid, st); break;
-            case 16:
-                if (c.wide) brick_launch<Brick2D16W, false>(c, a, samples, grid, st);
-                else if (comp) brick_launch<Brick2D16C, true>(c, a, samples, grid, st);
-                else brick_launch<Brick2D16, false>(c, a, samples, grid, st);
-                break;
-            case 8: GB_BRICK(Brick2D8); break;
-            case 4: GB_BRICK(Brick2D4); break;
-            case 2: GB_BRICK(Brick2D2); break;
-            default: GB_BRICK(Brick2D1); break;
-        }
-    } else {
-        switch (c.cg) {
-            case 32: brick_launch<Brick3D32, false>(c, a, samples, grid, st); break;
-            case 16:
-                if (comp) brick_launch<Brick3D16C, true>(c, a, samples, grid, st);
-                else brick_launch<Brick3D16, false>(c, a, samples, grid, st);
-                break;
-            case 8:
-                if (comp) brick_launch<Brick3D8C, true>(c, a, samples, grid, st);
-                else brick_launch<Brick3D8, false>(c, a, samples, grid, st);
-                break;
-            case 4: GB_BRICK(Brick3D4); break;
-            case 2: GB_BRICK(Brick3D2); break;
-            default: GB_BRICK(Brick3D1); break;
-        }
-    }
-#undef GB_BRICK
+    with_brick(p.kp.D, c.cg, comp, c.wide, [&](auto shape, auto comp_c) {
+        brick_launch<decltype(shape), decltype(comp_c)::value>(c, a, samples, grid, st);
+    });
     GB_CUDA(cudaGetLastError());
 }
 

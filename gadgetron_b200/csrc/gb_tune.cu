@@ -68,6 +68,32 @@ bool try_tiling(NufftPlan &p, const TuneResult &r) {
     }
 }
 
+struct Event {
+    cudaEvent_t e = nullptr;
+    Event() { GB_CUDA(cudaEventCreate(&e)); }
+    ~Event() { cudaEventDestroy(e); }
+    Event(const Event &) = delete;
+};
+
+// Milliseconds of one gridding and one degridding of nb batches in the plan's
+// tiling.
+float time_tiling(NufftPlan &p, float2 *samples, float2 *grid, int nb, const std::vector<uint64_t> &offs,
+                  const Event &e0, const Event &e1, cudaStream_t st) {
+    plan_preprocess(p, p.traj_copy.get(), (uint64_t)p.Mtot, (uint32_t)(offs.size() - 1), offs.data(), p.prep_mode, st);
+    launch_grid_prepare(p, nb, st);
+    const SampleLayout lay = normal_op_layout(p, nb);
+    for (int pass = 0; pass < 2; pass++) {   // the first pass untimed (module loading, caches)
+        if (pass) GB_CUDA(cudaEventRecord(e0.e, st));
+        launch_grid(p, samples, grid, nb, lay, nullptr, true, false, st);
+        launch_degrid(p, grid, samples, nb, lay, nullptr, 1, true, false, st);
+    }
+    GB_CUDA(cudaEventRecord(e1.e, st));
+    GB_CUDA(cudaEventSynchronize(e1.e));
+    float ms = 0.f;
+    GB_CUDA(cudaEventElapsedTime(&ms, e0.e, e1.e));
+    return ms;
+}
+
 }  // namespace
 
 void plan_autotune(NufftPlan &p, int nb, cudaStream_t st) {
@@ -77,7 +103,7 @@ void plan_autotune(NufftPlan &p, int nb, cudaStream_t st) {
                       (int)p.F, nb, p.W, (int64_t)(std::log((double)p.Mtot) / std::log(1.05))};
     const int64_t M = p.Mtot;
     const uint32_t F = p.F;
-    std::vector<uint64_t> offs(p.frame_off.begin(), p.frame_off.end());
+    const std::vector<uint64_t> offs(p.frame_off.begin(), p.frame_off.end());
     const TuneResult start{{p.tiling.tile[0], p.tiling.tile[1], p.tiling.tile[2]}, p.tiling.cg};
     TuneResult best = start;
     bool cached = false;
@@ -95,32 +121,21 @@ void plan_autotune(NufftPlan &p, int nb, cudaStream_t st) {
         samples.ensure(ns);
         grid.ensure((size_t)nb * F * p.kp.G);
         GB_CUDA(cudaMemsetAsync(samples.get(), 0, ns * sizeof(float2), st));
-        cudaEvent_t e0, e1;
-        GB_CUDA(cudaEventCreate(&e0));
-        GB_CUDA(cudaEventCreate(&e1));
+        Event e0, e1;
         float best_ms = 1e30f;
         for (const TuneResult &c : candidates(p)) {
-            if (!try_tiling(p, c)) continue;
-            plan_preprocess(p, p.traj_copy.get(), (uint64_t)M, F, offs.data(), p.prep_mode, st);
-            launch_grid_prepare(p, nb, st);
-            const SampleLayout lay = normal_op_layout(p, nb);
-            // one untimed pass (module loading, caches), then one timed pass
-            launch_grid(p, samples.get(), grid.get(), nb, lay, nullptr, true, false, st);
-            launch_degrid(p, grid.get(), samples.get(), nb, lay, nullptr, 1, true, false, st);
-            GB_CUDA(cudaEventRecord(e0, st));
-            launch_grid(p, samples.get(), grid.get(), nb, lay, nullptr, true, false, st);
-            launch_degrid(p, grid.get(), samples.get(), nb, lay, nullptr, 1, true, false, st);
-            GB_CUDA(cudaEventRecord(e1, st));
-            GB_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            GB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            if (ms < best_ms) {
-                best_ms = ms;
-                best = c;
+            try {
+                plan_set_tiling(p, c.tile, c.cg);
+                const float ms = time_tiling(p, samples.get(), grid.get(), nb, offs, e0, e1, st);
+                if (ms < best_ms) {
+                    best_ms = ms;
+                    best = c;
+                }
+            } catch (...) {
+                // a tiling that this plan does not take, or has no room for; an
+                // error that outlasts the launch shows in the preprocess below
             }
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
         std::lock_guard<std::mutex> lock(g_tune_mu);
         g_tune_cache[key] = best;
     }

@@ -85,6 +85,49 @@ def test_wide_form_of_16_coils(cuda):
         assert rel_l2(x[:, f].cpu().numpy(), ref[:, 0]) <= PARITY_TOL, f
 
 
+def _series(coils, frames, seed):
+    """Short radial frames of 64^2 on 128^2 and their samples."""
+    trajs = [S.radial_golden_angle_2d(5 + f % 3, 64, profile_offset=13 * f) for f in range(frames)]
+    offs = np.cumsum([0] + [t.shape[0] for t in trajs]).tolist()
+    return trajs, offs, _samples(coils, offs[-1], seed)
+
+
+@pytest.mark.parametrize("tile", [(32, 16), (16, 32), (64, 8), (32, 32), (16, 8), (8, 16)])
+@pytest.mark.parametrize("coils", [16, 32])
+def test_wide_form_on_every_tile(cuda, tile, coils):
+    """Enough frames for the wide 16-coil form (14208 bricks of the narrow one)
+    on tiles of 128 to 1024 cells: 2 to 16 bricks a tile, one or several CTAs."""
+    N, mos, W = (64, 64), (128, 128), 5.5
+    bricks = tile[0] // 4 * (tile[1] // 8)
+    F = -(-14208 * 16 // (coils * bricks * (128 * 128 // (tile[0] * tile[1]))))
+    trajs, offs, y = _series(coils, F, 3)
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.set_tiling(tile, 16)
+    plan.preprocess(torch.from_numpy(np.concatenate(trajs)).to(cuda), frame_offsets=offs)
+    x = torch.empty((coils, F, 64, 64), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(y).to(cuda), x, None, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+    for f in (0, F // 2, F - 1):
+        orc = O.OraclePlan(N, mos, W)
+        orc.preprocess(trajs[f][None])
+        ref = orc.backwards_nc2c(y[:, offs[f]:offs[f + 1]])
+        assert rel_l2(x[:, f].cpu().numpy(), ref[:, 0]) <= PARITY_TOL, f
+
+
+def test_autotune_of_a_16_coil_series(cuda):
+    """The autotuner times every candidate tile on a launch of the wide form,
+    and leaves a plan that reconstructs."""
+    N, mos, W, C, F = (64, 64), (128, 128), 5.5, 16, 30
+    trajs, offs, y = _series(C, F, 5)
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(np.concatenate(trajs)).to(cuda), frame_offsets=offs)
+    plan.autotune(C)
+    x = torch.empty((C, F, 64, 64), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(y).to(cuda), x, None, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+    orc = O.OraclePlan(N, mos, W)
+    orc.preprocess(trajs[7][None])
+    assert rel_l2(x[:, 7].cpu().numpy(), orc.backwards_nc2c(y[:, offs[7]:offs[8]])[:, 0]) <= PARITY_TOL
+
+
 @pytest.mark.parametrize("coils", [1, 2, 4, 8, 12, 16])
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
 def test_nonfinite_sample_stays_in_its_footprint(cuda, coils, bad):
