@@ -840,11 +840,12 @@ void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, Samp
     // The caller's samples are one plane per coil: from kIlMinCoils coils on
     // they are first laid into sorted coil-interleaved rows (density weights
     // folded in), so that a hit loads its coils as one run instead of one
-    // sector per coil.  Not when that would have to allocate during a capture, or
-    // has no room.
+    // sector per coil.  Only for coil pairs per lane (a coil group of 1 can be
+    // asked for with any coil count), and not when that would have to allocate
+    // during a capture, or has no room.
     const float2 *src = samples;
     SampleLayout lay = layout;
-    if (use_ws && c.brick && layout != LAYOUT_SORTED_IL && nb >= kIlMinCoils && samples != p.samp_ws.get()) {
+    if (use_ws && c.brick && c.cg >= 2 && layout == LAYOUT_ORIGINAL && nb >= kIlMinCoils) {
         const size_t need = (size_t)il_stride_for(nb) * p.Mtot;
         bool room = p.samp_ws.n >= need;
         if (!room) {

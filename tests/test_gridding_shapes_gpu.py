@@ -128,6 +128,31 @@ def test_autotune_of_a_16_coil_series(cuda):
     assert rel_l2(x[:, 7].cpu().numpy(), orc.backwards_nc2c(y[:, offs[7]:offs[8]])[:, 0]) <= PARITY_TOL
 
 
+@pytest.mark.parametrize("group", [1, 2, 4])
+@pytest.mark.parametrize("coils", [4, 5, 17])
+@pytest.mark.parametrize("D", [2, 3])
+def test_coil_groups_smaller_than_the_coil_count(cuda, D, coils, group):
+    """A coil group set by the caller, on both sides of the coil count from
+    which the adjoint lays its samples into rows; every direction."""
+    N, mos, tile = ((64, 32), (128, 64), (16, 16)) if D == 2 else ((32, 32, 32), (64, 64, 64), (8, 8, 8))
+    traj = S.radial_golden_angle_2d(24, 96) if D == 2 else S.kooshball_golden_means_3d(60, 48)
+    plan = gb.NFFT.make_plan(N, mos, 4.0)
+    plan.set_tiling(tile, group)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    orc = O.OraclePlan(N, mos, 4.0)
+    orc.preprocess(traj.reshape(1, -1, D))
+    y, w = _samples(coils, traj.shape[0], coils), S.ramp_dcw(traj)
+    img = S.gaussian_image((coils, 1) + tuple(reversed(N)), 7)
+    it, wt = torch.from_numpy(img).to(cuda), torch.from_numpy(w).to(cuda)
+    x, out = torch.empty_like(it), torch.empty((coils, traj.shape[0]), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(y).to(cuda), x, wt, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+    assert rel_l2(x.cpu().numpy(), orc.backwards_nc2c(y, w[None])) <= PARITY_TOL
+    plan.compute(it, out, None, gb.NFFT_comp_mode.FORWARDS_C2NC)
+    assert rel_l2(out.cpu().numpy(), orc.forward_c2nc(img)) <= PARITY_TOL
+    plan.mult_MH_M(it, x, wt)
+    assert rel_l2(x.cpu().numpy(), orc.mult_MH_M(img, w[None])) <= PARITY_TOL
+
+
 @pytest.mark.parametrize("coils", [1, 2, 4, 8, 12, 16])
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
 def test_nonfinite_sample_stays_in_its_footprint(cuda, coils, bad):
