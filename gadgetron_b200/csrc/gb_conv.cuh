@@ -39,6 +39,18 @@ struct ConvArgs {
     int lcta, lparts;         //   per CTA, warps per brick
 };
 
+// Taps of a sample at padded coordinate s along one dimension: first cell
+// (unpadded) and count.  The same float expressions as the weight table's, which
+// starts at that cell: from the unpadded coordinate s - pad/2, whose float grid is
+// finer, the first cell can come out one further (W = 5.3, s just above a power of
+// two), and every weight would sit one cell off.  The cell that rounding may add
+// at an end lies beyond W/2 and has weight zero.
+__device__ __forceinline__ int first_tap(const KParams &k, float s, int &n) {
+    const int lo = (int)ceilf(s - k.radius);
+    n = (int)floorf(s + k.radius) - lo + 1;
+    return lo - k.hw;
+}
+
 __device__ __forceinline__ float sign_of(int g) { return (g & 1) ? -1.f : 1.f; }
 
 // Which gridding kernel runs for a plan and batch count, with its coil group

@@ -141,9 +141,9 @@ __device__ __forceinline__ void unpack_taps(const ConvArgs &a, const TapRaw &r, 
     for (int t = 0; t < NT; t++) w[2][t] = (t == 0) ? 1.f : 0.f;
 #pragma unroll
     for (int d = 0; d < D; d++) {
-        const float sp = r.sp[d] - (float)k.hw;
-        const int lo = (int)ceilf(sp - k.radius);
-        n[d] = valid ? min((int)floorf(sp + k.radius) - lo + 1, NT) : 0;
+        int taps;
+        const int lo = first_tap(k, r.sp[d], taps);
+        n[d] = valid ? min(taps, NT) : 0;
         const int od = d == 0 ? org0 : (d == 1 ? org1 : org2);
         int x = lo - od + k.hw;   // region-local start, |x| < 2 mos
         x = x < 0 ? x + k.mos[d] : (x >= k.mos[d] ? x - k.mos[d] : x);
@@ -328,11 +328,11 @@ k_traj_grad(ConvArgs a, const float2 *__restrict__ grid, const float2 *__restric
                 const int s = e / (D * kWMax), d = (e / kWMax) % D, t = e % kWMax;
                 float dw = 0.f;
                 if (base + s < it.end) {
-                    const float sp = a.pos[(int64_t)d * a.Mtot + base + s] - (float)k.hw;
-                    const int lo = (int)ceilf(sp - k.radius);
-                    const int n = min((int)floorf(sp + k.radius) - lo + 1, NT);
-                    if (t < n) {
-                        const float diff = sp - (float)(lo + t);
+                    const float sp = a.pos[(int64_t)d * a.Mtot + base + s];
+                    int n;
+                    const int lo = first_tap(k, sp, n);
+                    if (t < min(n, NT)) {
+                        const float diff = sp - (float)(lo + k.hw + t);
                         dw = kb_deriv_1d(fabsf(diff), k.mos_f[d], k.one_over_W, k.beta[d], k.radius);
                         if (diff < 0.f) dw = -dw;
                         if (a.sign_fold && ((lo + t) & 1)) dw = -dw;

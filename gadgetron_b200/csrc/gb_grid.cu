@@ -11,9 +11,9 @@
 // [ceil(s - W/2), floor(s + W/2)] per dimension, each tap's weight is the
 // product over dimensions of the 1D Kaiser-Bessel value of |s - cell|
 // (zero beyond W/2, non-finite weights dropped), and the periodic wrap maps a
-// tap to (cell mod mos).  For NC2C s is the padded-grid coordinate and the
-// cell is folded by -pad/2; for C2NC s - pad/2 is used directly
-// (ConvolverC2NC.cuh:239-241).
+// tap to (cell mod mos).  s is the padded-grid coordinate and the cell is folded
+// by -pad/2; the reference's C2NC starts from s - pad/2 (ConvolverC2NC.cuh:239-241),
+// which gives the same taps of nonzero weight.
 //
 // The 2D and 3D kernels for the usual tiles are in gb_brick.cu (gridding) and
 // gb_degrid.cu (degridding, trajectory gradient); the kernels here serve 1D
@@ -542,14 +542,14 @@ k_degrid_c2nc(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__ 
             const int i = base + s;
             float w = 0.f, dw = 0.f;
             if (i < it.end && d < k.D) {
-                const float sp = a.pos[(int64_t)d * a.Mtot + i] - (float)k.hw;
-                const int lo = (int)ceilf(sp - k.radius);
-                const int n = min((int)floorf(sp + k.radius) - lo + 1, kWMax);
+                const float sp = a.pos[(int64_t)d * a.Mtot + i];
+                int n;
+                const int lo = first_tap(k, sp, n);
+                n = min(n, kWMax);
                 if (t < n) {
                     const int g = lo + t;
-                    const float diff = sp - (float)g;
+                    const float diff = sp - (float)(g + k.hw);   // exact
                     // tap t of the sample's table row is the weight of |diff|
-                    // (both differences are exact in float)
                     w = GRAD ? kb_weight_1d(fabsf(diff), k.mos_f[d], k.one_over_W, k.beta[d], k.radius)
                              : a.wtab[((int64_t)i * k.D + d) * kWMax + t];
                     if (GRAD) {

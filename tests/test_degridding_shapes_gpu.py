@@ -73,3 +73,44 @@ def test_trajectory_gradient_adds_over_coils(cuda, D, coils):
     one = sum(plan.traj_grad(img[c:c + 1].contiguous(), w[c:c + 1].contiguous(), dcw).double() for c in range(coils))
     # 32-bit sums of W^D taps and `coils` coils in another order
     assert rel_l2(total.cpu().numpy(), one.cpu().numpy()) <= 2e-6
+
+
+def _first_tap_trajectory(D, W, mos):
+    """Samples whose first cell comes out differently from the padded and from
+    the unpadded float coordinate along some dimension, random along the others."""
+    r, hw = np.float32(W) * np.float32(0.5), int(np.ceil(W / 2))
+    bias = float((mos + 2 * hw) >> 1)
+    odd = []
+    for p in (16.0, 32.0, 64.0, 128.0):   # every float of the padded coordinate just above a power of two
+        c = np.arange(p, p + hw, 2.0 ** -23 * p).astype(np.float32)
+        c = c[np.ceil(c - r) != np.ceil((c - np.float32(hw)) - r) + hw]
+        k = ((c.astype(np.float64) - bias) / mos).astype(np.float32)
+        odd += k[((k.astype(np.float64) * mos + bias).astype(np.float32) == c) & (np.abs(k) < 0.5)].tolist()
+    assert odd
+    rng = np.random.default_rng(int(10 * W))
+    traj = rng.uniform(-0.5, 0.5, (64 * D, D)).astype(np.float32)
+    for d in range(D):
+        traj[64 * d:64 * (d + 1), d] = rng.choice(odd, 64)
+    return traj
+
+
+@pytest.mark.parametrize("D,W,flags", [(1, 5.3, 0), (2, 5.3, 0), (2, 5.3, 1), (2, 3.7, 0), (2, 2.7, 0), (3, 5.3, 0),
+                                       (3, 4.6, 1)])
+@pytest.mark.parametrize("coils", [1, 2, 16])
+def test_first_tap_where_float_grids_differ(cuda, D, W, flags, coils):
+    """Just above a power of two the padded coordinate's floats are coarser than
+    the unpadded one's; the taps have to start where the weight table does."""
+    N, mos = ((64,) * D, (128,) * D) if D < 3 else ((32,) * D, (64,) * D)
+    traj = _first_tap_trajectory(D, W, mos[0])
+    plan = gb.NFFT.make_plan(N, mos, W, flags=gb.FLAG_COMPENSATED if flags else 0)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    orc = O.OraclePlan(N, mos, W)
+    orc.preprocess(traj.reshape(1, -1, D))
+    rng = np.random.default_rng(1)
+    g = (rng.standard_normal((coils, 1) + mos) + 1j * rng.standard_normal((coils, 1) + mos)).astype(np.complex64)
+    w = _samples(coils, traj.shape[0], 2)
+    out = torch.empty((coils, traj.shape[0]), dtype=torch.complex64, device=cuda)
+    plan.convolve(torch.from_numpy(g).to(cuda), out, gb.NFFT_conv_mode.C2NC)
+    assert rel_l2(out.cpu().numpy(), orc.convolve_c2nc(g)) <= PARITY_TOL
+    grad = plan.traj_grad_from_grid(torch.from_numpy(g).to(cuda), torch.from_numpy(w).to(cuda))
+    assert rel_l2(grad.cpu().numpy(), orc.traj_grad_from_grid(g, w)) <= PARITY_TOL
