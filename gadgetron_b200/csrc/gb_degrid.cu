@@ -12,8 +12,10 @@
 // into registers one pass ahead and runs a fully unrolled NT x NT (x NT) tap
 // nest: one shared load and the multiply-adds per tap.  NT is the largest tap
 // count a footprint can have, floor(W) + 1; a footprint has NT or NT - 1 taps
-// per dimension, and the last tap of the shorter one re-reads the tap before
-// it with weight zero, so nothing outside the footprint is ever read.
+// per dimension, and the last one is skipped where it has NT - 1: nothing outside
+// the footprint is ever read, and no cell is read with a weight of zero (which
+// would make a NaN of an infinite one).  Against re-reading the tap before it with
+// weight zero: 278 -> 262 us (1.13 M samples in 23 frames, 5 coils, 512^2, W 5.5).
 //
 // Before, 1 and 2 coils and compensated sums went through k_degrid_c2nc, which
 // evaluates and stages the weights per warp and predicates every tap: 28.4 ->
@@ -198,8 +200,7 @@ k_degrid_table(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__
 #pragma unroll
         for (int c = 0; c < CPL; c++) acc[c] = cmp[c] = make_float2(0.f, 0.f);
         const float2 *base_s = tile_s + (((size_t)rs[2] * R1 + rs[1]) * R0 + rs[0]) * CS + ll * CPL;
-        const int last_x = (n[0] < NT ? NT - 2 : NT - 1) * CS;      // tap NT - 1 along x and y
-        const int last_y = (n[1] < NT ? NT - 2 : NT - 1) * R0 * CS;
+        const bool full_x = n[0] >= NT, full_y = n[1] >= NT;   // tap NT - 1 along x and y
         auto tap = [&](float2 wv, float2 v, int c) {
             if (COMP) {
                 const float2 t = __ffma2_rn(wv, v, neg2(cmp[c]));
@@ -220,13 +221,15 @@ k_degrid_table(ConvArgs a, const float2 *__restrict__ grid, float2 *__restrict__
                 if (tz < n[2]) {
 #pragma unroll
                     for (int ty = 0; ty < NTT; ty++) {
+                        if (ty == NT - 1 && !full_y) continue;
                         const float wyz = D3 ? w[1][ty] * w[2][tz] : w[1][ty];
-                        const float2 *row = base_s + (size_t)tz * R1 * R0 * CS + (ty == NT - 1 ? last_y : ty * R0 * CS);
+                        const float2 *row = base_s + (size_t)tz * R1 * R0 * CS + ty * R0 * CS;
 #pragma unroll
                         for (int t = 0; t < NTT; t++) {
+                            if (t == NT - 1 && !full_x) continue;
                             const float wv = w[0][t] * wyz;
                             const float2 wv2 = make_float2(wv, wv);
-                            const float2 *cell = row + (t == NT - 1 ? last_x : t * CS);
+                            const float2 *cell = row + t * CS;
                             if (CPL == 2) {
                                 const float4 q = *reinterpret_cast<const float4 *>(cell);
                                 tap(wv2, make_float2(q.x, q.y), 0);
@@ -349,8 +352,7 @@ k_traj_grad(ConvArgs a, const float2 *__restrict__ grid, const float2 *__restric
 #pragma unroll
             for (int t = 0; t < NT; t++) dx[t] = dws[t];
             const float2 *base_s = tile_s + (((size_t)rs[2] * R1 + rs[1]) * R0 + rs[0]) * CS + ll * CPL;
-            const int last_x = (n[0] < NT ? NT - 2 : NT - 1) * CS;
-            const int last_y = (n[1] < NT ? NT - 2 : NT - 1) * R0 * CS;
+            const bool full_x = n[0] >= NT, full_y = n[1] >= NT;
             float2 r[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
             for (int tz = 0; tz < (D3 ? NT : 1); tz++) {
@@ -359,11 +361,13 @@ k_traj_grad(ConvArgs a, const float2 *__restrict__ grid, const float2 *__restric
                 const float2 *slice = base_s + (size_t)tz * R1 * R0 * CS;
 #pragma unroll
                 for (int ty = 0; ty < NT; ty++) {
-                    const float2 *row = slice + (ty == NT - 1 ? last_y : ty * R0 * CS);
+                    if (ty == NT - 1 && !full_y) continue;
+                    const float2 *row = slice + ty * R0 * CS;
                     float2 A = make_float2(0.f, 0.f), B = make_float2(0.f, 0.f);   // sums with the weights, the derivatives
 #pragma unroll
                     for (int t = 0; t < NT; t++) {
-                        const float2 *cell = row + (t == NT - 1 ? last_x : t * CS);
+                        if (t == NT - 1 && !full_x) continue;
+                        const float2 *cell = row + t * CS;
                         float2 s;
                         if (CPL == 2) {
                             const float4 q = *reinterpret_cast<const float4 *>(cell);

@@ -114,3 +114,37 @@ def test_first_tap_where_float_grids_differ(cuda, D, W, flags, coils):
     assert rel_l2(out.cpu().numpy(), orc.convolve_c2nc(g)) <= PARITY_TOL
     grad = plan.traj_grad_from_grid(torch.from_numpy(g).to(cuda), torch.from_numpy(w).to(cuda))
     assert rel_l2(grad.cpu().numpy(), orc.traj_grad_from_grid(g, w)) <= PARITY_TOL
+
+
+def _kinds(a):
+    """-1, 1: that infinity; 2: NaN; 0: finite."""
+    return np.where(np.isnan(a), 2, np.where(np.isinf(a), np.sign(a), 0)).astype(int)
+
+
+@pytest.mark.parametrize("coils", [1, 2, 4, 8, 12, 16])
+@pytest.mark.parametrize("D,W", [(2, 5.5), (2, 4.0), (3, 4.0)])
+def test_infinite_cell_gives_infinite_samples(cuda, D, W, coils):
+    """Footprints have floor(W) or floor(W) + 1 taps a dimension; in the shorter
+    ones no cell may be read with a weight of zero (0 * inf)."""
+    N, mos = (32,) * D, (64,) * D
+    rng = np.random.default_rng(8)
+    traj = rng.uniform(-0.08, 0.08, (600, D)).astype(np.float32)
+    g = (rng.standard_normal((coils, 1) + mos) + 1j * rng.standard_normal((coils, 1) + mos)).astype(np.complex64)
+    g.real[(0, 0) + (30,) * D] = -np.inf
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    out = torch.empty((coils, 600), dtype=torch.complex64, device=cuda)
+    plan.convolve(torch.from_numpy(g).to(cuda), out, gb.NFFT_conv_mode.C2NC)
+    y = out.cpu().numpy()
+    over = np.array([footprint_cells(k, mos, W)[(30,) * D] for k in traj])
+    assert over.sum() >= 20
+    assert np.array_equal(_kinds(y.real[0]), -1 * over)
+    assert np.all(np.isfinite(y.imag)) and np.all(np.isfinite(y[1:]))
+    # the gradient: infinite with the sign of the weights' derivative
+    orc = O.OraclePlan(N, mos, W)
+    orc.preprocess(traj.reshape(1, -1, D))
+    w = np.ones((coils, 600), np.complex64)
+    grad = plan.traj_grad_from_grid(torch.from_numpy(g).to(cuda), torch.from_numpy(w).to(cuda)).cpu().numpy()
+    big = np.where(np.isinf(g.real), np.float32(-1e30), g.real) + 1j * g.imag
+    sign = np.sign(orc.traj_grad_from_grid(big, w))
+    assert np.array_equal(_kinds(grad), np.where(over[:, None], sign, 0))
