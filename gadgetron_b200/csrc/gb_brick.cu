@@ -23,16 +23,19 @@
 // What bounds it, and what was tried: loading a hit's operands straight from
 // L2 one hit ahead left every warp waiting on that latency (118 us for the
 // launch below against 36 us); one staged hit per copy spent 115 instructions
-// a hit on staging, batches of 4 to 8 spend about 15.  Now 16 coils in 2D run
-// at 52 % of the issue slots with the shared-memory pipe at 75 % (value and
-// weight loads, scattered 32-byte stores); 3D is issue- and latency-bound at
-// 16 warps per SM (64 accumulators a lane).  Launch times before (a CTA per
-// tile staging chunks through registers or a producer warp) and after:
+// a hit on staging, batches of 4 to 8 spend about 15.  Now 16 coils in 2D (wide
+// form, 1.13 M samples on 384^2) issue on 55 % of the cycles with the shared-memory
+// pipe at 41 %, 85 instructions a hit, and wait on their few warps' chains; 3D is
+// issue- and latency-bound at 16 warps per SM (64 accumulators a lane).  Launch
+// times before (a CTA per tile staging chunks through registers or a producer
+// warp) and after:
 //   32768 radial samples, 1 coil, 256^2 grid           63.6 -> 17 us
 //   98304 spiral samples, 32 coils, compensated, 640^2  411 -> 140 us
 //   5.12 M kooshball samples, 32 coils, 192^3          13.2 -> 7.5 ms
-//   1.29 M samples in 64 frames, 12 coils, 384^2        630 -> 490 us
+//   1.13 M samples in 23 frames, 12 coils, 512^2        485 -> 364 us
+//   the same, 16 coils / 18 coils                       499 -> 448 / 935 -> 839 us
 //   49152 radial samples, 16 coils, 512^2                37 -> 35 us
+//   46000 samples, 16 coils, 96^2                       203 -> 43 us
 //
 // A zero weight times an infinity would put a NaN into cells the footprint
 // does not touch, so a brick whose sums came out non-finite is summed again
@@ -70,7 +73,8 @@ constexpr int kBrickDepth = 3;    // batches of hits in the ring of a warp
 constexpr int kBrickQueue = 64;   // pending hits of a warp
 constexpr int kBrickMax = 16;     // bricks per tile
 constexpr int kBrickFillWarps = 148 * 12;   // warps that fill the GPU
-constexpr int kBrickWideWarps = 148 * 24 * 4;   // narrow-form warps from which the wide form is taken
+constexpr int kBrickWideWarps = 148 * 24 * 4;   // narrow-form warps from which the wide forms are taken
+constexpr int kBrickWideList = 512;     // average list up to which they are
 
 // Asynchronous copy of BYTES to shared memory; zeros instead when !full.
 template <int BYTES>
@@ -242,12 +246,21 @@ k_grid_brick(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict_
                 for (int c = 0; c < V; c++) v[c] = dw * v[c];
             }
             const float wx = wf[(x0 & 3) * (S::BX < 4) + lx];
+            // Row pairs the footprint misses are skipped where they are the
+            // same for every lane (a lane's column is the whole brick): 2.1 of 4
+            // are met at W = 5.5.
+            constexpr bool SKIP = !D3 && !COMP && S::YL == 1;
             float2 wxy[YP];
+            float pair_w[SKIP ? YP : 1];
             const float2 wx2 = make_float2(wx, wx);
             if (YC % 4 == 0) {
 #pragma unroll
                 for (int q = 0; q < YC / 4; q++) {
                     const float4 w = reinterpret_cast<const float4 *>(slot + VC + XC)[ly * (YC / 4) + q];
+                    if (SKIP) {   // weights are not negative
+                        pair_w[(2 * q) % (SKIP ? YP : 1)] = fmaxf(w.x, w.y);
+                        pair_w[(2 * q + 1) % (SKIP ? YP : 1)] = fmaxf(w.z, w.w);
+                    }
                     wxy[2 * q] = __fmul2_rn(make_float2(w.x, w.y), wx2);
                     wxy[(2 * q + 1) % YP] = __fmul2_rn(make_float2(w.z, w.w), wx2);
                 }
@@ -277,6 +290,7 @@ k_grid_brick(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict_
                 if (ZC > 2 && wz == 0.f) continue;   // a slice the footprint misses (the same for every lane)
 #pragma unroll
                 for (int y = 0; y < YP; y++) {
+                    if (SKIP && pair_w[y % (SKIP ? YP : 1)] == 0.f) continue;
                     const float2 w = D3 ? __fmul2_rn(wxy[y], make_float2(wz, wz)) : wxy[y];
 #pragma unroll
                     for (int c = 0; c < V; c++) {
@@ -523,19 +537,30 @@ void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *d
 // The lanes left over by the coils of a group run along x (then y), so that a
 // group of any size fills the warp.  A brick of 8 x 8 cells is met by 2.4
 // times as many (sample, brick) pairs as there are samples at W = 5.5, one of
-// 4 x 8 by 3.3 times: the wide form of 16 coils (4 coils per lane, 4 warps a
-// tile) runs fewer instructions and serves launches with many waves of tiles,
-// the narrow one (2 coils per lane, 8 warps a tile) has shorter chains and
-// serves the small ones.  12 coils have a form of their own (3 per lane, no idle lanes).
+// 4 x 8 by 3.3 times.  16 coils in 2D have two forms: the wide one (4 coils per
+// lane, 4 bricks to a tile of 16 x 16) runs fewer instructions and serves launches
+// of many tiles with short lists; the narrow one (2 coils per lane, 8 bricks) has
+// shorter chains and serves small launches and long lists.  12 coils have a
+// wide form of their own (3 per lane, no idle lanes).
+// Gridding in us, 96 x 512 radial samples a frame on 512^2, wide / narrow:
+//   1 frame, 16 coils 39.4 / 35.1; 2 frames 49.9 / 53.9; 4 frames 85.5 / 98.9; 23: 457 / 535
+//   1 frame, 12 coils 37.1 / 34.1; 2 frames 46.5 / 50.0; 4 frames 70.2 / 90.7; 23: 370 / 489
+// so the line lies between 1 and 2 frames of 1024 tiles.  On 96^2 with 46000
+// samples a frame (2000 to a tile) the narrow form is the faster one at 23 frames:
+// 264 against 306 us (16 coils), 484 against 552 (18).
+// A CTA of one brick for the wide forms: its slot is free when its brick is done
+// (4 bricks per CTA: 470 us for the 23 frames above with 16 coils, 378 with 12).  The narrow form
+// takes 8 bricks per CTA where lists are short (they share the list's reads: 35.1
+// against 37.9 us for 1 frame) and 2 where they are long (96^2, 1 frame: 59 against 166 us) or
+// where that lets several warps share a brick's list (10400 samples on 192 x 128: 24 against 32 us).
 // 3D bricks are two slices thick (W = 4 meets 2.5 of them: 80 % of the slices
 // computed are hit).
-// (8 bricks per CTA: the short lists of the narrow form leave no imbalance to speak of)
 using Brick2D16 = BrickShape<2, 8, 4, 1, 8, 1, false, 256, 3, 8>;
 // Compensated; 8 CTAs per SM instead of 6: 11.52 -> 11.40 ms per refined solve at
 // 512^2 -> 640^2, 32 coils.
 using Brick2D16C = BrickShape<2, 8, 4, 1, 8, 1, false, 128, 8>;
-using Brick2D16W = BrickShape<4, 4, 8, 1, 8, 1, false, 128, 4>;
-using Brick2D12 = BrickShape<3, 4, 8, 1, 8, 1, false, 128, 5>;
+using Brick2D16W = BrickShape<4, 4, 8, 1, 8, 1, false, 128, 4, 1>;
+using Brick2D12 = BrickShape<3, 4, 8, 1, 8, 1, false, 128, 5, 1>;
 using Brick2D8 = BrickShape<2, 4, 8, 1, 8, 1, false, 256, 3>;
 using Brick2D4 = BrickShape<2, 2, 8, 2, 4, 1, false, 512, 2>;
 using Brick2D2 = BrickShape<2, 1, 8, 4, 2, 1, false, 512, 2>;
@@ -619,13 +644,20 @@ bool brick_config(const NufftPlan &p, int nb, GridCfg &c) {
     // 3D, more than 16 coils: one group of 32 visits a sample's bricks once
     // instead of twice
     if (k.D == 3 && cg == 16 && nb > 16 && cut_tile(k, 32, comp, false, c)) return true;
-    if (k.D == 2 && cg == 16 && nb % 12 == 0 && nb % 16 != 0 && cut_tile(k, 12, comp, false, c)) return true;
-    if (!cut_tile(k, cg, comp, false, c)) return false;
-    GridCfg w = c;
-    if (k.D == 2 && cg == 16 && !comp &&
-        (int64_t)p.n_grd_items * ((nb + cg - 1) / cg) * c.nbricks >= kBrickWideWarps && cut_tile(k, cg, comp, true, w))
-        c = w;
-    return true;
+    if (k.D == 2 && cg == 16 && !comp) {
+        const int64_t avg = p.total_pairs / std::max<int64_t>(1, (int64_t)p.F * k.ntiles_total);
+        const bool twelve = nb % 12 == 0 && nb % 16 != 0;
+        if (!cut_tile(k, cg, comp, false, c)) return false;
+        const int64_t warps = (int64_t)p.n_grd_items * ((nb + cg - 1) / cg) * c.nbricks;
+        if (warps >= kBrickWideWarps && avg <= kBrickWideList) {
+            GridCfg w = c;
+            if ((twelve && cut_tile(k, 12, comp, false, w)) || cut_tile(k, cg, comp, true, w)) c = w;
+        } else if (avg > kBrickWideList || warps < kBrickFillWarps) {
+            c.groups = std::max(1, c.nbricks / 2);
+        }
+        return true;
+    }
+    return cut_tile(k, cg, comp, false, c);
 }
 
 template <class S, bool COMP>

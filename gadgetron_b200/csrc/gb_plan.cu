@@ -634,14 +634,24 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     // Gridding items: tiles of at most split_len pairs as they are, longer ones
     // in chunks.  The samples of a dense tile (a radial centre) crowd into one
     // or two of its bricks, so a chunk's time is the chain of the warp that owns
-    // the crowded brick: chunks are kept at the average tile's length (at least
-    // 96), far below the split threshold.  Chunks of that length need more
-    // partial tiles; the entry point with a fixed scratch takes chunks of up
-    // to split_len pairs when those do not fit (the coarse list).
+    // the crowded brick: chunks are kept at the average tile's length, far below the
+    // split threshold, within bounds.  At least 96 pairs, 128 where the launch has
+    // work enough to hide the chains: shorter ones pay more for their partial tiles
+    // (38675 spiral samples a frame, 16 coils, 512 x 384, at least 64 / 96 / 128 / 192: 2 frames
+    // 66 / 64 / 58 / 57 us, 4 frames 89 / 85 / 81 / 76; one radial frame of 49152 on 512^2:
+    // 43 / 40 / 40 / 46; a frame of 12288, 8 coils, 384^2, preprocess and solve: 128 costs 2 %).
+    // At most 512 or a 32nd of an SM's share, whichever is more: longer ones leave
+    // SMs idle where there are few tiles (131072 samples a frame, 256^2, 18 coils, at
+    // most 256 / 512 / 1024: 1 frame 124 / 123 / 137 us, 2 frames 190 / 183 / 203, 23 frames 1736 /
+    // 1687 / 1673; 5.12 M samples in 3D, 960 to a tile, 32 coils, 512 / 960: 16.81 / 16.50 ms for
+    // both directions).
+    // Chunks of that length need more partial tiles; the entry point with a fixed scratch
+    // takes chunks of up to split_len pairs when those do not fit (the coarse list).
     const int64_t total = goff[nkeys];
     const int64_t avg = total / std::max<uint32_t>(1, nkeys);
     const int split_len = (int)std::max<int64_t>(256, 2 * avg);
-    const int most[2] = {(int)std::max<int64_t>(96, avg), split_len};   // chunk lengths: fine, coarse
+    const int most[2] = {(int)std::min<int64_t>(std::max<int64_t>(total < 100000 ? 96 : 128, avg),
+                                                 std::max<int64_t>(512, total / (148 * 32))), split_len};   // chunk lengths: fine, coarse
     // equal lengths share a run up to 64K pairs; the few lists above keep key order in the last one
     const uint32_t cap = (uint32_t)std::min(split_len, 1 << 16);
     std::vector<uint32_t> light_at((size_t)cap + 1, 0u);

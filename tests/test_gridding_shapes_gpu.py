@@ -113,6 +113,38 @@ def test_wide_form_on_every_tile(cuda, tile, coils):
         assert rel_l2(x[:, f].cpu().numpy(), ref[:, 0]) <= PARITY_TOL, f
 
 
+@pytest.mark.parametrize("coils", [9, 12, 24])
+def test_wide_forms_of_other_coil_counts(cuda, coils):
+    """The wide form with idle coils, and the 12-coil form, which takes over at
+    the same launch size; a frame by itself takes the narrow form."""
+    N, mos, W = (64, 64), (128, 128), 5.5
+    F = -(-14208 // (64 * 8 * -(-coils // 16)))
+    trajs, offs, y = _series(coils, F, 4)
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(np.concatenate(trajs)).to(cuda), frame_offsets=offs)
+    x = torch.empty((coils, F, 64, 64), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(y).to(cuda), x, None, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+    for f in (0, F - 1):
+        one = gb.NFFT.make_plan(N, mos, W)
+        one.preprocess(torch.from_numpy(trajs[f]).to(cuda))
+        xo = torch.empty((coils, 1, 64, 64), dtype=torch.complex64, device=cuda)
+        yf = np.ascontiguousarray(y[:, offs[f]:offs[f + 1]])
+        one.compute(torch.from_numpy(yf).to(cuda), xo, None, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+        orc = O.OraclePlan(N, mos, W)
+        orc.preprocess(trajs[f][None])
+        ref = orc.backwards_nc2c(yf)[:, 0]
+        assert rel_l2(x[:, f].cpu().numpy(), ref) <= PARITY_TOL
+        assert rel_l2(xo[:, 0].cpu().numpy(), ref) <= PARITY_TOL
+
+
+@pytest.mark.parametrize("coils", [8, 12, 16, 18])
+@pytest.mark.parametrize("W", [4.0, 5.5])
+def test_long_lists(cuda, coils, W):
+    """Thousands of samples to a tile: lists cut into chunks of 512, two bricks
+    per CTA with several warps to a brick."""
+    _adjoint_and_normal((32, 32), (64, 64), W, S.radial_golden_angle_2d(150, 200), coils, 0, cuda)
+
+
 def test_autotune_of_a_16_coil_series(cuda):
     """The autotuner times every candidate tile on a launch of the wide form,
     and leaves a plan that reconstructs."""
