@@ -827,7 +827,11 @@ void launch_grid_prepare(NufftPlan &p, int nb, cudaStream_t st) {
     }
 }
 
-constexpr int kIlMinCoils = 5;
+// Coils from which the adjoint lays the caller's samples into rows (2D, 3D).
+// Adjoint in us, gathering / with rows: 49152 samples on 512^2, 5 coils 43.5 / 46.5, 8
+// coils 48.4 / 50.2, 12 coils 62.0 / 59.8, 16 coils 69.2 / 65.0; 873 samples, 8 coils 22.8 /
+// 24.8; 2.56 M samples on 192^3, 5 coils 1773 / 1686, 8 coils 1969 / 1866.
+constexpr int kIlMinCoils[2] = {9, 5};
 
 void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, SampleLayout layout,
                  const float *dcw, bool sign_fold, bool accumulate, cudaStream_t st, const KLayout *kl, bool use_ws) {
@@ -845,7 +849,7 @@ void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, Samp
     // during a capture, or has no room.
     const float2 *src = samples;
     SampleLayout lay = layout;
-    if (use_ws && c.brick && c.cg >= 2 && layout == LAYOUT_ORIGINAL && nb >= kIlMinCoils) {
+    if (use_ws && c.brick && c.cg >= 2 && layout == LAYOUT_ORIGINAL && nb >= kIlMinCoils[p.D == 3]) {
         const size_t need = (size_t)il_stride_for(nb) * p.Mtot;
         bool room = p.samp_ws.n >= need;
         if (!room) {
