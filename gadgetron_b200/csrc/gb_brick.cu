@@ -74,6 +74,7 @@ constexpr int kBrickQueue = 64;   // pending hits of a warp
 constexpr int kBrickMax = 16;     // bricks per tile
 constexpr int kBrickFillWarps = 148 * 12;   // warps that fill the GPU
 constexpr int kBrickWideWarps = 148 * 24 * 4;   // narrow-form warps from which the wide forms are taken
+constexpr int64_t kBrick3DWidePairs = 4 << 20;   // pairs from which 8 coils in 3D take four slices
 constexpr int kBrickWideList = 512;     // average list up to which they are
 
 // Asynchronous copy of BYTES to shared memory; zeros instead when !full.
@@ -553,8 +554,13 @@ void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *d
 // takes 8 bricks per CTA where lists are short (they share the list's reads: 35.1
 // against 37.9 us for 1 frame) and 2 where they are long (96^2, 1 frame: 59 against 166 us) or
 // where that lets several warps share a brick's list (10400 samples on 192 x 128: 24 against 32 us).
-// 3D bricks are two slices thick (W = 4 meets 2.5 of them: 80 % of the slices
-// computed are hit).
+// 3D bricks of 16 and 32 coils are four slices thick, of the others two (W = 4
+// meets 2.5 of two: 80 % of the slices computed are hit).  8 coils have both: two
+// slices leave registers for 24 warps per SM instead of 16, four have fewer
+// (sample, brick) pairs.  Gridding of 5 coils, two / four slices, us: 64000 samples on 96^3 71 / 79,
+// 256000 on 64^3 205 / 276, 768000 on 160^3 (2 M pairs) 438 / 459, 2.56 M on 192^3 (6.7 M pairs) 1309 /
+// 1194.  One brick per CTA here too, two with 32 coils (2.56 M samples, 16 coils, 4 / 2 / 1: 2143 /
+// 2050 / 2005; 32 coils 4232 / 4222 / 4293).
 using Brick2D16 = BrickShape<2, 8, 4, 1, 8, 1, false, 256, 3, 8>;
 // Compensated; 8 CTAs per SM instead of 6: 11.52 -> 11.40 ms per refined solve at
 // 512^2 -> 640^2, 32 coils.
@@ -565,9 +571,10 @@ using Brick2D8 = BrickShape<2, 4, 8, 1, 8, 1, false, 256, 3>;
 using Brick2D4 = BrickShape<2, 2, 8, 2, 4, 1, false, 512, 2>;
 using Brick2D2 = BrickShape<2, 1, 8, 4, 2, 1, false, 512, 2>;
 using Brick2D1 = BrickShape<1, 1, 8, 4, 2, 1, false, 512, 2>;
-using Brick3D32 = BrickShape<2, 16, 2, 1, 4, 4, true, 128, 4>;
-using Brick3D16 = BrickShape<2, 8, 4, 1, 4, 4, true, 128, 4>;
-using Brick3D8 = BrickShape<2, 4, 8, 1, 4, 4, true, 128, 4>;
+using Brick3D32 = BrickShape<2, 16, 2, 1, 4, 4, true, 128, 4, 2>;
+using Brick3D16 = BrickShape<2, 8, 4, 1, 4, 4, true, 128, 4, 1>;
+using Brick3D8 = BrickShape<2, 4, 8, 1, 4, 2, true, 128, 6, 1>;
+using Brick3D8W = BrickShape<2, 4, 8, 1, 4, 4, true, 128, 4, 1>;
 using Brick3D16C = BrickShape<2, 8, 4, 1, 4, 2, true, 128, 4>;    // compensated
 using Brick3D8C = BrickShape<2, 4, 8, 1, 4, 2, true, 128, 4>;
 using Brick3D4 = BrickShape<2, 2, 8, 2, 4, 2, true, 256, 3>;
@@ -607,6 +614,7 @@ static bool with_brick(int D, int cg, bool comp, bool wide, F &&f) {
             return true;
         case 8:
             if (comp) f(Brick3D8C{}, C{});
+            else if (wide) f(Brick3D8W{}, P{});
             else f(Brick3D8{}, P{});
             return true;
         case 4: GB_EITHER(Brick3D4); return true;
@@ -657,7 +665,7 @@ bool brick_config(const NufftPlan &p, int nb, GridCfg &c) {
         }
         return true;
     }
-    return cut_tile(k, cg, comp, false, c);
+    return cut_tile(k, cg, comp, k.D == 3 && p.total_pairs >= kBrick3DWidePairs, c);
 }
 
 template <class S, bool COMP>

@@ -59,7 +59,7 @@ struct GridCfg {
     bool brick;       // k_grid_brick (else k_grid_nc2c)
     int cg;
     int nbricks;      // brick kernel: bricks per tile
-    bool wide;        // brick kernel: wide form of 16 coils
+    bool wide;        // brick kernel: the form for large launches
     int groups = 1;   // CTAs (split-tile counters) per tile
     int cpt;          // cell variant: cells per thread
     int ncg;

@@ -643,15 +643,17 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     // At most 512 or a 32nd of an SM's share, whichever is more: longer ones leave
     // SMs idle where there are few tiles (131072 samples a frame, 256^2, 18 coils, at
     // most 256 / 512 / 1024: 1 frame 124 / 123 / 137 us, 2 frames 190 / 183 / 203, 23 frames 1736 /
-    // 1687 / 1673; 5.12 M samples in 3D, 960 to a tile, 32 coils, 512 / 960: 16.81 / 16.50 ms for
-    // both directions).
+    // 1687 / 1673).  Not in 3D, whose partial tiles are larger (256000 samples on 64^3, 8
+    // coils, 512 / 1500: 318 / 275 us; 5.12 M on 192^3, 32 coils, 512 / 960: 16.81 / 16.50 ms
+    // for both directions).
     // Chunks of that length need more partial tiles; the entry point with a fixed scratch
     // takes chunks of up to split_len pairs when those do not fit (the coarse list).
     const int64_t total = goff[nkeys];
     const int64_t avg = total / std::max<uint32_t>(1, nkeys);
     const int split_len = (int)std::max<int64_t>(256, 2 * avg);
-    const int most[2] = {(int)std::min<int64_t>(std::max<int64_t>(total < 100000 ? 96 : 128, avg),
-                                                 std::max<int64_t>(512, total / (148 * 32))), split_len};   // chunk lengths: fine, coarse
+    const int64_t longest = k.D == 2 ? std::max<int64_t>(512, total / (148 * 32)) : avg;
+    const int most[2] = {(int)std::max<int64_t>(total < 100000 ? 96 : 128, std::min(avg, longest)),
+                         split_len};   // chunk lengths: fine, coarse
     // equal lengths share a run up to 64K pairs; the few lists above keep key order in the last one
     const uint32_t cap = (uint32_t)std::min(split_len, 1 << 16);
     std::vector<uint32_t> light_at((size_t)cap + 1, 0u);

@@ -145,6 +145,20 @@ def test_long_lists(cuda, coils, W):
     _adjoint_and_normal((32, 32), (64, 64), W, S.radial_golden_angle_2d(150, 200), coils, 0, cuda)
 
 
+def test_3d_four_slices_of_8_coils(cuda):
+    """More than 4 M (tile, sample) pairs: the four-slice form of 5 to 8 coils."""
+    N, mos, W, coils = (32, 32, 32), (64, 64, 64), 4.0, 5
+    traj = np.random.default_rng(2).uniform(-0.5, 0.5, (1400000, 3)).astype(np.float32)
+    y = _samples(coils, traj.shape[0], 6)
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    g = torch.empty((coils, 1) + mos, dtype=torch.complex64, device=cuda)
+    plan.convolve(torch.from_numpy(y).to(cuda), g, gb.NFFT_conv_mode.NC2C)
+    orc = O.OraclePlan(N, mos, W)
+    orc.preprocess(traj.reshape(1, -1, 3))
+    assert rel_l2(g.cpu().numpy(), orc.convolve_nc2c(y)) <= PARITY_TOL
+
+
 def test_autotune_of_a_16_coil_series(cuda):
     """The autotuner times every candidate tile on a launch of the wide form,
     and leaves a plan that reconstructs."""
