@@ -491,35 +491,39 @@ k_grid_brick(ConvArgs a, const float2 *__restrict__ samples, float2 *__restrict_
     }
 }
 
-// 32 samples x 32 coils per block through shared memory: the planes are read
-// along the samples, the rows written along the coils.
+// CT coils x 1024 / CT samples per block through shared memory: the planes are
+// read along the samples, the rows written along the coils.
+template <int CT>
 __global__ void __launch_bounds__(256) k_samples_il(const float2 *__restrict__ samples, const float *__restrict__ dcw,
                                                     const uint32_t *__restrict__ perm, int64_t M, int nb, int il,
                                                     float2 *__restrict__ rows) {
-    __shared__ float2 t[32][33];
+    constexpr int SB = 1024 / CT;   // samples per block
+    __shared__ float2 t[CT][SB + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t i0 = (int64_t)blockIdx.x * 32;
-    const int c0 = (int)blockIdx.y * 32;
-    const int64_t i = i0 + lane;
-    uint32_t j = 0;
-    float w = 1.f;
-    if (i < M) {
-        j = perm[i];
-        if (dcw) w = dcw[j];
+    const int64_t i0 = (int64_t)blockIdx.x * SB;
+    const int c0 = (int)blockIdx.y * CT;
+    uint32_t j[SB / 32];
+    float w[SB / 32];
+#pragma unroll
+    for (int g = 0; g < SB / 32; g++) {
+        const int64_t i = i0 + 32 * g + lane;
+        j[g] = i < M ? perm[i] : 0u;
+        w[g] = dcw && i < M ? dcw[j[g]] : 1.f;
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        const int c = c0 + warp + 8 * q;
+        const int ct = warp + 8 * (q % (CT / 8)), g = q / (CT / 8);
+        const int c = c0 + ct;
         float2 v = make_float2(0.f, 0.f);
-        if (i < M && c < nb) {
-            v = samples[(int64_t)c * M + j];
-            if (dcw) v = make_float2(w * v.x, w * v.y);
+        if (i0 + 32 * g + lane < M && c < nb) {
+            v = samples[(int64_t)c * M + j[g]];
+            if (dcw) v = make_float2(w[g] * v.x, w[g] * v.y);
         }
-        t[warp + 8 * q][lane] = v;
+        t[ct][32 * g + lane] = v;
     }
     __syncthreads();
-    const int cn = min(32, il - c0);
-    for (int e = threadIdx.x; e < 32 * cn; e += 256) {
+    const int cn = min(CT, il - c0);
+    for (int e = threadIdx.x; e < SB * cn; e += 256) {
         const int r = e / cn, c = e - r * cn;
         if (i0 + r < M) rows[(i0 + r) * il + c0 + c] = t[c][r];
     }
@@ -528,8 +532,13 @@ __global__ void __launch_bounds__(256) k_samples_il(const float2 *__restrict__ s
 void launch_samples_il(const NufftPlan &p, const float2 *samples, const float *dcw, int nb, float2 *rows,
                        cudaStream_t st) {
     const int il = il_stride_for(nb);
-    const dim3 g((unsigned)((p.Mtot + 31) / 32), (unsigned)((il + 31) / 32));
-    k_samples_il<<<g, 256, 0, st>>>(samples, dcw, p.perm.get(), p.Mtot, nb, il, rows); note_launch();
+    auto go = [&](auto kern, int ct) {
+        const dim3 g((unsigned)((p.Mtot + 1024 / ct - 1) / (1024 / ct)), (unsigned)((il + ct - 1) / ct));
+        kern<<<g, 256, 0, st>>>(samples, dcw, p.perm.get(), p.Mtot, nb, il, rows); note_launch();
+    };
+    if (il <= 8) go(k_samples_il<8>, 8);
+    else if (il <= 16) go(k_samples_il<16>, 16);
+    else go(k_samples_il<32>, 32);
     GB_CUDA(cudaGetLastError());
 }
 

@@ -834,7 +834,7 @@ void launch_grid_prepare(NufftPlan &p, int nb, cudaStream_t st) {
 constexpr int kIlMinCoils[2] = {9, 5};
 
 void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, SampleLayout layout,
-                 const float *dcw, bool sign_fold, bool accumulate, cudaStream_t st, const KLayout *kl, bool use_ws) {
+                 const float *dcw, bool sign_fold, bool accumulate, cudaStream_t st, const KLayout *kl, DevBuf<float2> *rows) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "preprocess has not been called");
     const GridCfg c = grid_config(p, nb);
     if (layout == LAYOUT_SORTED_IL && (!c.brick || dcw))
@@ -849,17 +849,17 @@ void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, Samp
     // during a capture, or has no room.
     const float2 *src = samples;
     SampleLayout lay = layout;
-    if (use_ws && c.brick && c.cg >= 2 && layout == LAYOUT_ORIGINAL && nb >= kIlMinCoils[p.D == 3]) {
+    if (rows && c.brick && c.cg >= 2 && layout == LAYOUT_ORIGINAL && nb >= kIlMinCoils[p.D == 3]) {
         const size_t need = (size_t)il_stride_for(nb) * p.Mtot;
-        bool room = p.samp_ws.n >= need;
+        bool room = rows->n >= need;
         if (!room) {
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             GB_CUDA(cudaStreamIsCapturing(st, &cs));
-            room = cs == cudaStreamCaptureStatusNone && p.samp_ws.try_ensure(need);
+            room = cs == cudaStreamCaptureStatusNone && rows->try_ensure(need);
         }
         if (room) {
-            launch_samples_il(p, samples, dcw, nb, p.samp_ws.get(), st);
-            src = p.samp_ws.get();
+            launch_samples_il(p, samples, dcw, nb, rows->get(), st);
+            src = rows->get();
             lay = LAYOUT_SORTED_IL;
         }
     }

@@ -306,6 +306,13 @@ struct NufftPlan {
     int64_t img_os_nbf = -1;       // batch count whose outer-major band the pad buffer holds
     DevBuf<float2> kgrid;     // k-space grid
     DevBuf<float2> samp_ws;   // samples in tile order [batches][Mtot]
+    // Interleaved samples of the standalone gridding, whose calls may overlap on
+    // one plan (streams, threads): a call waits for the event of the last user.
+    struct ConvRows {
+        std::mutex mu;
+        DevBuf<float2> buf;
+        cudaEvent_t done = nullptr;
+    } conv_rows;
     std::map<int, cufftHandle> fft_plans;   // batch -> plan (standard layout, rank D)
     std::map<std::pair<int, int>, cufftHandle> fft_plans_om;   // (batch, pass) -> plan (outer-major)
     std::map<int, DevBuf<float2>> fft_tw;   // transform length -> W_N^e table (project-written passes)
@@ -380,12 +387,12 @@ void launch_degrid(NufftPlan &p, const float2 *grid, float2 *samples, int nb,
                    bool accumulate, cudaStream_t st, const KLayout *kl = nullptr);
 
 // Gridding: samples -> grid [nb][F][G] (overwritten unless accumulate).
-// dcw multiplies the input samples (may be null).  use_ws: the plan's sample
-// workspace may hold the interleaved samples (not for calls that may overlap
-// on one plan).
+// dcw multiplies the input samples (may be null).  rows: a buffer that may hold
+// the interleaved samples while the launch runs (may be null: they are gathered
+// from the caller's array).
 void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb,
                  SampleLayout layout, const float *dcw, bool sign_fold, bool accumulate,
-                 cudaStream_t st, const KLayout *kl = nullptr, bool use_ws = true);
+                 cudaStream_t st, const KLayout *kl = nullptr, DevBuf<float2> *rows = nullptr);
 
 // Trajectory gradient from a k-space grid (sign folded like the degridder).
 void launch_traj_grad(NufftPlan &p, const float2 *grid, const float2 *weights, int nb,

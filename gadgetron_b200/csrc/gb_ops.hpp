@@ -96,9 +96,9 @@ void nufft_compute(NufftPlan &p, const void *in, void *out, const float *dcw, gb
 void nufft_mult_MH_M(NufftPlan &p, const void *in, void *out, const float *dcw, int nb, cudaStream_t st);
 void nufft_time_normal_convolutions(NufftPlan &p, int nb, const float *dcw, int reps, void *flush,
                                     size_t flush_bytes, float *ms_grid, float *ms_degrid, cudaStream_t st);
-// use_ws: gridding may use the plan's sample workspace (the plan serves one call at a time).
+// one_call: the plan serves one call at a time (gridding may use its sample workspace).
 void nufft_convolve(NufftPlan &p, const void *in, void *out, gb_conv_mode mode, bool accumulate, int nb,
-                    cudaStream_t st, bool use_ws = false);
+                    cudaStream_t st, bool one_call = false);
 void nufft_fft(NufftPlan &p, void *data, gb_fft_mode mode, bool do_scale, int nbf, cudaStream_t st);
 void nufft_deapodize(NufftPlan &p, void *data, int nbf, cudaStream_t st);
 void nufft_traj_grad(NufftPlan &p, const float2 *img, const float2 *weights, const float *dcw, float *grad,

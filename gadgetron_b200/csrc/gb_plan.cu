@@ -32,6 +32,7 @@ NufftPlan::~NufftPlan() {
     for (auto &g : prep_graph)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     if (h_stage) cudaFreeHost(h_stage);
+    if (conv_rows.done) cudaEventDestroy(conv_rows.done);
     if (upload_done) {
         cudaEventSynchronize(upload_done);
         cudaEventDestroy(upload_done);

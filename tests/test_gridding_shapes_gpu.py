@@ -145,6 +145,40 @@ def test_long_lists(cuda, coils, W):
     _adjoint_and_normal((32, 32), (64, 64), W, S.radial_golden_angle_2d(150, 200), coils, 0, cuda)
 
 
+@pytest.mark.parametrize("coils,m", [(9, 32767), (9, 32768), (16, 33000), (20, 33000)])
+def test_convolve_on_two_streams(cuda, coils, m):
+    """The standalone gridding from the caller's array and, from 32768 samples
+    and 9 coils on, through the plan's rows: calls on two streams in turn, then
+    one under capture, give the same as the oracle."""
+    N, mos, W = (64, 64), (128, 128), 4.0
+    traj = np.random.default_rng(m).uniform(-0.5, 0.5, (m, 2)).astype(np.float32)
+    plan = gb.NFFT.make_plan(N, mos, W)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    orc = O.OraclePlan(N, mos, W)
+    orc.preprocess(traj[None])
+    ys = [_samples(coils, m, s) for s in (1, 2)]
+    yt = [torch.from_numpy(y).to(cuda) for y in ys]
+    out = [torch.empty((coils, 1) + mos, dtype=torch.complex64, device=cuda) for _ in ys]
+    plan.convolve(yt[0], out[0], gb.NFFT_conv_mode.NC2C)   # allocations before the overlap
+    streams = [torch.cuda.Stream() for _ in ys]
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for s, y, o in zip(streams, yt, out):
+            with torch.cuda.stream(s):
+                plan.convolve(y, o, gb.NFFT_conv_mode.NC2C)
+    torch.cuda.synchronize()
+    refs = [orc.convolve_nc2c(y) for y in ys]
+    for o, r in zip(out, refs):
+        assert rel_l2(o.cpu().numpy(), r) <= PARITY_TOL
+    graph = torch.cuda.CUDAGraph()
+    out[0].zero_()
+    with torch.cuda.graph(graph):
+        plan.convolve(yt[0], out[0], gb.NFFT_conv_mode.NC2C)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert rel_l2(out[0].cpu().numpy(), refs[0]) <= PARITY_TOL
+
+
 def test_3d_four_slices_of_8_coils(cuda):
     """More than 4 M (tile, sample) pairs: the four-slice form of 5 to 8 coils."""
     N, mos, W, coils = (32, 32, 32), (64, 64, 64), 4.0, 5
