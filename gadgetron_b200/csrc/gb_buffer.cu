@@ -14,15 +14,6 @@ namespace gb {
 
 namespace {
 
-__global__ void k_scale_samples(const float2 *__restrict__ in, const float *__restrict__ dcw, int nb, int64_t M,
-                                float2 *__restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)nb * M) return;
-    const float w = dcw[i % M];
-    const float2 v = in[i];
-    out[i] = make_float2(v.x * w, v.y * w);
-}
-
 // acc += cur; acc -= next
 __global__ void k_cycle_update(float2 *__restrict__ acc, const float2 *__restrict__ cur,
                                const float2 *__restrict__ next, int64_t n) {
@@ -111,15 +102,7 @@ bool SenseBuffer::add_frame_data(const float2 *samples, const float *traj, int64
     const int64_t slot = (int64_t)coils * p.kp.G;
     float2 *cur = cyc.get() + (int64_t)cur_idx * slot;
     plan_preprocess(p, traj, (uint64_t)M, 1, nullptr, GB_PREP_NC2C, st);
-    const float2 *in = samples;
-    if (dcw) {
-        scaled.ensure((size_t)coils * M);
-        k_scale_samples<<<blocks_of((int64_t)coils * M), 256, 0, st>>>(samples, dcw, coils, M, scaled.get());
-        note_launch();
-        GB_CUDA(cudaGetLastError());
-        in = scaled.get();
-    }
-    nufft_convolve(p, in, cur, GB_CONV_NC2C, true, coils, st, true);
+    nufft_convolve(p, samples, cur, GB_CONV_NC2C, true, coils, st, true, dcw);
     bool completed = false;
     if (cur_sub_idx == sub_cycle_length - 1) {
         completed = true;

@@ -732,7 +732,7 @@ static ConvArgs make_args(NufftPlan &p, int nb, SampleLayout layout, const float
     a.wtab = p.wtab.get();
     a.kl = klayout_standard(p.kp);
     a.prows = p.pair_rows.get();
-    a.prng = p.pair_rng.get();
+    a.prng = p.pair_rng;
     a.prow_floats = p.pair_row_stride;
     a.perm = p.perm.get();
     a.Mtot = p.Mtot;
@@ -812,20 +812,37 @@ static void grid_dispatch_cfg(const GridCfg &c, const NufftPlan &p, const ConvAr
     GB_CUDA(cudaGetLastError());
 }
 
-// Allocates the split-tile counters and partial buffers for `nb` batches
-// (must run outside stream capture).
-void launch_grid_prepare(NufftPlan &p, int nb, cudaStream_t st) {
-    const GridCfg c = grid_config(p, nb);
-    if (p.n_splits > 0) {
-        const size_t need_ctr = (size_t)p.n_splits * c.ncg * c.groups;
-        if (p.split_counters.n < need_ctr || p.split_counter_groups == 0) {
-            p.split_counters.ensure(need_ctr);
-            GB_CUDA(cudaMemsetAsync(p.split_counters.get(), 0, p.split_counters.n * sizeof(unsigned int), st));
-            p.split_counter_groups = c.ncg * c.groups;
-        }
-        p.partials.ensure((size_t)p.n_slots * c.ncg * c.part_elems);
+// Counters and partial tiles of the split tiles for one launch (null without
+// splits), grown where they have to be.
+struct SplitScratch {
+    unsigned int *counters = nullptr;
+    float2 *partials = nullptr;
+};
+
+static SplitScratch take_split_scratch(NufftPlan &p, const GridCfg &c, cudaStream_t st) {
+    SplitScratch g;
+    if (p.n_splits == 0) return g;
+    const size_t ctr = ((size_t)p.n_splits * c.ncg * c.groups * sizeof(unsigned int) + 255) & ~(size_t)255;
+    const size_t part = (size_t)p.n_slots * c.ncg * c.part_elems * sizeof(float2);
+    if (ctr > p.grid_ctr_bytes) {   // the partial tiles move: nothing recorded earlier may share the allocation
+        p.grid_ws.release();
+        p.grid_ctr_bytes = ctr;
     }
+    if (p.grid_ws.ensure(p.grid_ctr_bytes + part)) p.grid_ctr_clean = false;
+    if (!p.grid_ctr_clean) {
+        GB_CUDA(cudaMemsetAsync(p.grid_ws.get(), 0, p.grid_ctr_bytes, st));
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        GB_CUDA(cudaStreamIsCapturing(st, &cs));
+        p.grid_ctr_clean = cs == cudaStreamCaptureStatusNone;   // a captured clear has not run yet
+    }
+    g.counters = reinterpret_cast<unsigned int *>(p.grid_ws.get());
+    g.partials = reinterpret_cast<float2 *>(p.grid_ws.get() + p.grid_ctr_bytes);
+    return g;
 }
+
+// Allocates the gridding scratch for `nb` batches (must run outside stream
+// capture).
+void launch_grid_prepare(NufftPlan &p, int nb, cudaStream_t st) { take_split_scratch(p, grid_config(p, nb), st); }
 
 // Coils from which the adjoint lays the caller's samples into rows (2D, 3D).
 // Adjoint in us, gathering / with rows: 49152 samples on 512^2, 5 coils 43.5 / 46.5, 8
@@ -833,36 +850,33 @@ void launch_grid_prepare(NufftPlan &p, int nb, cudaStream_t st) {
 // 24.8; 2.56 M samples on 192^3, 5 coils 1773 / 1686, 8 coils 1969 / 1866.
 constexpr int kIlMinCoils[2] = {9, 5};
 
+// The caller's samples are one plane per coil: from kIlMinCoils coils on they
+// are first laid into sorted coil-interleaved rows (density weights folded in),
+// so that a hit loads its coils as one run instead of one sector per coil.
+// Only for coil pairs per lane (a coil group of 1 can be asked for with any
+// coil count).  0: no rows.
+size_t grid_row_elems(const NufftPlan &p, int nb) {
+    if (nb < kIlMinCoils[p.D == 3]) return 0;
+    const GridCfg c = grid_config(p, nb);
+    return c.brick && c.cg >= 2 ? (size_t)il_stride_for(nb) * p.Mtot : 0;
+}
+
 void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, SampleLayout layout,
-                 const float *dcw, bool sign_fold, bool accumulate, cudaStream_t st, const KLayout *kl, DevBuf<float2> *rows) {
+                 const float *dcw, bool sign_fold, bool accumulate, cudaStream_t st, const KLayout *kl, float2 *rows) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "preprocess has not been called");
     const GridCfg c = grid_config(p, nb);
     if (layout == LAYOUT_SORTED_IL && (!c.brick || dcw))
         fail(GB_ERR_INTERNAL, "interleaved samples need the brick gridding kernel and no density weights");
     if (p.n_grd_items == 0) return;
     const ConvArgs orig = make_args(p, nb, layout, dcw, 1, sign_fold, accumulate);
-    // The caller's samples are one plane per coil: from kIlMinCoils coils on
-    // they are first laid into sorted coil-interleaved rows (density weights
-    // folded in), so that a hit loads its coils as one run instead of one
-    // sector per coil.  Only for coil pairs per lane (a coil group of 1 can be
-    // asked for with any coil count), and not when that would have to allocate
-    // during a capture, or has no room.
     const float2 *src = samples;
     SampleLayout lay = layout;
-    if (rows && c.brick && c.cg >= 2 && layout == LAYOUT_ORIGINAL && nb >= kIlMinCoils[p.D == 3]) {
-        const size_t need = (size_t)il_stride_for(nb) * p.Mtot;
-        bool room = rows->n >= need;
-        if (!room) {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            GB_CUDA(cudaStreamIsCapturing(st, &cs));
-            room = cs == cudaStreamCaptureStatusNone && rows->try_ensure(need);
-        }
-        if (room) {
-            launch_samples_il(p, samples, dcw, nb, rows->get(), st);
-            src = rows->get();
-            lay = LAYOUT_SORTED_IL;
-        }
+    if (rows && layout == LAYOUT_ORIGINAL && grid_row_elems(p, nb) > 0) {
+        launch_samples_il(p, samples, dcw, nb, rows, st);
+        src = rows;
+        lay = LAYOUT_SORTED_IL;
     }
+    const SplitScratch ws = take_split_scratch(p, c, st);
     ConvArgs a = make_args(p, nb, lay, lay == layout ? dcw : nullptr, 1, sign_fold, accumulate);
     if (kl) a.kl = *kl;
     a.list = p.grid_list.get();
@@ -871,11 +885,8 @@ void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb, Samp
     a.splits = p.splits.get();
     a.ncg = c.ncg;
     a.part_elems = c.part_elems;
-    launch_grid_prepare(p, nb, st);
-    if (p.n_splits > 0) {
-        a.partials = p.partials.get();
-        a.counters = p.split_counters.get();
-    }
+    a.partials = ws.partials;
+    a.counters = ws.counters;
     grid_dispatch_cfg(c, p, a, src, grid, st);
     ConvArgs fix = orig;
     fix.kl = a.kl;

@@ -275,8 +275,9 @@ struct NufftPlan {
     // weights (tile z, 3D), padding to a multiple of 4; and the tile-local
     // footprint range, bytes (x lo, x hi, y lo, y hi, z lo, z hi, 0, 0).
     // Built at preprocess for D >= 2 (pair_row_stride = 0 when not built).
+    // (one allocation: the rows, then the ranges)
     DevBuf<float> pair_rows;
-    DevBuf<uint2> pair_rng;
+    uint2 *pair_rng = nullptr;
     int pair_row_stride = 0;
     DevBuf<unsigned int> err_flag;   // set by kernels whose bounded waits ran out
     DevBuf<uint32_t> grid_off;     // [F*ntiles + 1]
@@ -289,9 +290,12 @@ struct NufftPlan {
     // The split tiles in longer chunks: items after the n_grd_items of
     // grd_items, their n_splits table entries after the first n_splits.
     int n_light_items = 0, n_coarse_items = 0, n_coarse_slots = 0;
-    DevBuf<unsigned int> split_counters;   // [n_splits * max coil groups]
-    int split_counter_groups = 0;
-    DevBuf<float2> partials;               // [n_slots][cg_groups][cells*cg]
+    // Scratch of the split tiles, one allocation: counters [n_splits][coil
+    // groups][CTAs of a tile] (zero between launches), then partial tiles
+    // [n_slots][coil groups][cells * coils].
+    DevBuf<unsigned char> grid_ws;
+    size_t grid_ctr_bytes = 0;     // room for the counters
+    bool grid_ctr_clean = false;
     int64_t total_pairs = 0;
 
     // deapodization: per-dim reciprocal of the 1D kernel transform
@@ -304,7 +308,7 @@ struct NufftPlan {
     size_t img_os_batches_zeroed = 0;
     bool img_os_dirty = true;
     int64_t img_os_nbf = -1;       // batch count whose outer-major band the pad buffer holds
-    DevBuf<float2> kgrid;     // k-space grid
+    DevBuf<float2> kgrid;     // k-space grid, and after it room for the adjoint's sample rows
     DevBuf<float2> samp_ws;   // samples in tile order [batches][Mtot]
     // Interleaved samples of the standalone gridding, whose calls may overlap on
     // one plan (streams, threads): a call waits for the event of the last user.
@@ -387,12 +391,13 @@ void launch_degrid(NufftPlan &p, const float2 *grid, float2 *samples, int nb,
                    bool accumulate, cudaStream_t st, const KLayout *kl = nullptr);
 
 // Gridding: samples -> grid [nb][F][G] (overwritten unless accumulate).
-// dcw multiplies the input samples (may be null).  rows: a buffer that may hold
-// the interleaved samples while the launch runs (may be null: they are gathered
-// from the caller's array).
+// dcw multiplies the input samples (may be null).  rows: room for
+// grid_row_elems() elements that hold the interleaved samples while the launch
+// runs (null: they are gathered from the caller's array).
+size_t grid_row_elems(const NufftPlan &p, int nb);
 void launch_grid(NufftPlan &p, const float2 *samples, float2 *grid, int nb,
                  SampleLayout layout, const float *dcw, bool sign_fold, bool accumulate,
-                 cudaStream_t st, const KLayout *kl = nullptr, DevBuf<float2> *rows = nullptr);
+                 cudaStream_t st, const KLayout *kl = nullptr, float2 *rows = nullptr);
 
 // Trajectory gradient from a k-space grid (sign folded like the degridder).
 void launch_traj_grad(NufftPlan &p, const float2 *grid, const float2 *weights, int nb,

@@ -39,9 +39,26 @@ float2 *ensure_img_os(NufftPlan &p, int64_t nbf, cudaStream_t st) {
     return p.img_os.get();
 }
 
+// One allocation with the adjoint's sample rows behind the grid: a plan's first
+// adjoint would pay 0.3 ms for another one.  (Rows of a later, larger
+// trajectory go to the sample workspace: the grid is not moved for them.)
 float2 *ensure_kgrid(NufftPlan &p, int64_t nbf) {
-    p.kgrid.ensure((size_t)nbf * p.kp.G);
+    const size_t need = (size_t)nbf * p.kp.G;
+    const size_t rows = p.kgrid.n < need && p.F > 0 ? grid_row_elems(p, (int)(nbf / p.F)) : 0;
+    if (rows == 0 || !p.kgrid.try_ensure(need + rows)) p.kgrid.ensure(need);
     return p.kgrid.get();
+}
+
+// Room for `need` elements in `buf`; null when there is none, or when it would have to
+// be allocated in a capture.
+static float2 *rows_in(DevBuf<float2> &buf, size_t need, cudaStream_t st) {
+    if (need == 0) return nullptr;
+    if (buf.n < need) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        GB_CUDA(cudaStreamIsCapturing(st, &cs));
+        if (cs != cudaStreamCaptureStatusNone || !buf.try_ensure(need)) return nullptr;
+    }
+    return buf.get();
 }
 
 float2 *ensure_samp(NufftPlan &p, int nb) {
@@ -193,7 +210,9 @@ void nufft_adjoint(NufftPlan &p, const float2 *samples, SampleLayout layout, con
     const int64_t nbf = (int64_t)nb * p.F;
     const KLayout kl = ws_layout(p, nbf);
     float2 *kg = ensure_kgrid(p, nbf);
-    launch_grid(p, samples, kg, nb, layout, dcw, true, false, st, &kl, &p.samp_ws);
+    const size_t rows = layout == LAYOUT_ORIGINAL ? grid_row_elems(p, nb) : 0, cells = (size_t)nbf * p.kp.G;
+    launch_grid(p, samples, kg, nb, layout, dcw, true, false, st, &kl,
+                p.kgrid.n >= cells + rows ? kg + cells : rows_in(p.samp_ws, rows, st));
     fft_adjoint_ws(p, kg, (int)nbf, fft_dir, !img_os, st);
     launch_crop_adjoint(p, kg, csm, img, nb, img_os, accumulate, weight, fft_dir == CUFFT_FORWARD, st, &kl);
 }
@@ -282,15 +301,16 @@ void nufft_mult_MH_M(NufftPlan &p, const void *in, void *out, const float *dcw, 
 // 73.1 / 69.0; 32 coils 69.3 / 66.0 and 135 / 122.  Below, the extra launch costs what it saves.
 constexpr int64_t kConvRowsSamples = 32768;
 
-static void convolve_nc2c(NufftPlan &p, const float2 *in, float2 *out, int nb, bool accumulate, bool one_call,
-                          cudaStream_t st) {
-    auto grid = [&](DevBuf<float2> *rows) {
-        launch_grid(p, in, out, nb, LAYOUT_ORIGINAL, nullptr, false, accumulate, st, nullptr, rows);
+static void convolve_nc2c(NufftPlan &p, const float2 *in, float2 *out, const float *dcw, int nb, bool accumulate,
+                          bool one_call, cudaStream_t st) {
+    const size_t need = grid_row_elems(p, nb);
+    auto grid = [&](float2 *rows) {
+        launch_grid(p, in, out, nb, LAYOUT_ORIGINAL, dcw, false, accumulate, st, nullptr, rows);
     };
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     GB_CUDA(cudaStreamIsCapturing(st, &cs));
-    if (one_call || p.Mtot < kConvRowsSamples || cs != cudaStreamCaptureStatusNone) {
-        grid(one_call ? &p.samp_ws : nullptr);
+    if (one_call || need == 0 || p.Mtot < kConvRowsSamples || cs != cudaStreamCaptureStatusNone) {
+        grid(one_call ? rows_in(p.samp_ws, need, st) : nullptr);
         return;
     }
     // Calls on one plan may overlap: the rows pass from user to user by an event
@@ -298,19 +318,19 @@ static void convolve_nc2c(NufftPlan &p, const float2 *in, float2 *out, int nb, b
     std::lock_guard<std::mutex> lock(p.conv_rows.mu);
     if (!p.conv_rows.done) GB_CUDA(cudaEventCreateWithFlags(&p.conv_rows.done, cudaEventDisableTiming));
     GB_CUDA(cudaStreamWaitEvent(st, p.conv_rows.done, 0));
-    grid(&p.conv_rows.buf);
+    grid(rows_in(p.conv_rows.buf, need, st));
     GB_CUDA(cudaEventRecord(p.conv_rows.done, st));
 }
 
 void nufft_convolve(NufftPlan &p, const void *in, void *out, gb_conv_mode mode, bool accumulate, int nb,
-                    cudaStream_t st, bool one_call) {
+                    cudaStream_t st, bool one_call, const float *dcw) {
     if (!p.prepped) fail(GB_ERR_NOT_PREPROCESSED, "NFFT_plan::convolve: preprocess has not been called");
     if (!in || !out) fail(GB_ERR_INVALID_ARGUMENT, "NULL input/output");
     if (mode == GB_CONV_C2NC)
         launch_degrid(p, static_cast<const float2 *>(in), static_cast<float2 *>(out), nb, LAYOUT_ORIGINAL,
                       nullptr, 1, false, accumulate, st);
     else
-        convolve_nc2c(p, static_cast<const float2 *>(in), static_cast<float2 *>(out), nb, accumulate, one_call, st);
+        convolve_nc2c(p, static_cast<const float2 *>(in), static_cast<float2 *>(out), dcw, nb, accumulate, one_call, st);
 }
 
 void nufft_fft(NufftPlan &p, void *data, gb_fft_mode mode, bool do_scale, int nbf, cudaStream_t st) {

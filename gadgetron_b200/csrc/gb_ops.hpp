@@ -96,9 +96,10 @@ void nufft_compute(NufftPlan &p, const void *in, void *out, const float *dcw, gb
 void nufft_mult_MH_M(NufftPlan &p, const void *in, void *out, const float *dcw, int nb, cudaStream_t st);
 void nufft_time_normal_convolutions(NufftPlan &p, int nb, const float *dcw, int reps, void *flush,
                                     size_t flush_bytes, float *ms_grid, float *ms_degrid, cudaStream_t st);
-// one_call: the plan serves one call at a time (gridding may use its sample workspace).
+// one_call: the plan serves one call at a time (gridding may use its sample
+// workspace); dcw: weights of the samples (NC2C; may be null).
 void nufft_convolve(NufftPlan &p, const void *in, void *out, gb_conv_mode mode, bool accumulate, int nb,
-                    cudaStream_t st, bool one_call = false);
+                    cudaStream_t st, bool one_call = false, const float *dcw = nullptr);
 void nufft_fft(NufftPlan &p, void *data, gb_fft_mode mode, bool do_scale, int nbf, cudaStream_t st);
 void nufft_deapodize(NufftPlan &p, void *data, int nbf, cudaStream_t st);
 void nufft_traj_grad(NufftPlan &p, const float2 *img, const float2 *weights, const float *dcw, float *grad,
@@ -115,7 +116,7 @@ struct SenseBuffer {
     bool has_acc_image = false;   // the last accumulated coil images (reused by the combined image)
     const float *dcw = nullptr;   // retained
     const float2 *csm = nullptr;  // retained
-    DevBuf<float2> acc, cyc, scaled, work, acc_image;
+    DevBuf<float2> acc, cyc, work, acc_image;
     void setup(int D, const uint64_t *N, const uint64_t *mos, float W, int coils, int num_cycles,
                int num_sub_cycles, cudaStream_t st);
     void clear(cudaStream_t st);

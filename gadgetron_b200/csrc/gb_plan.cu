@@ -551,8 +551,8 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
     const bool rows = D >= 2 && pair_row_floats(k) <= 96 && npairs > 0;
     const int rf = rows ? pair_row_floats(k) : 0;
     if (rows) {
-        p.pair_rows.ensure((size_t)npairs * rf);
-        p.pair_rng.ensure(npairs);
+        p.pair_rows.ensure((size_t)npairs * (rf + 2));
+        p.pair_rng = reinterpret_cast<uint2 *>(p.pair_rows.get() + (size_t)npairs * rf);   // rf: a multiple of 4
     }
     uint64_t key_b = kp_hash;
     for (uint64_t v : {(uint64_t)npairs, (uint64_t)M, (uint64_t)nkeys, (uint64_t)rf,
@@ -560,7 +560,7 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
                        (uint64_t)(uintptr_t)poff.get(), (uint64_t)(uintptr_t)pkey.get(), (uint64_t)(uintptr_t)pval.get(),
                        (uint64_t)(uintptr_t)pkey_sorted.get(), (uint64_t)(uintptr_t)p.grid_list.get(),
                        (uint64_t)(uintptr_t)p.grid_off.get(), (uint64_t)(uintptr_t)p.wtab.get(),
-                       (uint64_t)(uintptr_t)p.pair_rows.get(), (uint64_t)(uintptr_t)p.pair_rng.get(),
+                       (uint64_t)(uintptr_t)p.pair_rows.get(),
                        (uint64_t)(uintptr_t)p.pp_sort.get(),
                        (uint64_t)p.pp_sort.n})
         key_b = mix_key(key_b, v);
@@ -576,7 +576,7 @@ void plan_preprocess(NufftPlan &p, const float *traj, uint64_t Mtot, uint32_t F,
             const int64_t ppb = 256 / (rf / 4);
             k_pair_rows<<<(unsigned)((npairs + ppb - 1) / ppb), 256, 0, s>>>(
                 k, M, (int64_t)npairs, p.pos_sorted.get(), p.wtab.get(), pkey_sorted.get(), p.grid_list.get(),
-                p.pair_rows.get(), rf, reinterpret_cast<uint16_t *>(p.pair_rng.get())); ::gb::note_launch();
+                p.pair_rows.get(), rf, reinterpret_cast<uint16_t *>(p.pair_rng)); ::gb::note_launch();
             GB_CUDA(cudaGetLastError());
         }
     });
@@ -733,7 +733,7 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     if (bg) GB_CUDA(cudaMemcpyAsync(p.grd_items.get(), grd, bg, cudaMemcpyHostToDevice, st));
     if (bs) GB_CUDA(cudaMemcpyAsync(p.splits.get(), splits, bs, cudaMemcpyHostToDevice, st));
     upload_issued(p, st);
-    p.split_counter_groups = 0;   // (re)allocated by the gridding launcher
+    p.grid_ctr_clean = false;   // cleared by the gridding launcher
 }
 
 uint64_t plan_layout_signature(const NufftPlan &p, int nbf) {
@@ -745,12 +745,12 @@ uint64_t plan_layout_signature(const NufftPlan &p, int nbf) {
         }
     };
     const void *ptrs[] = {p.pos_sorted.get(), p.wtab.get(), p.pair_rows.get(), p.perm.get(), p.grid_list.get(), p.grd_items.get(),
-                          p.deg_items.get(), p.splits.get(), p.partials.get(), p.split_counters.get(), p.pair_rng.get(),
+                          p.deg_items.get(), p.splits.get(), p.grid_ws.get(), p.pair_rng,
                           p.img_os.get(), p.kgrid.get(), p.samp_ws.get(), p.deap_img.get(), p.deap_os.get()};
     for (const void *q : ptrs) mix((uint64_t)(uintptr_t)q);
     const int64_t vals[] = {p.n_deg_items, p.n_grd_items, p.n_splits, p.n_slots, p.Mtot, (int64_t)p.F,
                             p.tiling.tile[0], p.tiling.tile[1], p.tiling.tile[2], p.tiling.cg, p.tiling.schedule,
-                            p.split_counter_groups, (int64_t)p.split_counters.n, (int64_t)p.partials.n, nbf};
+                            (int64_t)p.grid_ctr_bytes, (int64_t)p.grid_ws.n, nbf};
     for (int64_t v : vals) mix((uint64_t)v);
     auto it = p.fft_plans.find(nbf);
     mix(it == p.fft_plans.end() ? 0ull : (uint64_t)it->second);
