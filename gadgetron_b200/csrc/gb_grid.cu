@@ -909,6 +909,18 @@ void grid_scratch_need(const NufftPlan &p, int nb, bool coarse, size_t *partial_
     *counter_elems = p.n_splits > 0 ? (size_t)p.n_splits * c.ncg * c.groups : 0;
 }
 
+// Partial-tile elements by which the fixed-scratch entry point accepts a call:
+// long chunks, the batches rounded up to the plan's coil group (with compensated
+// sums, to a group whose sums fit the cell kernel's registers).  The forms may
+// take larger groups; such a call then runs on fewer batches at a time.
+size_t grid_scratch_accepted(const NufftPlan &p, int nb) {
+    const KParams &k = p.kp;
+    const int cells = k.tile[0] * k.tile[1] * k.tile[2], cpt = (cells + kThreads - 1) / kThreads;
+    int cg = choose_cg(p.tiling.cg, nb);
+    if (p.flags & GB_FLAG_COMPENSATED) cg = std::min(cg, std::max(1, 16 / cpt));
+    return p.n_splits > 0 ? (size_t)p.n_coarse_slots * ((nb + cg - 1) / cg * cg) * cells : 0;
+}
+
 // The gridding launch of launch_grid with caller-provided scratch: no device
 // allocation.  `counters` must hold counter_elems zeros on entry (the kernel
 // leaves them zero again when it completes).

@@ -20,6 +20,7 @@
 // every launch, the partial tiles are always written before they are read.
 // Calls that overlap on the GPU (other streams, other threads) race on the
 // array and must be serialised by the caller.
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -78,24 +79,38 @@ extern "C" GB_API gb_status gb_nufft_convolve_nc2c_noalloc(gb_nufft_plan plan, c
             int dev, cur;
             ~Restore() { if (dev != cur && dev >= 0) cudaSetDevice(dev); }
         } restore{old, p->device};
-        size_t need_partials = 0, need_counters = 0;
-        grid_scratch_need(*p, nb, false, &need_partials, &need_counters);
-        // split tiles in longer chunks when the short ones' partial tiles do not fit
-        const bool coarse = need_partials > kPartialElems;
-        if (coarse) grid_scratch_need(*p, nb, true, &need_partials, &need_counters);
-        if (need_partials > kPartialElems || need_counters > kCounterElems)
-            fail(GB_ERR_INVALID_ARGUMENT,
-                 "gb_nufft_convolve_nc2c_noalloc: this plan and batch count need " +
-                     std::to_string(need_partials * sizeof(float2) + need_counters * sizeof(unsigned int)) +
-                     " bytes of scratch, above the fixed " + std::to_string(kScratchBytes) + "-byte buffer");
+        size_t partials_elems = 0, counter_elems = 0;
+        auto fits = [&](int n, bool coarse) {
+            size_t c = 0;
+            grid_scratch_need(*p, n, coarse, &partials_elems, &c);
+            counter_elems = std::max(counter_elems, c);
+            return partials_elems <= kPartialElems && c <= kCounterElems;
+        };
+        // Split tiles in longer chunks when the short ones' partial tiles do not
+        // fit, and fewer batches at a time when those of all batches do not.
+        const bool coarse = !fits(nb, false);
+        int run = nb;
+        if (coarse && !fits(nb, true)) {
+            if (grid_scratch_accepted(*p, nb) > kPartialElems)
+                fail(GB_ERR_INVALID_ARGUMENT,
+                     "gb_nufft_convolve_nc2c_noalloc: this plan and batch count need " +
+                         std::to_string(partials_elems * sizeof(float2) + counter_elems * sizeof(unsigned int)) +
+                         " bytes of scratch, above the fixed " + std::to_string(kScratchBytes) + "-byte buffer");
+            while (run > 1 && !fits(run, true)) run = (run + 1) / 2;
+            if (!fits(run, true)) fail(GB_ERR_INTERNAL, "gridding scratch of one batch");
+        }
+        if (nb % run) fits(nb % run, coarse);   // the last, shorter run's counters
         unsigned char *base = static_cast<unsigned char *>(scratch_for_current_device());
         unsigned int *counters = reinterpret_cast<unsigned int *>(base);
         float2 *partials = reinterpret_cast<float2 *>(base + kCounterBytes);
         cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-        if (need_counters) check_cuda(cudaMemsetAsync(counters, 0, need_counters * sizeof(unsigned int), st),
-                                      "cudaMemsetAsync");
-        launch_grid_external_scratch(*p, static_cast<const float2 *>(samples), static_cast<float2 *>(grid),
-                                     nb, accumulate != 0, coarse, partials, counters, st);
+        counter_elems = std::min(counter_elems, kCounterElems);
+        if (counter_elems)   // left zero by every launch
+            check_cuda(cudaMemsetAsync(counters, 0, counter_elems * sizeof(unsigned int), st), "cudaMemsetAsync");
+        for (int b = 0; b < nb; b += run)
+            launch_grid_external_scratch(*p, static_cast<const float2 *>(samples) + (int64_t)b * p->Mtot,
+                                         static_cast<float2 *>(grid) + (int64_t)b * p->F * p->kp.G,
+                                         std::min(run, nb - b), accumulate != 0, coarse, partials, counters, st);
         return GB_OK;
     } catch (...) {
         return current_exception_status();

@@ -127,6 +127,7 @@ struct SenseBuffer {
 
 // Gridding with caller-provided scratch (no device allocation).
 void grid_scratch_need(const NufftPlan &p, int nb, bool coarse, size_t *partial_elems, size_t *counter_elems);
+size_t grid_scratch_accepted(const NufftPlan &p, int nb);
 void launch_grid_external_scratch(NufftPlan &p, const float2 *samples, float2 *grid, int nb, bool accumulate,
                                   bool coarse, float2 *partials, unsigned int *counters, cudaStream_t st);
 // The plan behind a C handle (defined with the C ABI).

@@ -272,3 +272,28 @@ def test_noalloc_long_chunks_when_the_short_ones_do_not_fit(cuda):
             accepted = nb
             assert rel_l2(out[:nb].cpu().numpy(), ref[:nb].cpu().numpy()) <= PARITY_TOL
     assert accepted >= 8
+
+
+def test_noalloc_groups_larger_than_the_scratch(cuda):
+    """48 coils in 3D run as two groups of 32 and need the scratch of 64; where
+    48 coils' partial tiles fit and 64 coils' do not, the call is accepted and
+    runs on fewer coils at a time."""
+    N, mos, W, C = (32, 32, 32), (64, 64, 64), 4.0, 64
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def noalloc(plan, y, out, nb):
+        return lib.gb_nufft_convolve_nc2c_noalloc(plan._h, ctypes.c_void_p(y.data_ptr()),
+                                                  ctypes.c_void_p(out.data_ptr()), 0, nb, stream)
+
+    for spokes in range(40, 600, 20):
+        traj = S.kooshball_golden_means_3d(spokes, 48)
+        plan = gb.NFFT.make_plan(N, mos, W)
+        plan.preprocess(torch.from_numpy(traj).to(cuda))
+        y = torch.from_numpy(_samples(C, traj.shape[0], 2)).to(cuda)
+        out = torch.full((C, 1) + mos, float("nan"), dtype=torch.complex64, device=cuda)
+        if noalloc(plan, y, out, 48) == 0 and noalloc(plan, y, out, 64) == 1:
+            ref = torch.empty((48, 1) + mos, dtype=torch.complex64, device=cuda)
+            plan.convolve(y[:48].contiguous(), ref, gb.NFFT_conv_mode.NC2C)
+            assert rel_l2(out[:48].cpu().numpy(), ref.cpu().numpy()) <= PARITY_TOL
+            return
+    pytest.fail("no trajectory between the two scratch sizes")
