@@ -199,12 +199,12 @@ void sdc_iterations(const SdcArgs &a, const float *traj, float *w, float *grid, 
 // sample's first cell, zero outside the disc) that every iteration reads back
 // from L2: four coalesced loads per lane take the place of the square roots and
 // polynomials that bound the direct passes.  A tap that rounding may put beyond
-// the square lies at |u| = R, where the weight is zero.  49152 samples, width
-// 5.5, 512^2, 10 iterations: 534 -> 352 us a call; bound now by the L2 atomics
-// and gathers of the footprints.  The table is taken up to kSdcTableSamples
-// samples (128 MiB of scratch, what L2 holds); above, for one iteration (nothing
-// to reuse), for other dimensions and for wider kernels, every pass evaluates the
-// weights.
+// the square lies at |u| = R, where the weight is zero.  Width 5.5, 512^2, 10
+// iterations, without / with the table, us a call: 16384 samples 275 / 241, 49152 536 /
+// 355, 262144 2302 / 1334, 524288 4471 / 2483; bound now by the L2 atomics and gathers of the
+// footprints.  The table pays at every size; kSdcTableSamples bounds the scratch
+// kept between calls (128 MiB).  Above it, for one iteration (nothing to reuse),
+// for other dimensions and for wider kernels, every pass evaluates the weights.
 constexpr int kSdcRounds = 4;
 constexpr int64_t kSdcTableSamples = (int64_t)1 << 18;
 
@@ -320,6 +320,10 @@ void sdc_table_iterations(const SdcArgs &a, int cap, const float *traj, float *w
 }
 
 // Scratch kept per device between calls; the mutex is held for a whole call.
+// Beyond the one grid a call needs it keeps at most the table of
+// kSdcTableSamples samples (128 MiB) and a second grid of kSdcTwoGrids cells (64 MiB;
+// a larger grid is cleared by a copy engine pass that costs little beside its iteration).
+constexpr int64_t kSdcTwoGrids = (int64_t)1 << 24;
 struct SdcScratch {
     std::mutex mu;
     DevBuf<unsigned int> bad;
@@ -388,9 +392,9 @@ void sdc_estimate_dcw(int D, const uint64_t *N, float os_factor, int iterations,
     } else {
         k_fill<<<sb, tb, 0, st>>>(dcw, M, 1.f); note_launch();
     }
-    // two grids in turn up to 1 GiB each; where they or the table do not fit,
-    // one grid and the direct passes
-    const bool two = G <= ((int64_t)1 << 28) && sc.grid.try_ensure(2 * (size_t)G);
+    // two grids in turn up to kSdcTwoGrids cells; where they or the table do not
+    // fit, one grid and the direct passes
+    const bool two = G <= kSdcTwoGrids && sc.grid.try_ensure(2 * (size_t)G);
     if (!two) sc.grid.ensure((size_t)G);
     const int cap = sdc_table_cap(a, two, iterations);
     if (cap > 0 && sc.table.try_ensure((size_t)M * 32 * kSdcRounds))

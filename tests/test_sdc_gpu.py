@@ -153,3 +153,15 @@ def test_sdc_disc_edge_decided_by_the_quotient(cuda, D, iters):
     assert O.rel_l2(_estimate32(traj, mos, R, iters, reciprocal=True), ref) > 1e-5
     w = gb.sdc.estimate_dcw(torch.from_numpy(traj).to(cuda), (mos,) * D, 1.0, iters, 4.0)
     assert O.rel_l2(w.cpu().numpy(), ref) <= 1e-6
+
+
+def test_sdc_keeps_one_large_grid(cuda):
+    """A grid of more than 2^24 cells stays single: a call leaves no more device
+    memory behind than that grid."""
+    traj = S.kooshball_golden_means_3d(20, 32).astype(np.float32)
+    n, cells = (256, 256, 512), 256 * 256 * 512
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    w = gb.sdc.estimate_dcw(torch.from_numpy(traj).to(cuda), n, 1.0, 2, 4.0)
+    assert free - torch.cuda.mem_get_info()[0] < 1.5 * 4 * cells
+    assert bool(torch.isfinite(w).all()) and bool((w > 0).all())
