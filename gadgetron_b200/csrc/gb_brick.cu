@@ -72,8 +72,12 @@ struct BrickShape {
 constexpr int kBrickDepth = 3;    // batches of hits in the ring of a warp
 constexpr int kBrickQueue = 64;   // pending hits of a warp
 constexpr int kBrickMax = 16;     // bricks per tile
-constexpr int kBrickFillWarps = 148 * 12;   // warps that fill the GPU
-constexpr int kBrickWideWarps = 148 * 24 * 4;   // narrow-form warps from which the wide forms are taken
+// Warps up to which bricks share their lists among several warps (and the narrow
+// form takes 2 bricks per CTA).  Gridding in us at 0 / 888 / 1776 / 3552: 4096 samples on 128^2, 1
+// coil 15.9 / 13.3 / 13.2 / 12.8, 16 coils 23.0 / 19.7 / 18.2 / 18.4; 16384 samples on 256^2, 1 coil 17.0 /
+// 17.2 / 15.2 / 15.0.
+constexpr int kBrickFillWarps = kSMs * 12;
+constexpr int kBrickWideWarps = kSMs * 24 * 4;   // narrow-form warps from which the wide forms are taken
 constexpr int64_t kBrick3DWidePairs = 4 << 20;   // pairs from which 8 coils in 3D take four slices
 constexpr int kBrickWideList = 512;     // average list up to which they are
 

@@ -1,6 +1,6 @@
 // Arguments and launch configuration shared by the convolution kernels
-// (gridding: gb_brick.cu and k_grid_nc2c in gb_grid.cu; degridding and the
-// trajectory gradient: gb_grid.cu).
+// (gridding: gb_brick.cu; degridding and the trajectory gradient: gb_degrid.cu;
+// the general kernels for other tiles, widths and 1D, and the launchers: gb_grid.cu).
 #pragma once
 
 #include "gb_internal.cuh"

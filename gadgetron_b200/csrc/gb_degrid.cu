@@ -300,7 +300,7 @@ k_traj_grad(ConvArgs a, const float2 *__restrict__ grid, const float2 *__restric
     const KParams &k = a.k;
     const WorkItem it = a.items[blockIdx.x];
     const int org0 = it.tx * k.tile[0], org1 = it.ty * k.tile[1], org2 = it.tz * k.tile[2];
-    const int R0 = region_dim_t(k, 0), R1 = region_dim_t(k, 1), R2 = region_dim_t(k, 2);
+    const int R0 = region_dim_t(k, 0), R1 = region_dim_t(k, 1);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sl = lane / LPS, ll = lane % LPS;
     float *dwt = reinterpret_cast<float *>(smem_raw) + warp * (SPW * D * kWMax);   // [sample][dim][tap]
@@ -403,7 +403,6 @@ k_traj_grad(ConvArgs a, const float2 *__restrict__ grid, const float2 *__restric
             }
         }
     }
-    (void)R2;
 }
 
 // ------------------------------------------------------------- dispatch ---

@@ -280,14 +280,14 @@ __global__ void k_multiply_dcw(const float *__restrict__ dcw, float2 *__restrict
 
 static unsigned grid_for(int64_t n) {
     int64_t b = (n + 255) / 256;
-    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, 148 * 16));
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, kSMs * 16));
 }
 
 // Blocks for the row kernels: one pass over all image rows, at most 16 per SM.
 static unsigned rows_grid(int64_t rows, int width) {
     const int n0c = std::min(width, 256);
     const int64_t rpb = 256 / n0c;
-    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + rpb - 1) / rpb, 148 * 16));
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + rpb - 1) / rpb, kSMs * 16));
 }
 
 static unsigned rows_grid(const NufftPlan &p) {

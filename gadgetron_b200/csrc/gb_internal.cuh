@@ -30,6 +30,7 @@ namespace gb {
 
 constexpr int kMaxD = 3;
 constexpr int kWMax = 8;          // max taps per dimension (W <= 7)
+constexpr int kSMs = 148;       // B200
 constexpr int kThreads = 256;     // threads per CTA for the tile kernels
 constexpr int kChunk = 64;        // samples staged per pass (gridding)
 

@@ -611,7 +611,7 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     const int64_t M = p.Mtot;
     // (large enough that a tile is staged once or a few times; the region
     // copy is a large share of an item's work in 2D)
-    int deg_chunk = (int)std::max<int64_t>(256, std::min<int64_t>(1024, M / (148 * 4) + 1));
+    int deg_chunk = (int)std::max<int64_t>(256, std::min<int64_t>(1024, M / (kSMs * 4) + 1));
     // Both lists run longest item first, equal lengths in key order: a
     // counting sort on the length, written straight into the upload staging
     // (this runs in every preprocess).  First the counts.
@@ -652,7 +652,7 @@ void plan_build_work(NufftPlan &p, cudaStream_t st) {
     const int64_t total = goff[nkeys];
     const int64_t avg = total / std::max<uint32_t>(1, nkeys);
     const int split_len = (int)std::max<int64_t>(256, 2 * avg);
-    const int64_t longest = k.D == 2 ? std::max<int64_t>(512, total / (148 * 32)) : avg;
+    const int64_t longest = k.D == 2 ? std::max<int64_t>(512, total / (kSMs * 32)) : avg;
     const int most[2] = {(int)std::max<int64_t>(total < 100000 ? 96 : 128, std::min(avg, longest)),
                          split_len};   // chunk lengths: fine, coarse
     // equal lengths share a run up to 64K pairs; the few lists above keep key order in the last one
@@ -749,7 +749,7 @@ uint64_t plan_layout_signature(const NufftPlan &p, int nbf) {
                           p.img_os.get(), p.kgrid.get(), p.samp_ws.get(), p.deap_img.get(), p.deap_os.get()};
     for (const void *q : ptrs) mix((uint64_t)(uintptr_t)q);
     const int64_t vals[] = {p.n_deg_items, p.n_grd_items, p.n_splits, p.n_slots, p.Mtot, (int64_t)p.F,
-                            p.tiling.tile[0], p.tiling.tile[1], p.tiling.tile[2], p.tiling.cg, p.tiling.schedule,
+                            p.tiling.tile[0], p.tiling.tile[1], p.tiling.tile[2], p.tiling.cg,
                             (int64_t)p.grid_ctr_bytes, (int64_t)p.grid_ws.n, nbf};
     for (int64_t v : vals) mix((uint64_t)v);
     auto it = p.fft_plans.find(nbf);

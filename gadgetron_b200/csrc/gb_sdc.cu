@@ -307,7 +307,7 @@ int sdc_table_cap(const SdcArgs &a, bool two, int iterations) {
 void sdc_table_iterations(const SdcArgs &a, int cap, const float *traj, float *w, float *grid, float *tab, int64_t G,
                           int iterations, cudaStream_t st) {
     const unsigned int all = (unsigned int)((a.M + 7) / 8);   // one warp per sample
-    const unsigned int blocks = std::min(all, 148u * 16u);    // a few samples per warp
+    const unsigned int blocks = std::min(all, (unsigned int)kSMs * 16u);    // a few samples per warp
     k_sdc_table<<<all, 256, 0, st>>>(a, cap, traj, tab); note_launch();
     float *cur = grid, *next = grid + G;
     GB_CUDA(cudaMemsetAsync(cur, 0, (size_t)G * sizeof(float), st));

@@ -6,7 +6,7 @@
 // kernel width and on the number of coils.  For a preprocessed plan this
 // re-bins the trajectory for each candidate, times one gridding and one
 // degridding pass on `nb` batches with CUDA events -- as the normal operator
-// runs them (its sample workspace layout and gridding schedule), since the
+// runs them (its sample workspace layout), since the
 // CG-SENSE iteration is where the convolutions' time goes -- and keeps the
 // fastest.
 // Results are cached per (D, N, mos, W, frames, samples within 5%, batches)

@@ -158,8 +158,8 @@ GB_API gb_status gb_nufft_convolve(gb_nufft_plan plan, const void *in, void *out
  * code running in a host callback or a real-time thread with a fixed memory
  * budget, or under another allocator that must not be bypassed.  Its scratch (the partial tiles of heavily loaded tiles) is
  * a fixed 16 MiB array in device memory that each GPU loading this library
- * keeps until exit; a plan and batch count needing more is rejected with
- * GB_ERR_INVALID_ARGUMENT.  The first call on a device looks up the array's
+ * keeps until exit; a plan and batch count needing more (the batches rounded up
+ * to the plan's coil group) is rejected with GB_ERR_INVALID_ARGUMENT.  The first call on a device looks up the array's
  * device address (cudaGetSymbolAddress), so make it before any stream
  * capture.  All calls share the array: calls that overlap on the GPU race and
  * must be serialised by the caller.  The plan must be preprocessed. */
@@ -240,7 +240,7 @@ GB_API gb_status gb_nufft_set_tiling(gb_nufft_plan plan, const int *tile, int co
 /* Gridding schedule of the normal operator (mult_MH_M, the CG-SENSE
  * iteration): 0 (default), 1 or 2, kept by the plan and returned by the getter.
  * One gridding kernel, chosen by shape, now serves every value: results and
- * speed are the same.  (A captured CG graph is re-captured when it changes.)
+ * speed are the same.
  * No reference counterpart (tuning). */
 GB_API gb_status gb_nufft_set_grid_schedule(gb_nufft_plan plan, int schedule);
 GB_API gb_status gb_nufft_get_grid_schedule(gb_nufft_plan plan, int *schedule);

@@ -171,14 +171,12 @@ def test_traj_grad_fd_3d_alpha_1_5_w4():
     assert err <= FD_TOL, err
 
 
-def test_batched_many_frames_deep_launch_schedules():
+def test_batched_many_frames_deep_launch():
     """48 uneven frames of 64^2 (mos 128, 64 tiles a frame): the gridding
-    launch of E^H E is more than 8 resident waves deep.  Schedule 1 takes the
-    register-staged gridding over the plan's sorted sample layout, schedule 2
-    (and the default) the persistent work-queue kernel over the interleaved
-    layout (small launches take the per-item warp-specialized kernel,
-    covered by every other CG test).  Both give the same images bit for bit;
-    frame-independent CG against one oracle solve per frame."""
+    launch of E^H E is many resident waves deep.  Frame-independent CG against
+    one oracle solve per frame, with and without the graph; solved twice, the
+    images are the same bit for bit (one gridding kernel serves both schedule
+    values, and its sums have a fixed order)."""
     dev = torch.device("cuda:0")
     N, mos, W, C, F, iters = 64, 128, 5.5, 8, 48, 6
     spokes = [4 + (f * 5) % 9 for f in range(F)]

@@ -177,13 +177,13 @@ def test_batched_uneven_frames_equal_per_frame_solves(cuda):
         assert rel_l2(xb[f], xr[0]) <= 1e-4, f
 
 
-def test_grid_schedules_bit_identical(cuda):
-    """The normal operator's gridding schedules -- one CTA per work item
-    (schedule 1; here the warp-specialized kernel on the interleaved sample
-    layout) and one persistent work-queue launch (schedule 2) -- give
-    forward, E^H E and CG results equal bit for bit, on uneven frames whose
-    dense radial centres are split over several work items, and match the
-    oracle."""
+def test_grid_schedule_value_is_kept_and_changes_nothing(cuda):
+    """The plan keeps the schedule value and refuses others; one gridding
+    kernel serves every value, so forward, E^H E and CG results are equal bit
+    for bit -- what this checks of the kernel is that it is deterministic -- on
+    uneven frames whose dense radial centres are split over several work items,
+    and match the oracle.  (Kernel forms that differ are compared in
+    test_gridding_shapes_gpu.py.)"""
     N, mos, W, C = 32, 64, 5.5, 12
     spokes = [64, 7, 13, 40, 5]
     trajs = [S.radial_golden_angle_2d(s, 64, profile_offset=11 * f) for f, s in enumerate(spokes)]
