@@ -290,6 +290,35 @@ def test_image_operator_matches_oracle(cuda):
     np.testing.assert_allclose(R.get().cpu().numpy(), ref3, rtol=2e-6)
 
 
+def test_image_operator_sizes_in_turn_and_from_threads(cuda):
+    """Calls share scratch per device: images of one block, a few and more blocks
+    than the grid holds, in turn and from four threads on streams of their own,
+    give what each gives against the oracle, bit for bit among themselves."""
+    from concurrent.futures import ThreadPoolExecutor
+    rng = np.random.default_rng(22)
+    zs = [(rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64) for n in (200, 9000, 400001)]
+    refs = [O.image_operator_compute(z) for z in zs]
+    torch.cuda.synchronize()
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got = []
+            for i in range(6):
+                R = gb.cuImageOperator()
+                R.compute(torch.from_numpy(zs[(k + i) % 3]).to(cuda))
+                got.append(((k + i) % 3, R.offset_, R.get().cpu().numpy()))
+            return got
+
+    first = {}
+    with ThreadPoolExecutor(4) as ex:
+        for got in ex.map(work, range(4)):
+            for i, off, img in got:
+                ref, ref_off = refs[i]
+                assert abs(off - ref_off) <= 1e-6 * ref_off
+                np.testing.assert_allclose(img, ref, rtol=2e-6)
+                assert np.array_equal(first.setdefault(i, img), img)
+
+
 def test_sense_precond_weights_matches_oracle(cuda):
     case = sense_case(coils=8, seed=5)
     E, orc = make_ops(case, cuda)
