@@ -113,6 +113,30 @@ def test_wide_form_on_every_tile(cuda, tile, coils):
         assert rel_l2(x[:, f].cpu().numpy(), ref[:, 0]) <= PARITY_TOL, f
 
 
+@pytest.mark.parametrize("group", [4, 8, 16])
+@pytest.mark.parametrize("tile", [(16, 16), (32, 16), (16, 32), (32, 32), (8, 32), (32, 8), (8, 8, 4), (8, 8, 8),
+                                  (16, 8, 8), (8, 16, 8), (16, 16, 4)])
+def test_every_tile_of_the_autotuner(cuda, tile, group):
+    """Every tile and coil group that the autotuner times, both directions of
+    17 coils against the oracle."""
+    D, coils = len(tile), 17
+    N, mos = ((32, 64), (64, 96)) if D == 2 else ((32, 32, 32), (64, 64, 64))
+    traj = S.radial_golden_angle_2d(40, 96) if D == 2 else S.kooshball_golden_means_3d(80, 48)
+    plan = gb.NFFT.make_plan(N, mos, 4.0)
+    plan.set_tiling(tile, group)
+    plan.preprocess(torch.from_numpy(traj).to(cuda))
+    orc = O.OraclePlan(N, mos, 4.0)
+    orc.preprocess(traj.reshape(1, -1, D))
+    y = _samples(coils, traj.shape[0], group)
+    x = torch.empty((coils, 1) + tuple(reversed(N)), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(y).to(cuda), x, None, gb.NFFT_comp_mode.BACKWARDS_NC2C)
+    assert rel_l2(x.cpu().numpy(), orc.backwards_nc2c(y)) <= PARITY_TOL
+    img = S.gaussian_image((coils, 1) + tuple(reversed(N)), 3)
+    out = torch.empty((coils, traj.shape[0]), dtype=torch.complex64, device=cuda)
+    plan.compute(torch.from_numpy(img).to(cuda), out, None, gb.NFFT_comp_mode.FORWARDS_C2NC)
+    assert rel_l2(out.cpu().numpy(), orc.forward_c2nc(img)) <= PARITY_TOL
+
+
 @pytest.mark.parametrize("coils", [9, 12, 24])
 def test_wide_forms_of_other_coil_counts(cuda, coils):
     """The wide form with idle coils, and the 12-coil form, which takes over at
